@@ -380,7 +380,7 @@ __device__ __forceinline__ unsigned to_tf32( float x )
 // update between sub-blocks is an 8 x 8 x 8 product on the FP64 tensor cores
 // (two DMMA m8n8k4).  The outer loops over sub-blocks stay rolled so the code
 // fits the instruction cache.
-constexpr int kPotrfThreads = 256;
+constexpr int kPotrfThreads = 384;
 constexpr int kTrsmThreads  = 256;
 constexpr int kSub          = 8;                     // sub-block edge
 constexpr int kSubs         = kPanel / kSub;         // 8 sub-blocks per panel edge
@@ -400,359 +400,421 @@ __device__ __forceinline__ void dmma_8x8x8( double (&acc)[2], FA a, FB b )
     }
 }
 
-constexpr size_t kPotrfSmemBytes = sizeof(double) * (2 * kPanel * (kPanel + 1) + 2 * kPanel + 1);
+constexpr int kPld = kPanel + 4;                     // padded smem row of the panel's blocks: DMMA fragments of a
+                                                     // block and of its transpose load without bank conflicts
+constexpr size_t kPotrfSmemBytes = sizeof(double) * (2 * kPanel * kPld + kPanel + 2);
 
 template<typename T> __device__ __forceinline__ double round_to( double v ) { return static_cast<double>( static_cast<T>( v ) ); }
 
-// Panel factorization state in shared memory.  D: the 64 x 64 block, upper
-// triangle (A, overwritten by U row block by row block); Ti: the inverse
-// T = U^{-1} (upper tiles; diagonal tiles zero below the diagonal; its
-// strictly lower tiles serve as per-warp scratch); inv_d: the reciprocal
-// pivots the row-block solves use.
+// Panel factorization state, at the start of the kernel's dynamic shared
+// memory.  D: the 64 x 64 block, upper triangle (A, overwritten by U tile row
+// by tile row); Ti: the inverse T = U^{-1}, upper 8 x 8 tiles (the diagonal
+// tiles are zero below the diagonal).
 struct PotrfShared
 {
-    double (*D)[kPanel + 1];
-    double (*Ti)[kPanel + 1];
-    double * inv_d;
+    double (*D)[kPld];
+    double (*Ti)[kPld];
     double * floor_s;
     int * fail;
     int * redo;
+    int * raised;                                       // bit q: tile q has raised pivots (mixed precision)
 };
 
-// The scratch tile of warp w = 1..7: the strictly lower tile (7, w - 1) of Ti.
-__device__ __forceinline__ double (*potrf_scratch( const PotrfShared & sh ))[kPanel + 1]
+__device__ __forceinline__ PotrfShared potrf_shared()
 {
-    return reinterpret_cast<double (*)[kPanel + 1]>( &sh.Ti[kPanel - kSub][kSub * ((threadIdx.x >> 5) - 1)] );
+    extern __shared__ __align__(16) double panel_smem[];
+    PotrfShared sh;
+    sh.D = reinterpret_cast<double (*)[kPld]>( panel_smem );
+    sh.Ti = reinterpret_cast<double (*)[kPld]>( panel_smem + kPanel * kPld );
+    sh.floor_s = panel_smem + 2 * kPanel * kPld;        // the panel's pivot floors (mixed precision)
+    sh.fail = reinterpret_cast<int *>( sh.floor_s + kPanel );
+    sh.redo = sh.fail + 1;
+    sh.raised = sh.fail + 2;
+    return sh;
 }
 
-// Stores a factored diagonal tile: U_qq, rounded to the storage type, over
-// the tile's upper triangle and its reciprocal pivots (of the unrounded
-// pivots) into inv_d.
-template<typename T>
-__device__ __forceinline__ void potrf_store_tile( const PotrfShared & sh, int o, const double (&a)[kSub][kSub], const double (&iv)[kSub] )
-{
-    if( (threadIdx.x & 31) == 0 )
-    {
-#pragma unroll
-        for( int r = 0; r < kSub; ++r )
-        {
-#pragma unroll
-            for( int c = r; c < kSub; ++c ) { sh.D[o + r][o + c] = round_to<T>( a[r][c] ); }
-            sh.inv_d[o + r] = iv[r];
-        }
-    }
-    __syncwarp();
-}
-
-// The diagonal tile's Cholesky with pivot floors (mixed precision): a pivot
-// lost to FP32 rounding (for a 1 x 1 supernode too: |a| can cancel to 0) is
-// raised to its floor (static pivoting); the FP64 refinement corrects it.
-// The raised pivot also bounds the row's entries in the block by beta =
-// sqrt(max |a_ii|), the growth bound of the modified Cholesky of Gill, Murray
-// and Wright: a small pivot under a large row would otherwise make the next
-// pivots of the block hugely negative, floored in turn, until FP32
-// overflows.  Runs only for tiles with a pivot at or below its floor, after
-// the tile's row block is complete.
-template<typename T>
-__device__ __noinline__ void potrf_tile_floored( const PotrfShared & sh, const PanelTask & t, int q, int nb, const T * __restrict__ arena,
+// Cholesky of the diagonal tile q of D by one warp, and W = U_qq^{-1} into
+// tile (q, q) of Ti.  Every lane holds the whole trailing tile in registers
+// and runs the same branch-free recurrence, so that a pivot's chain is one
+// reciprocal square root, one product and one fused multiply-add (83 cycles);
+// lane j also carries column j of the identity through the elimination, whose
+// row r is then L^{-1}_rj = W_jr (L = U_qq^T), off the pivot chain.  With FP32 storage U is rounded as it is
+// stored and W inverts the rounded rows (the reciprocal of a stored pivot by
+// one Newton step on the reciprocal square root, r = v (2 - u v)).
+//
+// A non-positive pivot (FP64) records the first failing row and lets NaNs run
+// on.  kFloored (mixed precision, run again for a tile that met a pivot at or
+// below its floor, once the tile's row block is complete): a pivot lost to
+// FP32 rounding (for a 1 x 1 supernode too: |a| can cancel to 0) is raised to
+// its floor (static pivoting); the FP64 refinement corrects it.  The raised
+// pivot also bounds the row's entries in the block by beta = sqrt(max |a_ii|),
+// the growth bound of the modified Cholesky of Gill, Murray and Wright: a small
+// pivot under a large row would otherwise make the next pivots of the block
+// hugely negative, floored in turn, until FP32 overflows.  Without kFloored
+// such a tile is left as it was and the function returns false.
+template<typename T, bool kFloored>
+__device__ __forceinline__ bool potrf_diag_tile( const PotrfShared & sh, const PanelTask & t, int q, int nb, const T * __restrict__ arena,
                                                  int * __restrict__ status, const double * __restrict__ pivot_floor )
 {
     const int lane = threadIdx.x & 31;
     const int o = kSub * q;
-    double a[kSub][kSub], iv[kSub];
-#pragma unroll
-    for( int r = 0; r < kSub; ++r )
-    {
-#pragma unroll
-        for( int c = r; c < kSub; ++c ) { a[r][c] = sh.D[o + r][o + c]; }
-    }
-#pragma unroll
-    for( int r = 0; r < kSub; ++r )
-    {
-        double d = a[r][r];
-        const bool single = (t.single_rows >> (o + r)) & 1;
-        if( single ) { d = fabs( d ); }                     // 1 x 1 reference supernodes: sqrt(|a|)
-        const double tau = sh.floor_s[o + r];
-        if( o + r < nb && !(d > tau) )
-        {
-            // the row's largest entry: this tile's columns, the rest of the
-            // block and the row's rest columns in U0 and U1, which the trsm
-            // divides by the pivot
-            double m = 0.0;
-#pragma unroll
-            for( int c = r + 1; c < kSub; ++c ) { m = fmax( m, fabs( a[r][c] ) ); }
-            for( int c = o + kSub + lane; c < kPanel; c += 32 ) { m = fmax( m, fabs( sh.D[o + r][c] ) ); }
-            const std::int64_t grow = t.r0 + o + r;
-            for( int c = t.r0 + nb + lane; c < t.n0; c += 32 ) { m = fmax( m, fabs( static_cast<double>( arena[t.u0 + grow * t.ld0 + c] ) ) ); }
-            for( int c = lane; c < t.n1; c += 32 ) { m = fmax( m, fabs( static_cast<double>( arena[t.u1 + grow * t.ld1 + c] ) ) ); }
-#pragma unroll
-            for( int s2 = 16; s2 > 0; s2 >>= 1 ) { m = fmax( m, __shfl_xor_sync( 0xffffffffu, m, s2 ) ); }
-            if( lane == 0 ) { atomicAdd( status + 2, 1 ); }
-            const double beta2 = pivot_floor[0];
-            d = fmax( tau, beta2 > 0.0 ? m * m / beta2 : 0.0 );
-        }
-        iv[r] = rsqrt( d );
-        a[r][r] = d * iv[r];
-#pragma unroll
-        for( int c = r + 1; c < kSub; ++c ) { a[r][c] *= iv[r]; }
-#pragma unroll
-        for( int r2 = r + 1; r2 < kSub; ++r2 )
-        {
-#pragma unroll
-            for( int c = r2; c < kSub; ++c ) { a[r2][c] -= a[r][r2] * a[r][c]; }
-        }
-    }
-    potrf_store_tile<T>( sh, o, a, iv );
-}
-
-// Cholesky of the diagonal tile q of D by one warp.  Every lane holds the
-// whole tile in registers and runs the same branch-free recurrence, so that
-// a pivot's chain is one reciprocal square root, one product and one fused
-// multiply-add; pivot checks come after the tile.  A non-positive pivot (FP64)
-// records the first failing row and lets NaNs run on, as before.  With pivot
-// floors (mixed precision), a tile that has a pivot at or below its floor is
-// factored again by potrf_tile_floored, whose raised pivots depend on the
-// whole row: speculative (the tile's row block right of it may still be
-// changing) returns false instead, with nothing written.
-template<typename T>
-__device__ bool potrf_diag_tile( const PotrfShared & sh, const PanelTask & t, int q, int nb, const T * __restrict__ arena,
-                                 int * __restrict__ status, const double * __restrict__ pivot_floor, bool speculative )
-{
-    const int lane = threadIdx.x & 31;
-    const int o = kSub * q;
     const unsigned singles = static_cast<unsigned>( (t.single_rows >> o) & 0xff );
-    double a[kSub][kSub], iv[kSub], piv[kSub], fl[kSub];
+    double a[kSub][kSub], w[kSub];
 #pragma unroll
     for( int r = 0; r < kSub; ++r )
     {
+        w[r] = lane == r ? 1.0 : 0.0;
 #pragma unroll
         for( int c = r; c < kSub; ++c ) { a[r][c] = sh.D[o + r][o + c]; }
-        // the pivot floors are read with the tile, off the pivot chain
-        if constexpr ( sizeof(T) == 4 ) { fl[r] = sh.floor_s[o + r]; }
     }
+    auto store_row = [&]( int r, const double (&v)[kSub] )
+    {
+        if( lane != 0 ) { return; }
+        if( r & 1 ) { sh.D[o + r][o + r] = v[r]; }
+#pragma unroll
+        for( int c = 0; c < kSub; c += 2 )
+        {
+            if( c >= r ) { *reinterpret_cast<double2 *>( &sh.D[o + r][o + c] ) = make_double2( v[c], v[c + 1] ); }
+        }
+    };
+    unsigned nonpos = 0u, low = 0u;                     // rows whose pivot is not positive / not above its floor
 #pragma unroll
     for( int r = 0; r < kSub; ++r )
     {
-        const double d = ((singles >> r) & 1) ? fabs( a[r][r] ) : a[r][r];   // 1 x 1 reference supernodes: sqrt(|a|)
-        piv[r] = d;
-        iv[r] = rsqrt( d );
-        a[r][r] = d * iv[r];
+        double d = ((singles >> r) & 1) ? fabs( a[r][r] ) : a[r][r];   // 1 x 1 reference supernodes: sqrt(|a|)
+        if constexpr ( sizeof(T) == 4 )
+        {
+            const double tau = sh.floor_s[o + r];
+            if constexpr ( kFloored )
+            {
+                if( o + r < nb && !(d > tau) )
+                {
+                    // the row's largest entry: this tile's columns, the rest of the
+                    // block and the row's rest columns in U0 and U1, which the trsm
+                    // divides by the pivot
+                    double m = 0.0;
 #pragma unroll
-        for( int c = r + 1; c < kSub; ++c ) { a[r][c] *= iv[r]; }
+                    for( int c = r + 1; c < kSub; ++c ) { m = fmax( m, fabs( a[r][c] ) ); }
+                    for( int c = o + kSub + lane; c < kPanel; c += 32 ) { m = fmax( m, fabs( sh.D[o + r][c] ) ); }
+                    const std::int64_t grow = t.r0 + o + r;
+                    for( int c = t.r0 + nb + lane; c < t.n0; c += 32 ) { m = fmax( m, fabs( static_cast<double>( arena[t.u0 + grow * t.ld0 + c] ) ) ); }
+                    for( int c = lane; c < t.n1; c += 32 ) { m = fmax( m, fabs( static_cast<double>( arena[t.u1 + grow * t.ld1 + c] ) ) ); }
+#pragma unroll
+                    for( int s2 = 16; s2 > 0; s2 >>= 1 ) { m = fmax( m, __shfl_xor_sync( 0xffffffffu, m, s2 ) ); }
+                    if( lane == 0 ) { atomicAdd( status + 2, 1 ); }
+                    const double beta2 = pivot_floor[0];
+                    d = fmax( tau, beta2 > 0.0 ? m * m / beta2 : 0.0 );
+                }
+            }
+            else { if( o + r < nb && !(d > tau) ) { low |= 1u << r; } }
+        }
+        if( !(d > 0.0) ) { nonpos |= 1u << r; }
+        const double iv = rsqrt( d );
+        double us[kSub];
+        a[r][r] = d * iv;
+        us[r] = round_to<T>( a[r][r] );
+#pragma unroll
+        for( int c = r + 1; c < kSub; ++c ) { a[r][c] *= iv; us[c] = round_to<T>( a[r][c] ); }
+        w[r] *= iv * fma( -us[r], iv, 2.0 );
 #pragma unroll
         for( int r2 = r + 1; r2 < kSub; ++r2 )
         {
 #pragma unroll
             for( int c = r2; c < kSub; ++c ) { a[r2][c] -= a[r][r2] * a[r][c]; }
+            w[r2] -= us[r2] * w[r];
         }
+        // FP64: the row goes out as it is formed, in the shadow of the pivot chain
+        if constexpr ( sizeof(T) == 8 ) { store_row( r, us ); }
+        else
+        {
+#pragma unroll
+            for( int c = r; c < kSub; ++c ) { a[r][c] = us[c]; }
+        }
+    }
+    if constexpr ( sizeof(T) == 4 && !kFloored )
+    {
+        if( low != 0u && pivot_floor != nullptr ) { return false; }
+    }
+    nonpos &= ~singles;
+    if( nb - o < kSub ) { nonpos &= (1u << (nb - o)) - 1u; }
+    if( lane == 0 && nonpos != 0u && *sh.fail < 0 ) { *sh.fail = o + __ffs( nonpos ) - 1; }
+    if( lane < kSub )
+    {
+#pragma unroll
+        for( int i = 0; i < kSub; i += 2 ) { *reinterpret_cast<double2 *>( &sh.Ti[o + lane][o + i] ) = make_double2( w[i], w[i + 1] ); }
     }
     if constexpr ( sizeof(T) == 4 )
     {
-        bool low = false;
 #pragma unroll
-        for( int r = 0; r < kSub; ++r ) { low |= o + r < nb && !(piv[r] > fl[r]); }
-        if( low && pivot_floor != nullptr )
-        {
-            if( speculative ) { return false; }
-            potrf_tile_floored<T>( sh, t, q, nb, arena, status, pivot_floor );
-            return true;
-        }
+        for( int r = 0; r < kSub; ++r ) { store_row( r, a[r] ); }
     }
-    if( lane == 0 )
+    __syncwarp();
+    return true;
+}
+
+// The floored factorization of a tile: rare, kept out of the kernel's code.
+template<typename T>
+__device__ __noinline__ void potrf_tile_floored( const PanelTask & t, int q, int nb, const T * __restrict__ arena,
+                                                 int * __restrict__ status, const double * __restrict__ pivot_floor )
+{
+    const PotrfShared sh = potrf_shared();
+    potrf_diag_tile<T, true>( sh, t, q, nb, arena, status, pivot_floor );
+    if( (threadIdx.x & 31) == 0 ) { *sh.raised |= 1 << q; }
+}
+
+// U_bc = U_bb^{-T} A_bc for tile (b, c) of D (tile corners o, oc), one column per lane.
+template<typename T>
+__device__ __noinline__ void potrf_row_substitution( int o, int oc )
+{
+    const PotrfShared sh = potrf_shared();
+    const int lane = threadIdx.x & 31;
+    if( lane < kSub )
     {
+        double x[kSub];
+#pragma unroll
+        for( int r = 0; r < kSub; ++r ) { x[r] = sh.D[o + r][oc + lane]; }
 #pragma unroll
         for( int r = 0; r < kSub; ++r )
         {
-            if( !((singles >> r) & 1) && o + r < nb && !(piv[r] > 0.0) && *sh.fail < 0 ) { *sh.fail = o + r; }
+            x[r] /= sh.D[o + r][o + r];
+#pragma unroll
+            for( int r2 = r + 1; r2 < kSub; ++r2 ) { x[r2] -= sh.D[o + r][o + r2] * x[r]; }
         }
+#pragma unroll
+        for( int r = 0; r < kSub; ++r ) { sh.D[o + r][oc + lane] = round_to<T>( x[r] ); }
     }
-    potrf_store_tile<T>( sh, o, a, iv );
-    return true;
 }
 
 // Cholesky of one panel's 64 x 64 diagonal block D (identity beyond nb) and
 // the inverse T = D^{-1} of its factor (LAPACK potrf of FactorizeSupernode,
 // Multifrontal.hpp:438-449, plus the inverse the panel's trsm and the solves
-// use), right-looking by 8 x 8 tiles, two barriers per tile step b:
-//   1. U_bc = U_bb^{-T} A_bc for the columns right of tile b, one column per
-//      thread; one warp forms W_b = U_bb^{-1} (tile (b, b) of T).
-//   2. warp 0 applies row block b's update to tile (b+1, b+1) and factors
-//      that tile ahead; the other warps update the other trailing tiles and
-//      form column block b of T, T_ib = -(sum_{k=i..b-1} T_ik U_kb) W_b.
-// Tile products run on the FP64 tensor cores (two DMMA m8n8k4 each).  A row
+// use), right-looking by 8 x 8 tiles.  The bound is the chain of 64 pivots
+// (~93 cycles each), so warp 0 runs only that chain: per tile step b it forms
+// U_b,b+1 = W_b^T A_b,b+1 (W_b = U_bb^{-1}, left by the tile's
+// factorization), updates tile (b+1, b+1) and factors it.  Meanwhile the
+// other warps
+//   1. form U_bc = W_b^T A_bc for c > b+1 and T_ib = -S_ib W_b for i < b, and
+//   2. (behind a barrier that warp 0 passes without waiting) update the other
+//      trailing tiles, and sum S_i,b+1 = sum_{k=i..b} T_ik U_k,b+1; then
+//      they write out what step b-1 finished,
+// one 8 x 8 tile per warp and job, each a few DMMA m8n8k4; one full barrier
+// ends the step.  After the last tile only T's last column is left.  A row
 // that forms a 1 x 1 reference supernode takes sqrt(|a|) as the reference
 // does (:471) and never reports failure.  With FP32 storage every U value is
 // rounded to FP32 as it is formed, so the in-panel updates, W and T use the
 // stored factor (T inverts it), as the updates of later panels do.
-template<typename T>
+// kThreads: 384 in the level launches, 256 in the persistent kernel.
+template<typename T, int kThreads>
 __device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict__ arena, int * __restrict__ status,
-                                            double * smem, const double * __restrict__ pivot_floor, double * __restrict__ tinv )
+                                            const double * __restrict__ pivot_floor, double * __restrict__ tinv )
 {
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const int nb = min( kPanel, t.n0 - t.r0 );
-    PotrfShared sh;
-    sh.D = reinterpret_cast<double (*)[kPanel + 1]>( smem );
-    sh.Ti = reinterpret_cast<double (*)[kPanel + 1]>( smem + kPanel * (kPanel + 1) );
-    sh.inv_d = smem + 2 * kPanel * (kPanel + 1);
-    sh.floor_s = sh.inv_d + kPanel;                     // the panel's pivot floors (mixed precision)
-    sh.fail = reinterpret_cast<int *>( sh.floor_s + kPanel );
-    sh.redo = sh.fail + 1;
+    const PotrfShared sh = potrf_shared();
 
     T * U0 = arena + t.u0 + (std::int64_t)t.r0 * t.ld0 + t.r0;
-    auto stage_src = [&]( int idx, double & fill ) -> const T *
+    // 16-byte pieces of the rows (16-byte aligned: offsets and leading dimensions are multiples of
+    // kLdAlign entries), all of a thread's in flight together; pieces below the diagonal are not read
+    // later and not loaded; identity padding beyond nb
+    constexpr int kV = 16 / static_cast<int>( sizeof(T) );
+    constexpr int kAll = kPanel * kPanel / kV, kPieces = (kAll + kThreads - 1) / kThreads;
+    if constexpr ( sizeof(T) == 8 )
     {
-        const int r = idx / kPanel, c = idx % kPanel;
-        fill = (r >= nb && r == c) ? 1.0 : 0.0;      // identity padding beyond nb
-        return (r < nb && c < nb && r <= c) ? U0 + (std::int64_t)r * t.ld0 + c : nullptr;
-    };
-    auto stage_dst = [&]( int idx ) { return &sh.D[idx / kPanel][idx % kPanel]; };
-    stage_block<T, kPanel * kPanel / kPotrfThreads, kPotrfThreads>( U0, stage_src, stage_dst );
+#pragma unroll
+        for( int u = 0; u < kPieces; ++u )
+        {
+            const int idx = kV * (tid + u * kThreads), r = idx / kPanel, c = idx % kPanel;
+            if( r >= kPanel ) {}
+            else if( r >= nb ) { sh.D[r][c] = r == c ? 1.0 : 0.0; sh.D[r][c + 1] = r == c + 1 ? 1.0 : 0.0; }
+            else if( c + 1 >= r ) { cp_async_16( &sh.D[r][c], c < nb ? U0 + (std::int64_t)r * t.ld0 + c : U0, c + 1 < nb ? 16 : c < nb ? 8 : 0 ); }
+            if( u == 0 ) { cp_async_commit(); }         // the first rows: tile 0 starts when they are in
+        }
+        cp_async_commit();
+    }
+    else
+    {
+        float4 v[kPieces];
+#pragma unroll
+        for( int u = 0; u < kPieces; ++u )
+        {
+            const int idx = kV * (tid + u * kThreads), r = idx / kPanel, c = idx % kPanel;
+            v[u] = make_float4( 0.f, 0.f, 0.f, 0.f );
+            if( r < nb && c < nb && c + 3 >= r ) { v[u] = *reinterpret_cast<const float4 *>( U0 + (std::int64_t)r * t.ld0 + c ); }
+        }
+#pragma unroll
+        for( int u = 0; u < kPieces; ++u )
+        {
+            const int idx = kV * (tid + u * kThreads), r = idx / kPanel, c = idx % kPanel;
+            if( r >= kPanel ) { continue; }
+            const double pad = r >= nb ? 1.0 : 0.0;
+            const float f[4] = { v[u].x, v[u].y, v[u].z, v[u].w };
+#pragma unroll
+            for( int e = 0; e < 4; ++e ) { sh.D[r][c + e] = r < nb && c + e < nb ? static_cast<double>( f[e] ) : r == c + e ? pad : 0.0; }
+        }
+    }
     // the pivot floors after the block's copies are in flight (their loads overlap)
     if( pivot_floor != nullptr && tid < nb ) { sh.floor_s[tid] = pivot_floor[1 + t.row0 + t.r0 + tid]; }
-    if( tid == 0 ) { *sh.fail = -1; *sh.redo = 0; }
-    cp_async_wait_all();
-    stage_finish<T, kPanel * kPanel / kPotrfThreads, kPotrfThreads>( stage_src, stage_dst );
+    if( tid == 0 ) { *sh.fail = -1; *sh.redo = 0; *sh.raised = 0; }
+    cp_async_wait<1>();
     __syncthreads();
 
     const int nsub = (nb + kSub - 1) / kSub;
-    if( warp == 0 ) { potrf_diag_tile<T>( sh, t, 0, nb, arena, status, pivot_floor, false ); }
-    __syncthreads();
     const int i8 = lane >> 2, j8 = 2 * (lane & 3);        // this lane's entries of an 8 x 8 DMMA result
-    for( int b = 0; b < nsub; ++b )
+    // U_bc = W_b^T A_bc in place (tile (b, c) of D), rounded to the storage type.  Mixed precision,
+    // tiles with raised pivots: by substitution, as a raised pivot next to large entries makes W_b's
+    // entries grow beyond what the product can cancel.
+    auto row_tile = [&]( int o, int oc )
+    {
+        if constexpr ( sizeof(T) == 4 )
+        {
+            if( (sh.raised[0] >> (o / kSub)) & 1 )
+            {
+                potrf_row_substitution<T>( o, oc );
+                return;
+            }
+        }
+        double acc[2] = { 0.0, 0.0 };
+        dmma_8x8x8( acc, [&]( int ii, int k ) { return sh.Ti[o + k][o + ii]; }, [&]( int k, int jj ) { return sh.D[o + k][oc + jj]; } );
+        __syncwarp();
+        *reinterpret_cast<double2 *>( &sh.D[o + i8][oc + j8] ) = make_double2( round_to<T>( acc[0] ), round_to<T>( acc[1] ) );
+    };
+    // tile (r, c) of D -= U_b,r^T U_b,c (summed apart and subtracted once: one rounding at the tile's
+    // own magnitude per step)
+    auto trailing_tile = [&]( int o, int orow, int oc )
+    {
+        double2 * d = reinterpret_cast<double2 *>( &sh.D[orow + i8][oc + j8] );
+        const double2 v = *d;
+        double acc[2] = { 0.0, 0.0 };
+        dmma_8x8x8( acc, [&]( int ii, int k ) { return sh.D[o + k][orow + ii]; }, [&]( int k, int jj ) { return sh.D[o + k][oc + jj]; } );
+        *d = make_double2( v.x - acc[0], v.y - acc[1] );
+    };
+    // What step b finished, to global memory, in kSub + nsub units of 32 threads: U's row u of tile
+    // row b (columns from the diagonal on), then 8 rows of T's column block b (zero below the
+    // diagonal; the nsub leading tiles are all that the trsm and the solves read).
+    const int nbp = kSub * nsub;
+    double * out = tinv + (std::int64_t)t.panel * (kPanel * kPanel);
+    auto store_unit = [&]( int b, int u )
     {
         const int o = kSub * b;
-        const int rem = nsub - 1 - b;                   // trailing tile rows / columns
-        // 1. row block b right of its diagonal tile; W_b
-        if( tid < kSub * rem )
+        if( u < kSub )
         {
-            const int col = o + kSub + tid;
-            double x[kSub];
-#pragma unroll
-            for( int r = 0; r < kSub; ++r ) { x[r] = sh.D[o + r][col]; }
-#pragma unroll
-            for( int r = 0; r < kSub; ++r )
+            const int r = o + u, c = 2 * lane;
+            if( r >= nb ) { return; }
+            const double2 v = *reinterpret_cast<const double2 *>( &sh.D[r][c] );
+            T * dst = U0 + (std::int64_t)r * t.ld0 + c;
+            if( r <= c && c + 1 < nb )
             {
-                x[r] *= sh.inv_d[o + r];
-#pragma unroll
-                for( int r2 = r + 1; r2 < kSub; ++r2 ) { x[r2] -= sh.D[o + r][o + r2] * x[r]; }
+                if constexpr ( sizeof(T) == 8 ) { *reinterpret_cast<double2 *>( dst ) = v; }
+                else { *reinterpret_cast<float2 *>( dst ) = make_float2( static_cast<float>( v.x ), static_cast<float>( v.y ) ); }
             }
-#pragma unroll
-            for( int r = 0; r < kSub; ++r ) { sh.D[o + r][col] = round_to<T>( x[r] ); }
-        }
-        else if( warp == 7 )
-        {
-            // column j = lane of W_b = U_bb^{-1} (lanes 8-31 repeat lanes 0-7 and store nothing):
-            // w_jj = 1 / u_jj, then for k = j-1, .., 0 w_k = -(sum_{i>k} u_ki w_i) / u_kk, as one
-            // branch-free recurrence over k = 7..0.  The reciprocals of the stored pivots come from
-            // one Newton step on the tile's reciprocal square roots, r = v (2 - u v).
-            const int j = lane & (kSub - 1);
-            double rec[kSub], w[kSub], sum[kSub];
-#pragma unroll
-            for( int k = 0; k < kSub; ++k )
+            else
             {
-                const double v = sh.inv_d[o + k];
-                rec[k] = v * fma( -sh.D[o + k][o + k], v, 2.0 );
-                sum[k] = 0.0;
-            }
-#pragma unroll
-            for( int k = kSub - 1; k >= 0; --k )
-            {
-                w[k] = j == k ? rec[k] : (j > k ? -rec[k] * sum[k] : 0.0);
-#pragma unroll
-                for( int i = 0; i < k; ++i ) { sum[i] = fma( sh.D[o + i][o + k], w[k], sum[i] ); }
-            }
-            if( lane < kSub )
-            {
-#pragma unroll
-                for( int i = 0; i < kSub; ++i ) { sh.Ti[o + i][o + j] = w[i]; }
-            }
-        }
-        __syncthreads();
-        // 2. trailing tiles and T's column block b
-        if( warp == 0 )
-        {
-            if( rem > 0 )
-            {
-                const int o1 = o + kSub;
-                double acc[2] = { 0.0, 0.0 };
-                dmma_8x8x8( acc, [&]( int ii, int k ) { return sh.D[o + k][o1 + ii]; }, [&]( int k, int jj ) { return sh.D[o + k][o1 + jj]; } );
-                sh.D[o1 + i8][o1 + j8] -= acc[0];
-                sh.D[o1 + i8][o1 + j8 + 1] -= acc[1];
-                __syncwarp();
-                if( !potrf_diag_tile<T>( sh, t, b + 1, nb, arena, status, pivot_floor, true ) && lane == 0 ) { *sh.redo = 1; }
+                if( r <= c && c < nb ) { dst[0] = static_cast<T>( v.x ); }
+                if( r <= c + 1 && c + 1 < nb ) { dst[1] = static_cast<T>( v.y ); }
             }
         }
         else
         {
-            const int tiles = rem * (rem + 1) / 2 - (rem > 0 ? 1 : 0);     // all but (b+1, b+1)
-            // warp 4 shares warp 0's SM sub-partition (warp index mod 4) and
-            // stays idle, so that the tile factorization's FP64 chain does not
-            // wait behind tile products
-            for( int job = warp - (warp < 4 ? 1 : 2); warp != 4 && job < tiles + b; job += kPotrfThreads / 32 - 2 )
+            const int r = kSub * (u - kSub) + (lane >> 2), c = o + 2 * (lane & 3);
+            const double2 v = *reinterpret_cast<const double2 *>( &sh.Ti[r][c] );
+            *reinterpret_cast<double2 *>( out + r * kPanel + c ) = r < o + kSub ? v : make_double2( 0.0, 0.0 );
+        }
+    };
+    // step -1 only factors tile 0 (while the rest of the block arrives)
+    for( int b = -1; b < nsub; ++b )
+    {
+        const int o = kSub * b, o1 = o + kSub;
+        const int rem = nsub - 1 - b;                   // trailing tile rows / columns
+        if( warp == 0 )
+        {
+            if( rem > 0 )
             {
-                if( job < tiles )
+                if( b >= 0 )
                 {
-                    // job -> (b2, c), column by column of the trailing triangle after (b+1, b+1)
-                    int c = b + 2, left = job;
-                    while( left >= c - b ) { left -= c - b; ++c; }
-                    const int o2 = kSub * (b + 1 + left), oc = kSub * c;
-                    double acc[2] = { 0.0, 0.0 };
-                    dmma_8x8x8( acc, [&]( int ii, int k ) { return sh.D[o + k][o2 + ii]; }, [&]( int k, int jj ) { return sh.D[o + k][oc + jj]; } );
-                    sh.D[o2 + i8][oc + j8] -= acc[0];
-                    sh.D[o2 + i8][oc + j8 + 1] -= acc[1];
+                    row_tile( o, o1 );
+                    __syncwarp();
+                    asm volatile( "bar.arrive 1, %0;\n" :: "n"(kThreads) : "memory" );
+                    trailing_tile( o, o1, o1 );
+                    __syncwarp();
                 }
+                if( !potrf_diag_tile<T, false>( sh, t, b + 1, nb, arena, status, pivot_floor ) && lane == 0 ) { *sh.redo = 1; }
+            }
+        }
+        else if( b >= 0 )
+        {
+            // the warps that share warp 0's SM sub-partition (warp index mod 4)
+            // take no job, so that the pivot chain does not wait behind one
+            const int first = (warp & 3) == 0 ? INT_MAX : warp - 1 - (warp >> 2);
+            constexpr int kStep = kThreads / 128 * 3;
+            const int rows = rem > 0 ? rem - 1 : 0;
+            for( int job = first; job < rows + b; job += kStep )
+            {
+                if( job < rows ) { row_tile( o, o1 + kSub * (job + 1) ); }
                 else
                 {
-                    // T_ib, i = job - tiles < b
-                    const int oi = kSub * (job - tiles);
+                    const int oi = kSub * (job - rows);
                     double acc[2] = { 0.0, 0.0 };
-                    for( int ok = oi; ok < o; ok += kSub )
+                    dmma_8x8x8( acc, [&]( int ii, int k ) { return sh.Ti[oi + ii][o + k]; }, [&]( int k, int jj ) { return sh.Ti[o + k][o + jj]; } );
+                    __syncwarp();
+                    *reinterpret_cast<double2 *>( &sh.Ti[oi + i8][o + j8] ) = make_double2( -acc[0], -acc[1] );
+                }
+            }
+            if( rem > 0 )
+            {
+                asm volatile( "bar.sync 1, %0;\n" :: "n"(kThreads) : "memory" );
+                const int tiles = rem * (rem + 1) / 2 - 1;              // all but (b+1, b+1)
+                const int jobs = tiles + b + 1;
+                int c = b + 2, left = first;            // a trailing tile's column, and its place in it
+                for( int job = first; job < jobs + (b > 0 ? kSub + nsub : 0); job += kStep )
+                {
+                    if( job >= jobs ) { store_unit( b - 1, job - jobs ); }
+                    else if( job < tiles )
                     {
-                        dmma_8x8x8( acc, [&]( int ii, int kk ) { return sh.Ti[oi + ii][ok + kk]; },
-                                         [&]( int kk, int jj ) { return sh.D[ok + kk][o + jj]; } );
+                        // tile (b + 1 + left, c), column by column of the trailing triangle after (b+1, b+1)
+                        while( left >= c - b ) { left -= c - b; ++c; }
+                        trailing_tile( o, o1 + kSub * left, kSub * c );
+                        left += kStep;
                     }
-                    double (*S)[kPanel + 1] = potrf_scratch( sh );
-                    S[i8][j8] = acc[0];
-                    S[i8][j8 + 1] = acc[1];
-                    __syncwarp();
-                    double acc2[2] = { 0.0, 0.0 };
-                    dmma_8x8x8( acc2, [&]( int ii, int k ) { return S[ii][k]; }, [&]( int k, int jj ) { return sh.Ti[o + k][o + jj]; } );
-                    sh.Ti[oi + i8][o + j8] = -acc2[0];
-                    sh.Ti[oi + i8][o + j8 + 1] = -acc2[1];
-                    __syncwarp();
+                    else
+                    {
+                        // S_i,b+1 into tile (i, b+1) of Ti
+                        const int oi = kSub * (job - tiles);
+                        double acc[2] = { 0.0, 0.0 };
+                        for( int ok = oi; ok <= o; ok += kSub )
+                        {
+                            dmma_8x8x8( acc, [&]( int ii, int kk ) { return sh.Ti[oi + ii][ok + kk]; },
+                                             [&]( int kk, int jj ) { return sh.D[ok + kk][o1 + jj]; } );
+                        }
+                        *reinterpret_cast<double2 *>( &sh.Ti[oi + i8][o1 + j8] ) = make_double2( acc[0], acc[1] );
+                    }
                 }
             }
         }
+        if( b < 0 ) { cp_async_wait_all(); }
         __syncthreads();
-        if( *sh.redo )
+        if constexpr ( sizeof(T) == 4 )
         {
-            // a pivot of tile (b+1, b+1) needed its floor: factor the tile again
-            // now that its row block is complete
-            if( warp == 0 ) { potrf_diag_tile<T>( sh, t, b + 1, nb, arena, status, pivot_floor, false ); }
-            __syncthreads();
-            if( tid == 0 ) { *sh.redo = 0; }
-            __syncthreads();
+            if( *sh.redo )
+            {
+                // a pivot of tile (b+1, b+1) needed its floor: factor the tile again
+                // now that its row block is complete
+                if( warp == 0 ) { potrf_tile_floored<T>( t, b + 1, nb, arena, status, pivot_floor ); }
+                __syncthreads();
+                if( tid == 0 ) { *sh.redo = 0; }
+                __syncthreads();
+            }
         }
     }
-    for( int idx = tid; idx < kPanel * kPanel; idx += kPotrfThreads )
+    for( int u = warp; u < 2 * (kSub + nsub); u += kThreads / 32 )
     {
-        const int r = idx >> 6, c = idx & 63;
-        if( r <= c && c < nb ) { U0[(std::int64_t)r * t.ld0 + c] = static_cast<T>( sh.D[r][c] ); }
+        const bool last = u >= kSub + nsub;
+        if( last || nsub > 1 ) { store_unit( nsub - (last ? 1 : 2), last ? u - kSub - nsub : u ); }
     }
     if( tid == 0 && *sh.fail >= 0 )
     {
         atomicOr( status, 1 );
         atomicMin( status + 1, t.row0 + t.r0 + *sh.fail );
-    }
-    // only the leading nsub x nsub tiles of T are formed (the trsm and the
-    // solves read no more)
-    const int nbp = kSub * nsub;
-    double * out = tinv + (std::int64_t)t.panel * (kPanel * kPanel);
-    for( int idx = tid; idx < nbp * kPanel; idx += kPotrfThreads )
-    {
-        const int r = idx >> 6, c = idx & 63;
-        if( c < nbp ) { out[idx] = (r <= c) ? sh.Ti[r][c] : 0.0; }
     }
 }
 
@@ -762,11 +824,10 @@ __global__ __launch_bounds__(kPotrfThreads, 1) void potrf_kernel( const PanelTas
                                                                const double * __restrict__ pivot_floor,
                                                                double * __restrict__ tinv )
 {
-    extern __shared__ __align__(16) double psm[];
     pdl_allow_next();
     const PanelTask t = tasks[blockIdx.x];
     pdl_wait();
-    potrf_body( t, arena, status, psm, pivot_floor, tinv );
+    potrf_body<T, kPotrfThreads>( t, arena, status, pivot_floor, tinv );
 }
 
 // X = D^{-T} U for the rest columns [c0, c0 + kRestChunk) of a panel (trsm of
@@ -1670,8 +1731,8 @@ __global__ __launch_bounds__(kSolveThreads) void solve_dag_kernel( const SolveDa
 // thread 0 reads counters with ld.acquire.gpu and the CTA synchronises
 // before any thread touches the task's data.
 constexpr int kDagThreads = 256;
-constexpr size_t kDagSmemBytes = kTrsmSmemBytes > kGemmSmemBytes ? kTrsmSmemBytes : kGemmSmemBytes;
-static_assert( kDagSmemBytes >= kPotrfSmemBytes && kDagSmemBytes >= kGemmSmemBytesF, "persistent kernel shared memory too small" );
+constexpr size_t kDagSmemBytes = kPotrfSmemBytes > kGemmSmemBytes ? kPotrfSmemBytes : kGemmSmemBytes;
+static_assert( kDagSmemBytes >= kTrsmSmemBytes && kDagSmemBytes >= kGemmSmemBytesF, "persistent kernel shared memory too small" );
 
 __device__ __forceinline__ int ld_acquire( const int * p )
 {
@@ -1754,7 +1815,7 @@ __global__ __launch_bounds__(kDagThreads, 3) void factor_dag_kernel( const DagAr
         {
             case LaunchKind::Zero:   zero_body( a.zero[t.index], arena ); break;
             case LaunchKind::Extend: extend_body( a.extend[t.index], a.lut, arena ); break;
-            case LaunchKind::Potrf:  potrf_body( a.potrf[t.index], arena, a.status, dsm, a.pivot_floor, a.tinv ); break;
+            case LaunchKind::Potrf:  potrf_body<T, kDagThreads>( a.potrf[t.index], arena, a.status, a.pivot_floor, a.tinv ); break;
             case LaunchKind::Trsm:   trsm_body( a.panel[t.index], arena, a.tinv, dsm ); break;
             case LaunchKind::Gemm:
                 if constexpr ( sizeof(T) == 4 ) { gemm_body( a.gemm[t.index], arena, dsm, tc, a.status ); }
