@@ -155,6 +155,7 @@ struct tb_chol
     DeviceArray<tb::ExtendTask>     extend;
     DeviceArray<tb::ExtendPullTask> extend_pull;
     DeviceArray<tb::ExtendTask>     extend_segs;
+    DeviceArray<tb::FrontTask>      fronts;
     DeviceArray<tb::SolveDiagTask>  sdiag;
     DeviceArray<tb::SolveRestTask>  srest;
     DeviceArray<tb::SuperPanel>     spanels;     // super-panel solve of the large fronts (Plan::spanels)
@@ -394,6 +395,7 @@ int ensure_device( tb_chol * h )
     TB_TRY( h->extend.upload( pl.extend, st_ ) );
     TB_TRY( h->extend_pull.upload( pl.extend_pull, st_ ) );
     TB_TRY( h->extend_segs.upload( pl.extend_segs, st_ ) );
+    TB_TRY( h->fronts.upload( pl.fronts, st_ ) );
     TB_TRY( h->sdiag.upload( pl.sdiag, st_ ) );
     TB_TRY( h->srest.upload( pl.srest, st_ ) );
     TB_TRY( h->spanels.upload( pl.spanels, st_ ) );
@@ -458,6 +460,12 @@ void issue_gemm( tb_chol * h, const tb::Launch & L, T * A, cudaStream_t s )
         tb::launch_gemm( h->gemm.ptr + L.first, L.small_count, A, h->status.ptr, s );
         tb::launch_gemm_tc_tiles( h->tc.ptr + L.tc_first, L.tc_count, A, h->img_map, h->status.ptr, s );
     }
+}
+
+// The level schedule's launches: FP64 takes the small fronts whole.
+const std::vector<tb::Launch> & level_launches( const tb_chol * h )
+{
+    return h->precision == TB_PRECISION_MIXED ? h->plan.factor_launches : h->plan.whole_launches;
 }
 
 // Issues the numeric factorization on h->stream (capturable).  With
@@ -556,12 +564,20 @@ std::int64_t issue_factor_t( tb_chol * h, bool timed, std::vector<int> * kinds )
         cudaStreamWaitEvent( st, h->ev_rest, 0 );
         side_busy = false;
     };
-    for( const tb::Launch & L : pl.factor_launches )
+    for( const tb::Launch & L : level_launches( h ) )
     {
         cudaStream_t s = st;
         if( overlap )
         {
             if( L.level != level ) { join(); level = L.level; }
+            if( L.kind == tb::LaunchKind::Front && L.part == 1 )
+            {
+                // beside the level's other launches, after everything before the level
+                cudaEventRecord( h->ev_trsm, st );
+                cudaStreamWaitEvent( h->side, h->ev_trsm, 0 );
+                s = h->side;
+                side_busy = true;
+            }
             if( L.kind == tb::LaunchKind::Gemm )
             {
                 if( L.part == 0 ) { join(); }
@@ -580,13 +596,20 @@ std::int64_t issue_factor_t( tb_chol * h, bool timed, std::vector<int> * kinds )
             case tb::LaunchKind::ExtendPull:
                 tb::launch_extend_pull( h->extend_pull.ptr + L.first, L.count, h->extend_segs.ptr, h->lut.ptr, A, s );
                 break;
+            case tb::LaunchKind::Front:
+                if constexpr ( sizeof(T) == 8 )
+                {
+                    tb::launch_fronts( h->fronts.ptr + L.first, L.count, L.tc_count, L.small_count, h->extend_segs.ptr, h->lut.ptr, A, h->status.ptr,
+                                       h->tinv.ptr, s );
+                }
+                break;
             case tb::LaunchKind::Potrf:  tb::launch_potrf( h->potrf.ptr + L.first, L.count, A, h->status.ptr, floor, h->tinv.ptr, s ); break;
             case tb::LaunchKind::Trsm:   tb::launch_trsm( h->panel.ptr + L.first, L.count, A, h->tinv.ptr, s, img ); break;
             case tb::LaunchKind::Gemm:   issue_gemm( h, L, A, s ); break;
             default: break;
         }
         if( overlap && L.kind == tb::LaunchKind::Trsm ) { cudaEventRecord( h->ev_trsm, st ); }
-        mark( static_cast<int>( L.kind == tb::LaunchKind::ExtendPull ? tb::LaunchKind::Extend : L.kind ) );
+        mark( static_cast<int>( L.kind == tb::LaunchKind::ExtendPull ? tb::LaunchKind::Extend : L.kind == tb::LaunchKind::Front ? tb::LaunchKind::Solve : L.kind ) );
         ++launches;
     }
     if( overlap ) { join(); }
@@ -617,7 +640,7 @@ int run_factor( tb_chol * h, double reg )
     TB_CUDA( cudaMemcpyAsync( h->reg.ptr, pr, sizeof(double), cudaMemcpyHostToDevice, st ) );
     if( h->profiling )
     {
-        const std::size_t need = h->plan.factor_launches.size() + h->plan.sinv_launches.size() + 2;
+        const std::size_t need = level_launches( h ).size() + h->plan.sinv_launches.size() + 2;
         while( h->events.size() < need )
         {
             cudaEvent_t e;
@@ -2117,7 +2140,7 @@ int tb_chol_plan_stats( tb_chol * h, std::int64_t * out, std::int32_t cap )
     TB_TRY( ensure_symbolic( h ) );
     const tb::Plan & pl = h->plan;
     const std::int64_t v[] = {
-        pl.arena_size(), pl.v_size, pl.levels, static_cast<std::int64_t>( pl.factor_launches.size() ) + 2,
+        pl.arena_size(), pl.v_size, pl.levels, static_cast<std::int64_t>( level_launches( h ).size() ) + 2,
         static_cast<std::int64_t>( pl.gemm.size() ), static_cast<std::int64_t>( pl.panel.size() ),
         static_cast<std::int64_t>( pl.extend.size() ), static_cast<std::int64_t>( pl.lower_launches.size() ),
         static_cast<std::int64_t>( pl.upper_launches.size() ), h->sym.sn_count, pl.front_count,
@@ -2521,14 +2544,16 @@ int tb_chol_launch_profile( tb_chol * h, std::int64_t * info, double * ms, std::
         else if( info )
         {
             // the factor launches, then the super-panel inverse rounds (reported as Invert)
-            const std::size_t nf = h->plan.factor_launches.size();
+            const std::vector<tb::Launch> & list = level_launches( h );
+            const std::size_t nf = list.size();
             const std::size_t j = static_cast<std::size_t>( i - 1 );
-            const tb::Launch * L = j < nf ? &h->plan.factor_launches[j]
+            const tb::Launch * L = j < nf ? &list[j]
                                           : (j - nf < h->plan.sinv_launches.size() ? &h->plan.sinv_launches[j - nf] : nullptr);
             if( L == nullptr ) { info[4 * i] = -1; info[4 * i + 1] = -1; info[4 * i + 2] = -1; info[4 * i + 3] = 0; }
             else
             {
                 const tb::LaunchKind kind = L->kind == tb::LaunchKind::ExtendPull ? tb::LaunchKind::Extend
+                                          : L->kind == tb::LaunchKind::Front ? tb::LaunchKind::Solve
                                           : L->kind == tb::LaunchKind::SuperInv ? tb::LaunchKind::Invert : L->kind;
                 info[4 * i + 0] = static_cast<std::int64_t>( kind );
                 info[4 * i + 1] = L->level;

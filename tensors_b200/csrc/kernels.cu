@@ -406,32 +406,25 @@ constexpr size_t kPotrfSmemBytes = sizeof(double) * (2 * kPanel * kPld + kPanel 
 
 template<typename T> __device__ __forceinline__ double round_to( double v ) { return static_cast<double>( static_cast<T>( v ) ); }
 
-// Panel factorization state, at the start of the kernel's dynamic shared
-// memory.  D: the 64 x 64 block, upper triangle (A, overwritten by U tile row
-// by tile row); Ti: the inverse T = U^{-1}, upper 8 x 8 tiles (the diagonal
-// tiles are zero below the diagonal).
+// Panel factorization state in shared memory.  D: the diagonal block, upper
+// triangle (A, overwritten by U tile row by tile row); Ti: the inverse
+// T = U^{-1}, upper 8 x 8 tiles (the diagonal tiles are zero below the
+// diagonal).  kLd: the leading dimension of both, 0: given at run time.
+template<int kLd>
 struct PotrfShared
 {
-    double (*D)[kPld];
-    double (*Ti)[kPld];
-    double * floor_s;
-    int * fail;
-    int * redo;
-    int * raised;                                       // bit q: tile q has raised pivots (mixed precision)
+    double * d;
+    double * ti;
+    int ldd, ldt;                                       // used when kLd == 0
+    double * floor_s;                                   // the panel's pivot floors (mixed precision)
+    int * flags;                                        // first failing row (-1: none); a tile to factor again; bit q: tile
+                                                        // q has raised pivots (the last two: mixed precision)
+    __device__ __forceinline__ double & D( int r, int c ) const { return d[r * (kLd > 0 ? kLd : ldd) + c]; }
+    __device__ __forceinline__ double & Ti( int r, int c ) const { return ti[r * (kLd > 0 ? kLd : ldt) + c]; }
+    __device__ __forceinline__ int & fail() const { return flags[0]; }
+    __device__ __forceinline__ int & redo() const { return flags[1]; }
+    __device__ __forceinline__ int & raised() const { return flags[2]; }
 };
-
-__device__ __forceinline__ PotrfShared potrf_shared()
-{
-    extern __shared__ __align__(16) double panel_smem[];
-    PotrfShared sh;
-    sh.D = reinterpret_cast<double (*)[kPld]>( panel_smem );
-    sh.Ti = reinterpret_cast<double (*)[kPld]>( panel_smem + kPanel * kPld );
-    sh.floor_s = panel_smem + 2 * kPanel * kPld;        // the panel's pivot floors (mixed precision)
-    sh.fail = reinterpret_cast<int *>( sh.floor_s + kPanel );
-    sh.redo = sh.fail + 1;
-    sh.raised = sh.fail + 2;
-    return sh;
-}
 
 // Cholesky of the diagonal tile q of D by one warp, and W = U_qq^{-1} into
 // tile (q, q) of Ti.  Every lane holds the whole trailing tile in registers
@@ -440,7 +433,9 @@ __device__ __forceinline__ PotrfShared potrf_shared()
 // lane j also carries column j of the identity through the elimination, whose
 // row r is then L^{-1}_rj = W_jr (L = U_qq^T), off the pivot chain.  With FP32 storage U is rounded as it is
 // stored and W inverts the rounded rows (the reciprocal of a stored pivot by
-// one Newton step on the reciprocal square root, r = v (2 - u v)).
+// one Newton step on the reciprocal square root, r = v (2 - u v)); the tile's
+// row block is solved with the pivots before their rounding, by a second
+// inverse kept in the strictly lower tile (7, q) of Ti.
 //
 // A non-positive pivot (FP64) records the first failing row and lets NaNs run
 // on.  kFloored (mixed precision, run again for a tile that met a pivot at or
@@ -452,29 +447,30 @@ __device__ __forceinline__ PotrfShared potrf_shared()
 // pivot under a large row would otherwise make the next pivots of the block
 // hugely negative, floored in turn, until FP32 overflows.  Without kFloored
 // such a tile is left as it was and the function returns false.
-template<typename T, bool kFloored>
-__device__ __forceinline__ bool potrf_diag_tile( const PotrfShared & sh, const PanelTask & t, int q, int nb, const T * __restrict__ arena,
+template<typename T, bool kFloored, int kLd>
+__device__ __forceinline__ bool potrf_diag_tile( const PotrfShared<kLd> & sh, const PanelTask & t, int q, int nb, const T * __restrict__ arena,
                                                  int * __restrict__ status, const double * __restrict__ pivot_floor )
 {
     const int lane = threadIdx.x & 31;
     const int o = kSub * q;
     const unsigned singles = static_cast<unsigned>( (t.single_rows >> o) & 0xff );
-    double a[kSub][kSub], w[kSub];
+    double a[kSub][kSub], w[kSub], w2[kSub];
 #pragma unroll
     for( int r = 0; r < kSub; ++r )
     {
         w[r] = lane == r ? 1.0 : 0.0;
+        w2[r] = w[r];
 #pragma unroll
-        for( int c = r; c < kSub; ++c ) { a[r][c] = sh.D[o + r][o + c]; }
+        for( int c = r; c < kSub; ++c ) { a[r][c] = sh.D( o + r, o + c ); }
     }
     auto store_row = [&]( int r, const double (&v)[kSub] )
     {
         if( lane != 0 ) { return; }
-        if( r & 1 ) { sh.D[o + r][o + r] = v[r]; }
+        if( r & 1 ) { sh.D( o + r, o + r ) = v[r]; }
 #pragma unroll
         for( int c = 0; c < kSub; c += 2 )
         {
-            if( c >= r ) { *reinterpret_cast<double2 *>( &sh.D[o + r][o + c] ) = make_double2( v[c], v[c + 1] ); }
+            if( c >= r ) { *reinterpret_cast<double2 *>( &sh.D( o + r, o + c ) ) = make_double2( v[c], v[c + 1] ); }
         }
     };
     unsigned nonpos = 0u, low = 0u;                     // rows whose pivot is not positive / not above its floor
@@ -495,7 +491,7 @@ __device__ __forceinline__ bool potrf_diag_tile( const PotrfShared & sh, const P
                     double m = 0.0;
 #pragma unroll
                     for( int c = r + 1; c < kSub; ++c ) { m = fmax( m, fabs( a[r][c] ) ); }
-                    for( int c = o + kSub + lane; c < kPanel; c += 32 ) { m = fmax( m, fabs( sh.D[o + r][c] ) ); }
+                    for( int c = o + kSub + lane; c < nb; c += 32 ) { m = fmax( m, fabs( sh.D( o + r, c ) ) ); }
                     const std::int64_t grow = t.r0 + o + r;
                     for( int c = t.r0 + nb + lane; c < t.n0; c += 32 ) { m = fmax( m, fabs( static_cast<double>( arena[t.u0 + grow * t.ld0 + c] ) ) ); }
                     for( int c = lane; c < t.n1; c += 32 ) { m = fmax( m, fabs( static_cast<double>( arena[t.u1 + grow * t.ld1 + c] ) ) ); }
@@ -516,12 +512,14 @@ __device__ __forceinline__ bool potrf_diag_tile( const PotrfShared & sh, const P
 #pragma unroll
         for( int c = r + 1; c < kSub; ++c ) { a[r][c] *= iv; us[c] = round_to<T>( a[r][c] ); }
         w[r] *= iv * fma( -us[r], iv, 2.0 );
+        w2[r] *= iv;
 #pragma unroll
         for( int r2 = r + 1; r2 < kSub; ++r2 )
         {
 #pragma unroll
             for( int c = r2; c < kSub; ++c ) { a[r2][c] -= a[r][r2] * a[r][c]; }
             w[r2] -= us[r2] * w[r];
+            if constexpr ( sizeof(T) == 4 ) { w2[r2] -= us[r2] * w2[r]; }
         }
         // FP64: the row goes out as it is formed, in the shadow of the pivot chain
         if constexpr ( sizeof(T) == 8 ) { store_row( r, us ); }
@@ -537,11 +535,15 @@ __device__ __forceinline__ bool potrf_diag_tile( const PotrfShared & sh, const P
     }
     nonpos &= ~singles;
     if( nb - o < kSub ) { nonpos &= (1u << (nb - o)) - 1u; }
-    if( lane == 0 && nonpos != 0u && *sh.fail < 0 ) { *sh.fail = o + __ffs( nonpos ) - 1; }
+    if( lane == 0 && nonpos != 0u && sh.fail() < 0 ) { sh.fail() = o + __ffs( nonpos ) - 1; }
     if( lane < kSub )
     {
 #pragma unroll
-        for( int i = 0; i < kSub; i += 2 ) { *reinterpret_cast<double2 *>( &sh.Ti[o + lane][o + i] ) = make_double2( w[i], w[i + 1] ); }
+        for( int i = 0; i < kSub; i += 2 )
+        {
+            *reinterpret_cast<double2 *>( &sh.Ti( o + lane, o + i ) ) = make_double2( w[i], w[i + 1] );
+            if( sizeof(T) == 4 && o < kPanel - kSub ) { *reinterpret_cast<double2 *>( &sh.Ti( kPanel - kSub + lane, o + i ) ) = make_double2( w2[i], w2[i + 1] ); }
+        }
     }
     if constexpr ( sizeof(T) == 4 )
     {
@@ -553,112 +555,47 @@ __device__ __forceinline__ bool potrf_diag_tile( const PotrfShared & sh, const P
 }
 
 // The floored factorization of a tile: rare, kept out of the kernel's code.
-template<typename T>
-__device__ __noinline__ void potrf_tile_floored( const PanelTask & t, int q, int nb, const T * __restrict__ arena,
+template<typename T, int kLd>
+__device__ __noinline__ void potrf_tile_floored( const PotrfShared<kLd> sh, const PanelTask & t, int q, int nb, const T * __restrict__ arena,
                                                  int * __restrict__ status, const double * __restrict__ pivot_floor )
 {
-    const PotrfShared sh = potrf_shared();
     potrf_diag_tile<T, true>( sh, t, q, nb, arena, status, pivot_floor );
-    if( (threadIdx.x & 31) == 0 ) { *sh.raised |= 1 << q; }
+    if( (threadIdx.x & 31) == 0 ) { sh.raised() |= 1 << q; }
 }
 
 // U_bc = U_bb^{-T} A_bc for tile (b, c) of D (tile corners o, oc), one column per lane.
-template<typename T>
-__device__ __noinline__ void potrf_row_substitution( int o, int oc )
+template<typename T, int kLd>
+__device__ __noinline__ void potrf_row_substitution( const PotrfShared<kLd> sh, int o, int oc )
 {
-    const PotrfShared sh = potrf_shared();
     const int lane = threadIdx.x & 31;
     if( lane < kSub )
     {
         double x[kSub];
 #pragma unroll
-        for( int r = 0; r < kSub; ++r ) { x[r] = sh.D[o + r][oc + lane]; }
+        for( int r = 0; r < kSub; ++r ) { x[r] = sh.D( o + r, oc + lane ); }
 #pragma unroll
         for( int r = 0; r < kSub; ++r )
         {
-            x[r] /= sh.D[o + r][o + r];
+            x[r] *= sh.Ti( kPanel - kSub + r, o + r );      // the pivot's reciprocal
 #pragma unroll
-            for( int r2 = r + 1; r2 < kSub; ++r2 ) { x[r2] -= sh.D[o + r][o + r2] * x[r]; }
+            for( int r2 = r + 1; r2 < kSub; ++r2 ) { x[r2] -= sh.D( o + r, o + r2 ) * x[r]; }
         }
 #pragma unroll
-        for( int r = 0; r < kSub; ++r ) { sh.D[o + r][oc + lane] = round_to<T>( x[r] ); }
+        for( int r = 0; r < kSub; ++r ) { sh.D( o + r, oc + lane ) = round_to<T>( x[r] ); }
     }
 }
 
-// Cholesky of one panel's 64 x 64 diagonal block D (identity beyond nb) and
-// the inverse T = D^{-1} of its factor (LAPACK potrf of FactorizeSupernode,
-// Multifrontal.hpp:438-449, plus the inverse the panel's trsm and the solves
-// use), right-looking by 8 x 8 tiles.  The bound is the chain of 64 pivots
-// (~93 cycles each), so warp 0 runs only that chain: per tile step b it forms
-// U_b,b+1 = W_b^T A_b,b+1 (W_b = U_bb^{-1}, left by the tile's
-// factorization), updates tile (b+1, b+1) and factors it.  Meanwhile the
-// other warps
-//   1. form U_bc = W_b^T A_bc for c > b+1 and T_ib = -S_ib W_b for i < b, and
-//   2. (behind a barrier that warp 0 passes without waiting) update the other
-//      trailing tiles, and sum S_i,b+1 = sum_{k=i..b} T_ik U_k,b+1; then
-//      they write out what step b-1 finished,
-// one 8 x 8 tile per warp and job, each a few DMMA m8n8k4; one full barrier
-// ends the step.  After the last tile only T's last column is left.  A row
-// that forms a 1 x 1 reference supernode takes sqrt(|a|) as the reference
-// does (:471) and never reports failure.  With FP32 storage every U value is
-// rounded to FP32 as it is formed, so the in-panel updates, W and T use the
-// stored factor (T inverts it), as the updates of later panels do.
-// kThreads: 384 in the level launches, 256 in the persistent kernel.
-template<typename T, int kThreads>
-__device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict__ arena, int * __restrict__ status,
-                                            const double * __restrict__ pivot_floor, double * __restrict__ tinv )
+// kThreads: 384 in the panel launches and the larger small fronts, 128 in the
+// smaller ones, 256 in the persistent kernel.  The block (nb x nb, identity beyond
+// up to a multiple of 8) is in sh.D; pending: its cp.async copies may still be
+// in flight except tile 0's rows.  U goes to the arena, T to tinv.
+template<typename T, int kThreads, int kLd>
+__device__ __forceinline__ void potrf_core( const PotrfShared<kLd> & sh, const PanelTask & t, int nb, T * __restrict__ arena,
+                                            int * __restrict__ status, const double * __restrict__ pivot_floor, double * __restrict__ tinv )
 {
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
-    const int nb = min( kPanel, t.n0 - t.r0 );
-    const PotrfShared sh = potrf_shared();
-
     T * U0 = arena + t.u0 + (std::int64_t)t.r0 * t.ld0 + t.r0;
-    // 16-byte pieces of the rows (16-byte aligned: offsets and leading dimensions are multiples of
-    // kLdAlign entries), all of a thread's in flight together; pieces below the diagonal are not read
-    // later and not loaded; identity padding beyond nb
-    constexpr int kV = 16 / static_cast<int>( sizeof(T) );
-    constexpr int kAll = kPanel * kPanel / kV, kPieces = (kAll + kThreads - 1) / kThreads;
-    if constexpr ( sizeof(T) == 8 )
-    {
-#pragma unroll
-        for( int u = 0; u < kPieces; ++u )
-        {
-            const int idx = kV * (tid + u * kThreads), r = idx / kPanel, c = idx % kPanel;
-            if( r >= kPanel ) {}
-            else if( r >= nb ) { sh.D[r][c] = r == c ? 1.0 : 0.0; sh.D[r][c + 1] = r == c + 1 ? 1.0 : 0.0; }
-            else if( c + 1 >= r ) { cp_async_16( &sh.D[r][c], c < nb ? U0 + (std::int64_t)r * t.ld0 + c : U0, c + 1 < nb ? 16 : c < nb ? 8 : 0 ); }
-            if( u == 0 ) { cp_async_commit(); }         // the first rows: tile 0 starts when they are in
-        }
-        cp_async_commit();
-    }
-    else
-    {
-        float4 v[kPieces];
-#pragma unroll
-        for( int u = 0; u < kPieces; ++u )
-        {
-            const int idx = kV * (tid + u * kThreads), r = idx / kPanel, c = idx % kPanel;
-            v[u] = make_float4( 0.f, 0.f, 0.f, 0.f );
-            if( r < nb && c < nb && c + 3 >= r ) { v[u] = *reinterpret_cast<const float4 *>( U0 + (std::int64_t)r * t.ld0 + c ); }
-        }
-#pragma unroll
-        for( int u = 0; u < kPieces; ++u )
-        {
-            const int idx = kV * (tid + u * kThreads), r = idx / kPanel, c = idx % kPanel;
-            if( r >= kPanel ) { continue; }
-            const double pad = r >= nb ? 1.0 : 0.0;
-            const float f[4] = { v[u].x, v[u].y, v[u].z, v[u].w };
-#pragma unroll
-            for( int e = 0; e < 4; ++e ) { sh.D[r][c + e] = r < nb && c + e < nb ? static_cast<double>( f[e] ) : r == c + e ? pad : 0.0; }
-        }
-    }
-    // the pivot floors after the block's copies are in flight (their loads overlap)
-    if( pivot_floor != nullptr && tid < nb ) { sh.floor_s[tid] = pivot_floor[1 + t.row0 + t.r0 + tid]; }
-    if( tid == 0 ) { *sh.fail = -1; *sh.redo = 0; *sh.raised = 0; }
-    cp_async_wait<1>();
-    __syncthreads();
-
     const int nsub = (nb + kSub - 1) / kSub;
     const int i8 = lane >> 2, j8 = 2 * (lane & 3);        // this lane's entries of an 8 x 8 DMMA result
     // U_bc = W_b^T A_bc in place (tile (b, c) of D), rounded to the storage type.  Mixed precision,
@@ -668,25 +605,26 @@ __device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict_
     {
         if constexpr ( sizeof(T) == 4 )
         {
-            if( (sh.raised[0] >> (o / kSub)) & 1 )
+            if( (sh.raised() >> (o / kSub)) & 1 )
             {
-                potrf_row_substitution<T>( o, oc );
+                potrf_row_substitution<T>( sh, o, oc );
                 return;
             }
         }
+        const int ow = sizeof(T) == 4 ? kPanel - kSub : o;
         double acc[2] = { 0.0, 0.0 };
-        dmma_8x8x8( acc, [&]( int ii, int k ) { return sh.Ti[o + k][o + ii]; }, [&]( int k, int jj ) { return sh.D[o + k][oc + jj]; } );
+        dmma_8x8x8( acc, [&]( int ii, int k ) { return sh.Ti( ow + k, o + ii ); }, [&]( int k, int jj ) { return sh.D( o + k, oc + jj ); } );
         __syncwarp();
-        *reinterpret_cast<double2 *>( &sh.D[o + i8][oc + j8] ) = make_double2( round_to<T>( acc[0] ), round_to<T>( acc[1] ) );
+        *reinterpret_cast<double2 *>( &sh.D( o + i8, oc + j8 ) ) = make_double2( round_to<T>( acc[0] ), round_to<T>( acc[1] ) );
     };
     // tile (r, c) of D -= U_b,r^T U_b,c (summed apart and subtracted once: one rounding at the tile's
     // own magnitude per step)
     auto trailing_tile = [&]( int o, int orow, int oc )
     {
-        double2 * d = reinterpret_cast<double2 *>( &sh.D[orow + i8][oc + j8] );
+        double2 * d = reinterpret_cast<double2 *>( &sh.D( orow + i8, oc + j8 ) );
         const double2 v = *d;
         double acc[2] = { 0.0, 0.0 };
-        dmma_8x8x8( acc, [&]( int ii, int k ) { return sh.D[o + k][orow + ii]; }, [&]( int k, int jj ) { return sh.D[o + k][oc + jj]; } );
+        dmma_8x8x8( acc, [&]( int ii, int k ) { return sh.D( o + k, orow + ii ); }, [&]( int k, int jj ) { return sh.D( o + k, oc + jj ); } );
         *d = make_double2( v.x - acc[0], v.y - acc[1] );
     };
     // What step b finished, to global memory, in kSub + nsub units of 32 threads: U's row u of tile
@@ -700,8 +638,8 @@ __device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict_
         if( u < kSub )
         {
             const int r = o + u, c = 2 * lane;
-            if( r >= nb ) { return; }
-            const double2 v = *reinterpret_cast<const double2 *>( &sh.D[r][c] );
+            if( r >= nb || c >= nb ) { return; }
+            const double2 v = *reinterpret_cast<const double2 *>( &sh.D( r, c ) );
             T * dst = U0 + (std::int64_t)r * t.ld0 + c;
             if( r <= c && c + 1 < nb )
             {
@@ -710,14 +648,14 @@ __device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict_
             }
             else
             {
-                if( r <= c && c < nb ) { dst[0] = static_cast<T>( v.x ); }
+                if( r <= c ) { dst[0] = static_cast<T>( v.x ); }
                 if( r <= c + 1 && c + 1 < nb ) { dst[1] = static_cast<T>( v.y ); }
             }
         }
         else
         {
             const int r = kSub * (u - kSub) + (lane >> 2), c = o + 2 * (lane & 3);
-            const double2 v = *reinterpret_cast<const double2 *>( &sh.Ti[r][c] );
+            const double2 v = *reinterpret_cast<const double2 *>( &sh.Ti( r, c ) );
             *reinterpret_cast<double2 *>( out + r * kPanel + c ) = r < o + kSub ? v : make_double2( 0.0, 0.0 );
         }
     };
@@ -738,7 +676,7 @@ __device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict_
                     trailing_tile( o, o1, o1 );
                     __syncwarp();
                 }
-                if( !potrf_diag_tile<T, false>( sh, t, b + 1, nb, arena, status, pivot_floor ) && lane == 0 ) { *sh.redo = 1; }
+                if( !potrf_diag_tile<T, false>( sh, t, b + 1, nb, arena, status, pivot_floor ) && lane == 0 ) { sh.redo() = 1; }
             }
         }
         else if( b >= 0 )
@@ -755,9 +693,9 @@ __device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict_
                 {
                     const int oi = kSub * (job - rows);
                     double acc[2] = { 0.0, 0.0 };
-                    dmma_8x8x8( acc, [&]( int ii, int k ) { return sh.Ti[oi + ii][o + k]; }, [&]( int k, int jj ) { return sh.Ti[o + k][o + jj]; } );
+                    dmma_8x8x8( acc, [&]( int ii, int k ) { return sh.Ti( oi + ii, o + k ); }, [&]( int k, int jj ) { return sh.Ti( o + k, o + jj ); } );
                     __syncwarp();
-                    *reinterpret_cast<double2 *>( &sh.Ti[oi + i8][o + j8] ) = make_double2( -acc[0], -acc[1] );
+                    *reinterpret_cast<double2 *>( &sh.Ti( oi + i8, o + j8 ) ) = make_double2( -acc[0], -acc[1] );
                 }
             }
             if( rem > 0 )
@@ -783,10 +721,10 @@ __device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict_
                         double acc[2] = { 0.0, 0.0 };
                         for( int ok = oi; ok <= o; ok += kSub )
                         {
-                            dmma_8x8x8( acc, [&]( int ii, int kk ) { return sh.Ti[oi + ii][ok + kk]; },
-                                             [&]( int kk, int jj ) { return sh.D[ok + kk][o1 + jj]; } );
+                            dmma_8x8x8( acc, [&]( int ii, int kk ) { return sh.Ti( oi + ii, ok + kk ); },
+                                             [&]( int kk, int jj ) { return sh.D( ok + kk, o1 + jj ); } );
                         }
-                        *reinterpret_cast<double2 *>( &sh.Ti[oi + i8][o1 + j8] ) = make_double2( acc[0], acc[1] );
+                        *reinterpret_cast<double2 *>( &sh.Ti( oi + i8, o1 + j8 ) ) = make_double2( acc[0], acc[1] );
                     }
                 }
             }
@@ -795,13 +733,13 @@ __device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict_
         __syncthreads();
         if constexpr ( sizeof(T) == 4 )
         {
-            if( *sh.redo )
+            if( sh.redo() )
             {
                 // a pivot of tile (b+1, b+1) needed its floor: factor the tile again
                 // now that its row block is complete
-                if( warp == 0 ) { potrf_tile_floored<T>( t, b + 1, nb, arena, status, pivot_floor ); }
+                if( warp == 0 ) { potrf_tile_floored<T>( sh, t, b + 1, nb, arena, status, pivot_floor ); }
                 __syncthreads();
-                if( tid == 0 ) { *sh.redo = 0; }
+                if( tid == 0 ) { sh.redo() = 0; }
                 __syncthreads();
             }
         }
@@ -811,11 +749,75 @@ __device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict_
         const bool last = u >= kSub + nsub;
         if( last || nsub > 1 ) { store_unit( nsub - (last ? 1 : 2), last ? u - kSub - nsub : u ); }
     }
-    if( tid == 0 && *sh.fail >= 0 )
+    if( tid == 0 && sh.fail() >= 0 )
     {
         atomicOr( status, 1 );
-        atomicMin( status + 1, t.row0 + t.r0 + *sh.fail );
+        atomicMin( status + 1, t.row0 + t.r0 + sh.fail() );
     }
+}
+
+// The panel's diagonal block (64 x kPld cells of dynamic shared memory), then potrf_core.
+template<typename T, int kThreads>
+__device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict__ arena, int * __restrict__ status,
+                                            const double * __restrict__ pivot_floor, double * __restrict__ tinv )
+{
+    extern __shared__ __align__(16) double panel_smem[];
+    const int tid = threadIdx.x;
+    const int nb = min( kPanel, t.n0 - t.r0 );
+    PotrfShared<kPld> sh;
+    sh.d = panel_smem;
+    sh.ti = panel_smem + kPanel * kPld;
+    sh.ldd = sh.ldt = kPld;
+    sh.floor_s = panel_smem + 2 * kPanel * kPld;
+    sh.flags = reinterpret_cast<int *>( sh.floor_s + kPanel );
+
+    T * U0 = arena + t.u0 + (std::int64_t)t.r0 * t.ld0 + t.r0;
+    // 16-byte pieces of the rows (16-byte aligned: offsets and leading dimensions are multiples of
+    // kLdAlign entries), all of a thread's in flight together; pieces below the diagonal are not read
+    // later and not loaded; identity padding beyond nb
+    constexpr int kV = 16 / static_cast<int>( sizeof(T) );
+    constexpr int kAll = kPanel * kPanel / kV, kPieces = (kAll + kThreads - 1) / kThreads;
+    if constexpr ( sizeof(T) == 8 )
+    {
+#pragma unroll
+        for( int u = 0; u < kPieces; ++u )
+        {
+            const int idx = kV * (tid + u * kThreads), r = idx / kPanel, c = idx % kPanel;
+            if( r >= kPanel ) {}
+            else if( r >= nb ) { sh.D( r, c ) = r == c ? 1.0 : 0.0; sh.D( r, c + 1 ) = r == c + 1 ? 1.0 : 0.0; }
+            else if( c + 1 >= r ) { cp_async_16( &sh.D( r, c ), c < nb ? U0 + (std::int64_t)r * t.ld0 + c : U0, c + 1 < nb ? 16 : c < nb ? 8 : 0 ); }
+            if( u == 0 ) { cp_async_commit(); }         // the first rows: tile 0 starts when they are in
+        }
+        cp_async_commit();
+    }
+    else
+    {
+        float4 v[kPieces];
+#pragma unroll
+        for( int u = 0; u < kPieces; ++u )
+        {
+            const int idx = kV * (tid + u * kThreads), r = idx / kPanel, c = idx % kPanel;
+            v[u] = make_float4( 0.f, 0.f, 0.f, 0.f );
+            if( r < nb && c < nb && c + 3 >= r ) { v[u] = *reinterpret_cast<const float4 *>( U0 + (std::int64_t)r * t.ld0 + c ); }
+        }
+#pragma unroll
+        for( int u = 0; u < kPieces; ++u )
+        {
+            const int idx = kV * (tid + u * kThreads), r = idx / kPanel, c = idx % kPanel;
+            if( r >= kPanel ) { continue; }
+            const double pad = r >= nb ? 1.0 : 0.0;
+            const float f[4] = { v[u].x, v[u].y, v[u].z, v[u].w };
+#pragma unroll
+            for( int e = 0; e < 4; ++e ) { sh.D( r, c + e ) = r < nb && c + e < nb ? static_cast<double>( f[e] ) : r == c + e ? pad : 0.0; }
+        }
+    }
+    // the pivot floors after the block's copies are in flight (their loads overlap)
+    if( pivot_floor != nullptr && tid < nb ) { sh.floor_s[tid] = pivot_floor[1 + t.row0 + t.r0 + tid]; }
+    if( tid == 0 ) { sh.fail() = -1; sh.redo() = 0; sh.raised() = 0; }
+    cp_async_wait<1>();
+    __syncthreads();
+
+    potrf_core<T, kThreads>( sh, t, nb, arena, status, pivot_floor, tinv );
 }
 
 template<typename T>
@@ -828,6 +830,236 @@ __global__ __launch_bounds__(kPotrfThreads, 1) void potrf_kernel( const PanelTas
     const PanelTask t = tasks[blockIdx.x];
     pdl_wait();
     potrf_body<T, kPotrfThreads>( t, arena, status, pivot_floor, tinv );
+}
+
+// ------------------------------------------------------------ small fronts
+// A whole front with at most one panel of pivot rows (FrontTask) in one CTA's
+// shared memory: assembled rows, children added in rank order, potrf, rest
+// columns, update matrix.  The operations on each entry are those of the
+// separate launches in the same order (FP64: the same factor bit for bit),
+// without their passes over the front in global memory: zeroing, one
+// read-modify-write per child and one for the update, the rest columns
+// written and read back.  Blocks of a few dozen rows leave the bound to
+// latencies (the children's rows, the pivot chain), so what counts is CTAs
+// per SM and warps per CTA: the plan picks 128, 256 or 384 threads (three,
+// two, one CTA per SM) by the launch's front count and shared memory.
+//
+// The update matrix is kept by blocks of 8 rows from the diagonal on.  FP64
+// storage only.
+__device__ __forceinline__ int front_v_row( int n1p, int row )
+{
+    const int rb = row >> 3, width = n1p - 8 * rb;
+    return 8 * (rb * n1p - 4 * rb * (rb - 1)) + (row & 7) * width - 8 * rb;      // + column
+}
+
+template<int kThreads>
+__global__ __launch_bounds__(kThreads, kThreads == 128 ? 3 : kThreads == 256 ? 2 : 1)
+void front_kernel( const FrontTask * __restrict__ tasks, const ExtendTask * __restrict__ segs, const std::int32_t * __restrict__ lut_all,
+                   double * __restrict__ arena, int * __restrict__ status, double * __restrict__ tinv )
+{
+    extern __shared__ __align__(16) double fsm[];
+    pdl_allow_next();
+    const FrontTask ft = tasks[blockIdx.x];
+    const PanelTask & t = ft.p;
+    constexpr int kWarps = kThreads / 32;
+    constexpr int kV = 2;                                 // entries of a 16-byte piece
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n0 = t.n0, n1 = t.n1;
+    const int n0p = (n0 + 7) & ~7, n1p = (n1 + 7) & ~7;
+    PotrfShared<0> sh;
+    sh.ldd = n0p + n1p + 4;
+    sh.ldt = n0p + 4;
+    sh.d = fsm;
+    sh.ti = sh.d + n0p * sh.ldd;
+    double * V = sh.ti + n0p * sh.ldt;
+    sh.floor_s = V + 4 * n1p * (n1p / 8 + 1);
+    sh.flags = reinterpret_cast<int *>( sh.floor_s + kPanel );
+    double * X = sh.d + n0p;                              // rest columns, rows sh.ldd apart
+    const int ldx = sh.ldd;
+
+    if( ft.has_v ) { for( int e = 2 * tid; e < 4 * n1p * (n1p / 8 + 1); e += 2 * kThreads ) { *reinterpret_cast<double2 *>( V + e ) = make_double2( 0.0, 0.0 ); } }
+    if( tid == 0 ) { sh.fail() = -1; sh.redo() = 0; sh.raised() = 0; }
+    pdl_wait();
+    // the assembled rows: diagonal block (identity beyond n0; below the diagonal not read later), rest columns
+    {
+        const double * U0 = arena + t.u0;
+        const double * U1 = arena + t.u1;
+        // 16-byte pieces: a lane keeps its columns and steps over the warp's rows
+        const int per0 = n0p / kV, per = (n0p + n1p) / kV;
+        for( int q = lane; q < per; q += 32 )
+        {
+            const bool diag = q < per0;
+            const int c = kV * (diag ? q : q - per0), lim = diag ? n0 : n1;
+            const int ld = diag ? t.ld0 : t.ld1;
+            const double * src = (diag ? U0 : U1) + c + (std::int64_t)warp * ld;
+            double * dst = sh.d + warp * ldx + kV * q;
+            const int rows = c < lim ? min( n0, diag ? c + kV : n0 ) : 0;      // rows with entries of these columns
+            const int bytes = c + 1 < lim ? 16 : 8;
+#pragma unroll 2
+            for( int r = warp; r < n0p; r += kWarps, src += (std::int64_t)kWarps * ld, dst += kWarps * ldx )
+            {
+                if( r < rows ) { cp_async_16( dst, src, bytes ); }
+                else if( r >= n0 || c >= lim ) { *reinterpret_cast<double2 *>( dst ) = make_double2( diag && r == c ? 1.0 : 0.0, diag && r == c + 1 ? 1.0 : 0.0 ); }
+            }
+        }
+        cp_async_wait_all();
+    }
+    __syncthreads();
+    // children, one after the other (a barrier between two).  A warp's unit is kRows rows of a
+    // 32-column chunk of the child's upper triangle; the next unit's loads (the next child's first
+    // unit too) are in flight while this one is added, so that a child costs its additions and not
+    // a round trip to memory (two columns per lane measured the same: the pairs' shared-memory
+    // conflicts cost what the shared address arithmetic saves).
+    constexpr int kRows = 8, kSegs = 16;
+    struct Seg { const double * W; const std::int32_t * lut; int m1, mid, ldw; };
+    __shared__ Seg seg_s[kSegs];
+    // v: the unit's entries; li: lane u's row position in the parent (u < kRows); lj: the lane's column
+    struct Unit { double v[kRows]; int li; int lj; };
+    const int v0 = static_cast<int>( V - sh.d );
+    for( int g0 = 0; g0 < ft.seg_count; g0 += kSegs )
+    {
+        const int ng = min( kSegs, ft.seg_count - g0 );
+        if( g0 > 0 ) { __syncthreads(); }
+        if( tid < ng )
+        {
+            const ExtendTask & e = segs[ft.seg_first + g0 + tid];
+            seg_s[tid] = { arena + e.w, lut_all + e.lut, e.m1, e.mid, e.ldw };
+        }
+        __syncthreads();
+        auto load = [&]( Unit & un, int g, int j0, int i0 )
+        {
+            const Seg & e = seg_s[g];
+            const int j = j0 + lane, il = i0 + (lane & (kRows - 1)) * kWarps;
+            un.lj = j < e.m1 ? e.lut[j] : 0;
+            un.li = il < e.m1 ? e.lut[il] : 0;
+            const double * w = e.W + (std::int64_t)i0 * e.ldw + j;
+            const std::int64_t step = static_cast<std::int64_t>( kWarps ) * e.ldw;
+            const int last = j < e.m1 ? j - i0 : -1;
+#pragma unroll
+            for( int u = 0; u < kRows; ++u ) { un.v[u] = u * kWarps <= last ? w[u * step] : 0.0; }
+        };
+        Unit cur;
+        int g = 0, j0 = 0, i0 = warp;
+        load( cur, 0, 0, i0 );
+        while( g < ng )
+        {
+            const int m1 = seg_s[g].m1, mid = seg_s[g].mid;
+            // the following unit
+            int gn = g, jn = j0, in = i0 + kRows * kWarps;
+            if( in >= min( m1, j0 + 32 ) ) { jn += 32; in = warp; }
+            if( jn >= m1 ) { ++gn; jn = 0; }
+            Unit nxt;
+            if( gn < ng ) { load( nxt, gn, jn, in ); }
+            // offsets of the unit's rows from sh.d: lane u forms row u's, the others take it from there
+            const bool pivot_row = i0 + (lane & (kRows - 1)) * kWarps < mid;
+            const int base = pivot_row ? cur.li * ldx : v0 + front_v_row( n1p, cur.li );
+            const int j = j0 + lane, last = j < m1 ? j - i0 : -1;
+            const int cp = cur.lj + (j < mid ? 0 : n0p);                  // the column in a pivot row
+            double * dst[kRows];
+            double x[kRows];
+#pragma unroll
+            for( int u = 0; u < kRows; ++u )
+            {
+                const int row = __shfl_sync( 0xffffffffu, base, u );
+                dst[u] = sh.d + row + (i0 + u * kWarps < mid ? cp : cur.lj);
+                x[u] = u * kWarps <= last ? *dst[u] : 0.0;
+            }
+#pragma unroll
+            for( int u = 0; u < kRows; ++u )
+            {
+                if( u * kWarps <= last ) { *dst[u] = x[u] + cur.v[u]; }
+            }
+            if( gn != g ) { __syncthreads(); }
+            cur = nxt;
+            g = gn; j0 = jn; i0 = in;
+        }
+    }
+    potrf_core<double, kThreads>( sh, t, n0, arena, status, nullptr, tinv );
+    if( n1 == 0 ) { return; }
+    // rest columns X <- T^T X in place: a warp takes all row blocks of an 8-column tile
+    const int nsub = n0p / kSub, n1t = n1p / kSub;
+    const int fi = lane >> 2, fj = 2 * (lane & 3);
+    for( int ct = warp; ct < n1t; ct += kWarps )
+    {
+        double acc[kSubs][2];
+#pragma unroll
+        for( int rb = 0; rb < kSubs; ++rb ) { acc[rb][0] = 0.0; acc[rb][1] = 0.0; }
+#pragma unroll
+        for( int kb = 0; kb < kSubs; ++kb )
+        {
+            if( kb >= nsub ) { break; }
+            double b[2];
+#pragma unroll
+            for( int q = 0; q < 2; ++q ) { b[q] = X[(kSub * kb + (lane & 3) + 4 * q) * ldx + kSub * ct + fi]; }
+#pragma unroll
+            for( int rb = kb; rb < kSubs; ++rb )
+            {
+                if( rb >= nsub ) { break; }
+#pragma unroll
+                for( int q = 0; q < 2; ++q ) { dmma_8x8x4( acc[rb], sh.Ti( kSub * kb + (lane & 3) + 4 * q, kSub * rb + fi ), b[q] ); }
+            }
+        }
+        __syncwarp();
+        const int c = kSub * ct + fj;
+#pragma unroll
+        for( int rb = 0; rb < kSubs; ++rb )
+        {
+            if( rb >= nsub ) { break; }
+            const int r = kSub * rb + fi;
+            const double2 x = make_double2( acc[rb][0], acc[rb][1] );
+            *reinterpret_cast<double2 *>( X + r * ldx + c ) = x;
+            if( r < n0 && c < n1 )
+            {
+                // (a row's padding takes the tile's zero column: rows are padded to four entries)
+                double * dst = arena + t.u1 + (std::int64_t)r * t.ld1 + c;
+                *reinterpret_cast<double2 *>( dst ) = x;
+            }
+        }
+    }
+    if( !ft.has_v ) { return; }
+    __syncthreads();
+    // update matrix V - X^T X, 16 x 16 blocks of its upper triangle round the warps
+    const int nm = (n1t + 1) / 2;
+    int I = 0, J = warp;
+    while( I < nm )
+    {
+        if( J >= nm ) { J = J - nm + I + 1; ++I; if( I >= nm || J >= nm ) { continue; } }
+        double acc[2][2][2];
+#pragma unroll
+        for( int a = 0; a < 2; ++a )
+        {
+#pragma unroll
+            for( int b = 0; b < 2; ++b ) { acc[a][b][0] = 0.0; acc[a][b][1] = 0.0; }
+        }
+        const int r0 = 16 * I, c0 = 16 * J;
+        const int r1 = r0 + 8 < n1p ? r0 + 8 : r0, c1 = c0 + 8 < n1p ? c0 + 8 : c0;     // (a missing half repeats the first)
+#pragma unroll 4
+        for( int k = lane & 3; k < n0p; k += 4 )
+        {
+            const double * x = X + k * ldx + fi;
+            const double a0 = x[r0], a1 = x[r1], b0 = x[c0], b1 = x[c1];
+            dmma_8x8x4( acc[0][0], a0, b0 );
+            dmma_8x8x4( acc[0][1], a0, b1 );
+            dmma_8x8x4( acc[1][0], a1, b0 );
+            dmma_8x8x4( acc[1][1], a1, b1 );
+        }
+#pragma unroll
+        for( int a = 0; a < 2; ++a )
+        {
+#pragma unroll
+            for( int b = 0; b < 2; ++b )
+            {
+                const int row = r0 + 8 * a + fi, col = c0 + 8 * b + fj;
+                if( row >= n1 || col >= n1 || (I == J && a > b) ) { continue; }
+                const double2 v = *reinterpret_cast<const double2 *>( V + front_v_row( n1p, row ) + col );
+                const double x0 = v.x - acc[a][b][0], x1 = v.y - acc[a][b][1];
+                double * dst = arena + ft.v + (std::int64_t)row * t.ld1 + col;
+                if( row <= col ) { *reinterpret_cast<double2 *>( dst ) = make_double2( x0, x1 ); }
+                else if( row == col + 1 ) { dst[1] = x1; }
+            }
+        }
+        J += kWarps;
+    }
 }
 
 // X = D^{-T} U for the rest columns [c0, c0 + kRestChunk) of a panel (trsm of
@@ -2450,6 +2682,18 @@ void launch_extend_pull( const ExtendPullTask * tasks, int count, const ExtendTa
     if( count > 0 ) { launch_pdl( extend_pull_kernel<T>, count, 256, 0, st, tasks, segs, lut, arena ); }
 }
 
+void launch_fronts( const FrontTask * tasks, int count, int threads, int smem, const ExtendTask * segs, const std::int32_t * lut, double * arena,
+                    int * status, double * tinv, cudaStream_t st )
+{
+    if( count <= 0 ) { return; }
+    switch( threads )
+    {
+        case 128: launch_pdl( front_kernel<128>, count, 128, smem, st, tasks, segs, lut, arena, status, tinv ); break;
+        case 256: launch_pdl( front_kernel<256>, count, 256, smem, st, tasks, segs, lut, arena, status, tinv ); break;
+        default:  launch_pdl( front_kernel<384>, count, 384, smem, st, tasks, segs, lut, arena, status, tinv ); break;
+    }
+}
+
 template<typename T>
 void launch_potrf( const PanelTask * tasks, int count, T * arena, int * status, const double * pivot_floor, double * tinv,
                    cudaStream_t st )
@@ -2710,6 +2954,9 @@ void launch_residual( int n, const std::int64_t * outer, const std::int32_t * in
 cudaError_t configure_kernels()
 {
     const struct { const void * fn; size_t bytes; } attrs[] = {
+        { reinterpret_cast<const void *>( front_kernel<128> ), kFrontSmemSmall },
+        { reinterpret_cast<const void *>( front_kernel<256> ), kFrontSmemMid },
+        { reinterpret_cast<const void *>( front_kernel<384> ), kFrontSmemMax },
         { reinterpret_cast<const void *>( potrf_kernel<double> ), kPotrfSmemBytes },
         { reinterpret_cast<const void *>( potrf_kernel<float> ), kPotrfSmemBytes },
         { reinterpret_cast<const void *>( trsm_kernel<double> ), kTrsmSmemBytes },

@@ -28,6 +28,10 @@ template<typename T> void launch_extend( const ExtendTask * tasks, int count, co
 template<typename T>
 void launch_extend_pull( const ExtendPullTask * tasks, int count, const ExtendTask * segs, const std::int32_t * lut, T * arena,
                          cudaStream_t st );
+// Small fronts taken whole (plan.hpp, FrontTask), FP64 storage: threads (128, 256 or 384) and smem
+// bytes per CTA; the other arguments as launch_extend_pull's and launch_potrf's.
+void launch_fronts( const FrontTask * tasks, int count, int threads, int smem, const ExtendTask * segs, const std::int32_t * lut, double * arena,
+                    int * status, double * tinv, cudaStream_t st );
 // pivot_floor (mixed precision only, else null): element 0 the largest |a_ii|,
 // element 1 + i the value a non-positive or lost pivot of permuted row i is
 // raised to instead of failing; status[2] counts them.

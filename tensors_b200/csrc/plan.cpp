@@ -381,6 +381,20 @@ void Plan::build( const Symbolic & sym )
         }
     }
 
+    // ------------------------------------------------ small fronts
+    front_small.assign( static_cast<size_t>(F), 0 );
+    for( I32 h = 0; h < levels; ++h )
+    {
+        auto fits = [&]( I32 f ) { return front_n0[f] <= kPanel && front_smem_bytes( front_n0[f], front_n1[f] ) <= kFrontSmemMax; };
+        I64 count = 0;
+        for( I32 f : by_level[h] ) { count += fits( f ) ? 1 : 0; }
+        if( 2 * count < static_cast<I64>( by_level[h].size() ) ) { continue; }
+        for( I32 f : by_level[h] ) { front_small[static_cast<size_t>(f)] = fits( f ) ? 1 : 0; }
+        // the small ones last: the other launches' tasks are then contiguous
+        std::stable_partition( by_level[h].begin(), by_level[h].end(), [&]( I32 f ) { return !front_small[static_cast<size_t>(f)]; } );
+    }
+    fronts.clear();
+
     // ------------------------------------------------ operand image
     // Fronts whose widest update has at least 128 columns (and >= 16 pivot
     // rows) get an operand image and tensor-core tiles on the FP32 path; the
@@ -404,7 +418,7 @@ void Plan::build( const Symbolic & sym )
     extend_pull.clear(); extend_segs.clear();
     gemm_flops = 0.0;
     gemm_tile_flops = 0.0;
-    factor_launches.clear(); lower_launches.clear(); upper_launches.clear();
+    factor_launches.clear(); whole_launches.clear(); lower_launches.clear(); upper_launches.clear();
     dag.clear();
 
     struct Range { I64 first; I32 count; };
@@ -451,16 +465,77 @@ void Plan::build( const Symbolic & sym )
     std::vector<I32> panel_level, level_steps( static_cast<size_t>(levels), 0 );
     for( I32 h = 0; h < levels; ++h )
     {
-        const auto & L = by_level[h];
+        const auto & whole = by_level[h];
+        const auto small_begin = std::find_if( whole.begin(), whole.end(), [&]( I32 f ) { return front_small[static_cast<size_t>(f)] != 0; } );
+        const auto & L = whole;
+        const size_t n_large = static_cast<size_t>( small_begin - whole.begin() );   // the others come first
+        const std::vector<I32> S( small_begin, whole.end() );         // the small ones
         cur_level = h;
         const size_t extend_before = extend.size();   // this level's extend-adds signal its counter
+
+        // the small fronts: by shared memory, so that each launch's CTAs fit its class
+        std::vector<I64> front_task( S.size(), -1 );
+        I64 smem_max = 0;
+        for( I32 f : S ) { smem_max = std::max( smem_max, front_smem_bytes( front_n0[f], front_n1[f] ) ); }
+        // A few fronts: one launch, every CTA at once.  Many: by shared memory, most first, so that the
+        // smaller ones run several to an SM; 128 threads (three CTAs per SM) from kFrontMany fronts on,
+        // where throughput counts and not one front's latency.
+        const bool few = static_cast<I32>( S.size() ) <= kFrontFew;
+        const bool many = static_cast<I32>( S.size() ) >= kFrontMany;
+        const I64 limit[4] = { kFrontSmemMax, kFrontSmemMid, many ? kFrontSmemSmall : 0, 0 };
+        for( int cls = 0; cls < 3 && !S.empty(); ++cls )
+        {
+            const I64 first = static_cast<I64>( fronts.size() );
+            I64 smem = 0;
+            for( size_t k = 0; k < S.size(); ++k )
+            {
+                const I32 f = S[k];
+                const I64 need = front_smem_bytes( front_n0[f], front_n1[f] );
+                if( few ? cls != (smem_max > kFrontSmemMid ? 0 : 1) : need > limit[cls] || need <= limit[cls + 1] ) { continue; }
+                FrontTask t{};
+                t.v = front_v[f];
+                t.has_v = front_n1[f] > 0 && front_parent[f] < F ? 1 : 0;
+                t.seg_first = static_cast<I64>( extend_segs.size() );
+                for( I32 c = child_ptr[f]; c < child_ptr[f+1]; ++c )
+                {
+                    const I32 ct = child_idx[c];
+                    const I32 m1 = front_n1[ct];
+                    if( m1 == 0 ) { continue; }
+                    ExtendTask e{};
+                    e.w = front_v[ct];
+                    e.u0 = front_u0[f]; e.u1 = front_u1[f]; e.v = front_v[f];
+                    e.lut = front_lut[ct];
+                    e.m1 = m1; e.mid = mid[ct];
+                    e.n0p = front_n0[f]; e.n1p = front_n1[f];
+                    e.ldw = front_ld1[ct];
+                    e.ld0p = front_ld0[f]; e.ld1p = front_ld1[f]; e.ldvp = front_ld1[f];
+                    e.row_begin = 0; e.row_end = m1;
+                    extend_segs.push_back( e );
+                }
+                t.seg_count = static_cast<I32>( static_cast<I64>( extend_segs.size() ) - t.seg_first );
+                front_task[k] = static_cast<I64>( fronts.size() );
+                fronts.push_back( t );                          // its panel: filled in below
+                smem = std::max( smem, need );
+            }
+            const I32 count = static_cast<I32>( static_cast<I64>( fronts.size() ) - first );
+            if( count > 0 )
+            {
+                Launch Lf{ LaunchKind::Front, count, first, h, 0, n_large == 0 ? 0 : 1 };
+                Lf.small_count = static_cast<I32>( smem );
+                Lf.tc_count = cls == 0 ? 384 : cls == 1 ? 256 : 128;
+                whole_launches.push_back( Lf );
+            }
+        }
 
         // zero this level's update matrices before children add into them;
         // the regions may have been used by fronts consumed at earlier levels
         {
             const I64 first = static_cast<I64>(zero.size());
-            for( I32 f : L )
+            I32 large = 0;
+            for( size_t at = 0; at < L.size(); ++at )
             {
+                const I32 f = L[at];
+                if( at == n_large ) { large = static_cast<I32>( static_cast<I64>(zero.size()) - first ); }
                 // the upper triangle only, in groups of rows of about kZeroChunk entries
                 const I32 nv = front_n1[f];
                 for( I32 r = 0; r < nv; )
@@ -481,7 +556,9 @@ void Plan::build( const Symbolic & sym )
                 }
             }
             const I32 count = static_cast<I32>( static_cast<I64>(zero.size()) - first );
+            if( n_large == L.size() ) { large = count; }
             if( count > 0 ) { factor_launches.push_back( { LaunchKind::Zero, count, first, h, 0 } ); }
+            if( large > 0 ) { whole_launches.push_back( { LaunchKind::Zero, large, first, h, 0 } ); }
         }
 
         // extend-add passes by child rank (one child per parent and pass, so
@@ -539,8 +616,11 @@ void Plan::build( const Symbolic & sym )
         {
             const I64 pull_first = static_cast<I64>( extend_pull.size() );
             std::vector<I64> row_work;
-            for( I32 p : L )
+            I32 large = 0;
+            for( size_t at = 0; at < L.size(); ++at )
             {
+                const I32 p = L[at];
+                if( at == n_large ) { large = static_cast<I32>( static_cast<I64>( extend_pull.size() ) - pull_first ); }
                 const I32 cb = child_ptr[p], ce = child_ptr[p+1];
                 for( int space = 0; space < 2 && cb < ce; ++space )
                 {
@@ -601,6 +681,8 @@ void Plan::build( const Symbolic & sym )
                 Lp.tc_first = level_ext_first;
                 Lp.tc_count = static_cast<I32>( static_cast<I64>( extend.size() ) - level_ext_first );
                 factor_launches.push_back( Lp );
+                Lp.count = n_large == L.size() ? npull : large;
+                if( Lp.count > 0 ) { whole_launches.push_back( Lp ); }
             }
         }
 
@@ -620,13 +702,16 @@ void Plan::build( const Symbolic & sym )
             const I64 pfirst = static_cast<I64>(panel.size());
             const I64 gfirst = static_cast<I64>(gemm.size());
             const I64 rfirst = static_cast<I64>(srest.size());
+            I32 large_potrf = 0, large_trsm = 0;               // tasks of the fronts not taken whole (first in the step)
             std::vector<GemmTask> tiles;
             std::vector<I32> tile_panel, tile_prev;
             std::vector<char> tile_next, tile_small;
             std::vector<TcTask> tct;
             std::vector<char> tct_next;
-            for( I32 f : L )
+            for( size_t at = 0; at < whole.size(); ++at )
             {
+                const I32 f = whole[at];
+                const bool small = at >= n_large;
                 const I32 n0 = front_n0[f], n1 = front_n1[f];
                 const I32 r0 = q * kPanel;
                 if( r0 >= n0 ) { continue; }
@@ -652,6 +737,8 @@ void Plan::build( const Symbolic & sym )
                 t.single_rows = singles;
                 t.panel = pi;                   // == sdiag.size(): one potrf task and one SolveDiagTask per panel
                 t.img = front_img[f]; t.img_t0 = img_t0[f]; t.img_tf = img_tf[f];
+                if( small ) { fronts[static_cast<size_t>( front_task[at - n_large] )].p = t; }
+                else { ++large_potrf; large_trsm += static_cast<I32>( ceil_div( rest, kRestChunk ) ); }
                 {
                     PendingTask d = make( LaunchKind::Potrf, static_cast<I64>(potrf.size()) );
                     // the first panel starts once the children's contributions are in and
@@ -721,7 +808,9 @@ void Plan::build( const Symbolic & sym )
                                  front_v[f], ld1, n1, n1, true, tc_nmax );
                     }
                 }
-                for( size_t i = tfirst; i < tiles.size(); ++i ) { tile_small.push_back( front_img[f] < 0 ? 1 : 0 ); }
+                // the order of a step's tiles (within a part): taken whole without an image, others
+                // without, others with, taken whole with an image
+                for( size_t i = tfirst; i < tiles.size(); ++i ) { tile_small.push_back( front_img[f] < 0 ? (small ? 3 : 2) : (small ? 0 : 1) ); }
                 for( size_t i = tfirst; i < tiles.size(); ++i ) { tile_panel.push_back( pi ); tile_prev.push_back( prev ); }
                 {
                     SolveRestTask t{};
@@ -775,14 +864,18 @@ void Plan::build( const Symbolic & sym )
             const I32 gc = static_cast<I32>( static_cast<I64>(gemm.size()) - gfirst );
             if( oc > 0 ) { factor_launches.push_back( { LaunchKind::Potrf, oc, ofirst, h, q } ); }
             if( pc > 0 ) { factor_launches.push_back( { LaunchKind::Trsm, pc, pfirst, h, q } ); }
+            if( large_potrf > 0 ) { whole_launches.push_back( { LaunchKind::Potrf, large_potrf, ofirst, h, q } ); }
+            if( large_trsm > 0 ) { whole_launches.push_back( { LaunchKind::Trsm, large_trsm, pfirst, h, q } ); }
             {
                 // the step's tiles are in the order of `order`: the next panel's rows first,
                 // within each part the tiles of fronts without an operand image first
-                I32 gn = 0, sn0 = 0, sn1 = 0;
+                I32 gn = 0, sn0 = 0, sn1 = 0, before = 0, large = 0;
                 for( size_t i : order )
                 {
                     gn += tile_next[i] ? 1 : 0;
-                    if( tile_small[i] ) { (tile_next[i] ? sn0 : sn1) += 1; }
+                    if( tile_small[i] >= 2 ) { (tile_next[i] ? sn0 : sn1) += 1; }
+                    if( tile_small[i] == 3 ) { ++before; }
+                    if( !tile_next[i] && (tile_small[i] == 1 || tile_small[i] == 2) ) { ++large; }
                 }
                 // the same updates as tensor-core tiles: next-row tiles first, deepest first
                 std::vector<size_t> tord( tct.size() );
@@ -800,12 +893,15 @@ void Plan::build( const Symbolic & sym )
                     Launch L{ LaunchKind::Gemm, gn, gfirst, h, q, 0 };
                     L.small_count = sn0; L.tc_first = tfirst; L.tc_count = tn;
                     factor_launches.push_back( L );
+                    whole_launches.push_back( L );              // (small fronts have one panel: no next rows)
                 }
                 if( gc > gn )
                 {
                     Launch L{ LaunchKind::Gemm, gc - gn, gfirst + gn, h, q, 1 };
                     L.small_count = sn1; L.tc_first = tfirst + tn; L.tc_count = tcount - tn;
                     factor_launches.push_back( L );
+                    L.first += before; L.count = large;
+                    if( large > 0 ) { whole_launches.push_back( L ); }
                 }
             }
             rest_ranges[h][q] = { rfirst, static_cast<I32>( static_cast<I64>(srest.size()) - rfirst ) };

@@ -206,7 +206,7 @@ struct DagTask
 };
 
 enum class LaunchKind : std::int32_t { Zero = 0, Extend = 1, Trsm = 2, Gemm = 3, Invert = 4, Solve = 5, Potrf = 6,
-                                       SuperInv = 8, SuperDiag = 9, SuperRest = 10, ExtendPull = 11 };
+                                       SuperInv = 8, SuperDiag = 9, SuperRest = 10, ExtendPull = 11, Front = 12 };
 
 // Extend-add by parent rows (the level launches): one CTA adds, child by
 // child in rank order, the rows of every child that map into one block of
@@ -223,6 +223,40 @@ struct ExtendPullTask
     std::int32_t b0, b1;           // its parent rows [b0, b1) in that space
 };
 constexpr std::int64_t kExtendPullEntries = 4096;    // target child entries per pull task
+
+// A small front whole, in one CTA's shared memory: its assembled rows, the
+// children's update matrices added in rank order, the panel factorization, the
+// rest columns, and the update matrix written once (FrontTask, kernel
+// front_kernel).  It replaces five launches (zero, extend-add, potrf, trsm,
+// GEMM) and the passes over the front's entries between them.  Eligible: one
+// panel of pivot rows, and everything in kFrontSmemMax; a level takes the
+// kernel when at least half of its fronts are eligible (the others keep their
+// launches, which cost about the same for a few fronts as for many).  Every
+// front also has the separate tasks: those of the small ones come last in each
+// launch's range (GEMM tiles: around the others'), so that the launches
+// without them are ranges too.
+struct FrontTask
+{
+    PanelTask    p;                // its only panel (r0 = 0)
+    std::int64_t v;                // arena offset of its update matrix (leading dimension ld1); used when has_v
+    std::int64_t seg_first;        // its children in rank order: ExtendTasks of all their rows in Plan::extend_segs
+    std::int32_t seg_count;
+    std::int32_t has_v;
+};
+constexpr std::int64_t kFrontSmemMax   = 220 * 1024;  // one CTA of 384 threads per SM
+constexpr std::int64_t kFrontSmemMid   = 111 * 1024;  // two of 256 threads
+constexpr std::int64_t kFrontSmemSmall = 74 * 1024;   // three of 128 threads
+constexpr std::int32_t kFrontFew = 148, kFrontMany = 2000;
+
+// Shared memory of front_kernel in doubles: the front's rows (diagonal block
+// and rest columns, each rounded up to 8), the block's inverse, the update
+// matrix by 8-row blocks from the diagonal on, the pivot floors and flags.
+constexpr std::int64_t front_round8( std::int64_t x ) { return (x + 7) / 8 * 8; }
+constexpr std::int64_t front_smem_bytes( std::int64_t n0, std::int64_t n1 )
+{
+    const std::int64_t a = front_round8( n0 ), b = front_round8( n1 );
+    return 8 * (a * (a + b + 4) + a * (a + 4) + 4 * b * (b / 8 + 1) + kPanel + 2);
+}
 
 // The solve of a large front steps through its pivot rows 512 at a time
 // (super-panels) instead of 64 at a time: the inverse of each 512 x 512
@@ -281,6 +315,8 @@ struct Launch
     std::int64_t tc_first = 0;
     std::int32_t tc_count = 0;
     std::int32_t small_count = 0;
+    // Front launches: small_count = the launch's shared memory in bytes, tc_count = its threads; part 1: other
+    // fronts of the level keep their launches (the two may run side by side)
     // ExtendPull launches: the level's extend tasks in pass order are
     // [tc_first, tc_first + tc_count) of Plan::extend (what the persistent
     // schedule runs instead)
@@ -338,7 +374,11 @@ struct Plan
     std::vector<SolveDiagTask> sdiag;          // one per (front, panel); also the inverse-block list
     std::vector<SolveRestTask> srest;          // solve-step tasks, owner first per panel
 
-    std::vector<Launch> factor_launches;    // in order; the last one inverts the diagonal blocks
+    std::vector<Launch> factor_launches;    // in order, every front by the launches of its tasks' kinds
+    std::vector<Launch> whole_launches;     // FP64 level schedule: the same with the small fronts taken whole (Front
+                                            // launches) and left out of the others.  The factor is the same bit for bit;
+                                            // the FP32 path keeps factor_launches, as its tensor-core updates are rounded
+                                            // in their own order
     std::vector<DagTask> dag;               // the levels from dag_split_level up as one dependency-ordered task list
     std::int32_t dag_counters = 0;
     std::int32_t dag_min_steps = kDagMinSteps;   // set before build(): 0 puts every level in the task graph
@@ -360,6 +400,8 @@ struct Plan
     std::vector<Launch> sinv_launches;
     std::vector<SuperSolveTask> ssolve;
     std::vector<ExtendPullTask> extend_pull;
+    std::vector<FrontTask> fronts;             // the small fronts taken whole, by level
+    std::vector<char> front_small;             // per front: taken whole (FP64 level schedule)
     std::vector<ExtendTask> extend_segs;
     std::vector<Launch> lower_launches_sp, upper_launches_sp;
     std::int64_t super_inv_size = 0;        // doubles of all inverses

@@ -11,6 +11,7 @@
 #include "parallel.hpp"
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cmath>
 #include <map>
@@ -151,6 +152,104 @@ std::string check_plan( const Symbolic & sym, const Plan & pl )
         for( const auto & kv : rows )
         {
             for( I32 c : kv.second.second ) { if( c != 0 ) { return "extend pull launch does not add every child row once"; } }
+        }
+    }
+    // small fronts taken whole: dimensions inside the arena and the launch's shared memory, the panel's
+    // own task, and every child of the front once, all rows, in rank order
+    {
+        std::vector<char> seen( static_cast<size_t>( pl.front_count ), 0 );
+        std::map<I64, I32> by_u0;
+        for( I32 f = 0; f < pl.front_count; ++f ) { by_u0[pl.front_u0[static_cast<size_t>( f )]] = f; }
+        std::map<std::pair<I32, I64>, I32> by_v;                              // (level, update matrix) -> front
+        for( I32 f = 0; f < pl.front_count; ++f ) { if( pl.front_n1[static_cast<size_t>( f )] > 0 ) { by_v[{ pl.level_of[static_cast<size_t>( f )], pl.front_v[static_cast<size_t>( f )] }] = f; } }
+        std::vector<I32> kids( static_cast<size_t>( pl.front_count ), 0 );
+        std::map<I64, I32> by_lut;
+        for( I32 f = 0; f < pl.front_count; ++f )
+        {
+            if( pl.front_n1[static_cast<size_t>( f )] == 0 || pl.front_parent[static_cast<size_t>( f )] >= pl.front_count ) { continue; }
+            ++kids[static_cast<size_t>( pl.front_parent[static_cast<size_t>( f )] )];
+            by_lut[pl.front_lut[static_cast<size_t>( f )]] = f;
+        }
+        for( const Launch & L : pl.whole_launches )
+        {
+            if( L.kind != LaunchKind::Front ) { continue; }
+            if( L.count <= 0 || L.first < 0 || L.first + L.count > static_cast<I64>( pl.fronts.size() ) || L.small_count > (L.tc_count == 384 ? kFrontSmemMax : L.tc_count == 256 ? kFrontSmemMid : L.tc_count == 128 ? kFrontSmemSmall : 0) )
+            {
+                return "front launch out of bounds";
+            }
+            for( I64 k = L.first; k < L.first + L.count; ++k )
+            {
+                const FrontTask & t = pl.fronts[static_cast<size_t>( k )];
+                const std::string at = " (front task " + std::to_string( k ) + ")";
+                const auto it = by_u0.find( t.p.u0 );
+                if( it == by_u0.end() ) { return "front task names no front" + at; }
+                const size_t f = static_cast<size_t>( it->second );
+                if( seen[f]++ || !pl.front_small[f] || pl.level_of[f] != L.level ) { return "front task repeated or misplaced" + at; }
+                if( t.p.n0 != pl.front_n0[f] || t.p.n1 != pl.front_n1[f] || t.p.n0 > kPanel || t.p.r0 != 0 || t.p.u1 != pl.front_u1[f] || t.v != pl.front_v[f]
+                    || t.p.ld0 != pl.front_ld0[f] || t.p.ld1 != pl.front_ld1[f] || t.p.row0 != pl.front_row0[f] ) { return "front task dimensions" + at; }
+                if( t.p.panel < 0 || t.p.panel >= static_cast<I32>( pl.potrf.size() ) || pl.potrf[static_cast<size_t>( t.p.panel )].u0 != t.p.u0 ) { return "front task panel" + at; }
+                if( (t.p.u0 | t.p.u1 | t.v) % 4 != 0 || (t.p.ld0 | t.p.ld1) % 4 != 0 ) { return "front task alignment" + at; }
+                if( (t.has_v != 0) != (t.p.n1 > 0 && pl.front_parent[f] < pl.front_count) ) { return "front task update matrix" + at; }
+                const I64 need = front_smem_bytes( t.p.n0, t.p.n1 );
+                if( need > L.small_count ) { return "front task shared memory" + at; }
+                if( t.seg_count != kids[f] || t.seg_first < 0 || t.seg_first + t.seg_count > static_cast<I64>( pl.extend_segs.size() ) ) { return "front task children" + at; }
+                I32 last = -1;
+                for( I64 g = t.seg_first; g < t.seg_first + t.seg_count; ++g )
+                {
+                    const ExtendTask & e = pl.extend_segs[static_cast<size_t>( g )];
+                    const auto c = by_lut.find( e.lut );
+                    if( c == by_lut.end() || pl.front_parent[static_cast<size_t>( c->second )] != it->second || c->second <= last ) { return "front task child order" + at; }
+                    last = c->second;
+                    if( e.row_begin != 0 || e.row_end != e.m1 || e.m1 != pl.front_n1[static_cast<size_t>( last )] || e.w != pl.front_v[static_cast<size_t>( last )]
+                        || e.n0p != t.p.n0 || e.n1p != t.p.n1 ) { return "front task child" + at; }
+                }
+            }
+        }
+        for( I32 f = 0; f < pl.front_count; ++f ) { if( pl.front_small[static_cast<size_t>( f )] != seen[static_cast<size_t>( f )] ) { return "a small front without a task"; } }
+        // the other launches of the list: each inside the launch of the same kind, level, step and part
+        // with every front, and all and only the tasks of the other fronts
+        std::map<std::array<I64, 4>, const Launch *> full;
+        auto key = []( const Launch & L ) { return std::array<I64, 4>{ static_cast<I64>( L.kind ), L.level, L.step, L.part }; };
+        for( const Launch & L : pl.factor_launches ) { full[key( L )] = &L; }
+        auto of_small = [&]( const Launch & L, I64 k ) -> int                 // 1: a small front's task, 0: another's, -1: unknown
+        {
+            I64 u0 = -1;
+            switch( L.kind )
+            {
+                case LaunchKind::Potrf: u0 = pl.potrf[static_cast<size_t>( k )].u0; break;
+                case LaunchKind::Trsm:  u0 = pl.panel[static_cast<size_t>( k )].u0; break;
+                case LaunchKind::ExtendPull: u0 = pl.extend_segs[static_cast<size_t>( pl.extend_pull[static_cast<size_t>( k )].seg_first )].u0; break;
+                case LaunchKind::Zero:
+                {
+                    const auto v = by_v.find( { L.level, pl.zero[static_cast<size_t>( k )].offset } );
+                    return v == by_v.end() ? -1 : pl.front_small[static_cast<size_t>( v->second )];
+                }
+                case LaunchKind::Gemm:
+                {
+                    // (a small front's only tiles are those of its update matrix)
+                    const auto v = by_v.find( { L.level, pl.gemm[static_cast<size_t>( k )].c } );
+                    return v == by_v.end() ? 0 : pl.front_small[static_cast<size_t>( v->second )];
+                }
+                default: return -1;
+            }
+            const auto it = by_u0.find( u0 );
+            return it == by_u0.end() ? -1 : pl.front_small[static_cast<size_t>( it->second )];
+        };
+        for( const Launch & L : pl.whole_launches )
+        {
+            if( L.kind == LaunchKind::Front ) { continue; }
+            const auto it = full.find( key( L ) );
+            if( it == full.end() || L.first < it->second->first || L.first + L.count > it->second->first + it->second->count ) { return "launch list of small fronts: a launch outside its full one"; }
+            for( I64 k = it->second->first; k < it->second->first + it->second->count; ++k )
+            {
+                const bool in = k >= L.first && k < L.first + L.count;
+                if( of_small( *it->second, k ) != (in ? 0 : 1) ) { return "launch list of small fronts: a launch with the wrong tasks"; }
+            }
+            full.erase( it );
+        }
+        for( const auto & kv : full )
+        {
+            for( I64 k = kv.second->first; k < kv.second->first + kv.second->count; ++k ) { if( of_small( *kv.second, k ) != 1 ) { return "launch list of small fronts: a launch is missing"; } }
         }
     }
     for( int which = 0; which < 2; ++which )
@@ -409,11 +508,12 @@ std::string check_plan( const Symbolic & sym, const Plan & pl )
             case LaunchKind::Solve:  return static_cast<I64>( pl.srest.size() );
             case LaunchKind::Potrf:  return static_cast<I64>( pl.potrf.size() );
             case LaunchKind::ExtendPull: return static_cast<I64>( pl.extend_pull.size() );
+            case LaunchKind::Front:  return static_cast<I64>( pl.fronts.size() );
             default: break;
         }
         return -1;
     };
-    for( const std::vector<Launch> * list : { &pl.factor_launches, &pl.pre_dag_launches, &pl.lower_launches, &pl.upper_launches } )
+    for( const std::vector<Launch> * list : { &pl.factor_launches, &pl.whole_launches, &pl.pre_dag_launches, &pl.lower_launches, &pl.upper_launches } )
     {
         for( const Launch & L : *list )
         {
