@@ -115,7 +115,7 @@ struct tb_chol
     // second stream of the level schedule: the GEMM tiles of a panel step that
     // do not touch the next panel run there, overlapping the next potrf / trsm
     cudaStream_t side = nullptr;
-    cudaEvent_t ev_trsm = nullptr, ev_rest = nullptr;
+    cudaEvent_t ev_trsm = nullptr, ev_soon = nullptr, ev_rest = nullptr;
 
     // input pattern (copied, CholeskyDecomposition.hpp:313-371)
     std::int32_t n = 0;
@@ -248,6 +248,7 @@ struct tb_chol
         if( own_stream && stream ) { cudaStreamDestroy( stream ); }
         if( side ) { cudaStreamDestroy( side ); }
         if( ev_trsm ) { cudaEventDestroy( ev_trsm ); }
+        if( ev_soon ) { cudaEventDestroy( ev_soon ); }
         if( ev_rest ) { cudaEventDestroy( ev_rest ); }
     }
 
@@ -355,6 +356,7 @@ int ensure_device( tb_chol * h )
     {
         TB_CUDA( cudaStreamCreateWithFlags( &h->side, cudaStreamNonBlocking ) );
         TB_CUDA( cudaEventCreateWithFlags( &h->ev_trsm, cudaEventDisableTiming ) );
+        TB_CUDA( cudaEventCreateWithFlags( &h->ev_soon, cudaEventDisableTiming ) );
         TB_CUDA( cudaEventCreateWithFlags( &h->ev_rest, cudaEventDisableTiming ) );
     }
     if( !h->kernels_configured )
@@ -544,25 +546,28 @@ std::int64_t issue_factor_t( tb_chol * h, bool timed, std::vector<int> * kinds )
         }
         return launches;
     }
-    // One panel of look-ahead over two streams (the profiled path keeps one,
-    // so that every launch is timed alone).  Main stream: potrf(q), trsm(q),
-    // the tiles of step q that update panel q+1's rows (part 0).  Side
-    // stream: the other tiles of step q (part 1), after trsm(q); they run
-    // while potrf(q+1) and trsm(q+1) do.  Part 0 of step q waits for part 1
-    // of step q-1 (both update panel q+1's rows), which also orders
-    // potrf(q+1) after every update of its block; each C tile keeps the order
-    // of its updates, so the factor is the same bit for bit.
-    // Levels join the side stream at their boundaries (the next extend-adds
-    // read the update matrices the part-1 tiles write).
+    // Look-ahead over two streams (the profiled path keeps one, so that every
+    // launch is timed alone).  Main stream: potrf(q), trsm(q), the tiles of
+    // step q that update panel q+1's rows (part 0).  Side stream: the other
+    // tiles of step q, after trsm(q): first the rows of the panels up to the
+    // next full update (part 1), then the rest (part 2), which runs while the
+    // main stream goes through the next defer_steps panels.  Part 0 of a step
+    // waits for the part 1 of the last full update; part 0 of a full update for
+    // its part 2, which wrote panel q+1's rows last.  Each C tile keeps the
+    // order of its updates, so the factor is the same bit for bit.  Levels join
+    // the side stream at their boundaries (the next extend-adds read the update
+    // matrices the part-2 tiles write).
     const bool overlap = !timed && h->side != nullptr;
-    bool side_busy = false;
+    bool soon_busy = false, rest_busy = false;       // side-stream work of parts 1 / 2 the main stream has not waited for
     std::int32_t level = -1;
     auto join = [&]()
     {
-        if( !side_busy ) { return; }
-        cudaEventRecord( h->ev_rest, h->side );
-        cudaStreamWaitEvent( st, h->ev_rest, 0 );
-        side_busy = false;
+        if( rest_busy || soon_busy )
+        {
+            cudaEventRecord( h->ev_rest, h->side );
+            cudaStreamWaitEvent( st, h->ev_rest, 0 );
+        }
+        soon_busy = rest_busy = false;
     };
     for( const tb::Launch & L : level_launches( h ) )
     {
@@ -576,16 +581,20 @@ std::int64_t issue_factor_t( tb_chol * h, bool timed, std::vector<int> * kinds )
                 cudaEventRecord( h->ev_trsm, st );
                 cudaStreamWaitEvent( h->side, h->ev_trsm, 0 );
                 s = h->side;
-                side_busy = true;
+                rest_busy = true;
             }
             if( L.kind == tb::LaunchKind::Gemm )
             {
-                if( L.part == 0 ) { join(); }
+                if( L.part == 0 )
+                {
+                    if( L.step % pl.defer_steps == pl.defer_steps - 1 ) { join(); }
+                    else if( soon_busy ) { cudaStreamWaitEvent( st, h->ev_soon, 0 ); soon_busy = false; }
+                }
                 else
                 {
                     cudaStreamWaitEvent( h->side, h->ev_trsm, 0 );
                     s = h->side;
-                    side_busy = true;
+                    (L.part == 1 ? soon_busy : rest_busy) = true;
                 }
             }
         }
@@ -609,6 +618,7 @@ std::int64_t issue_factor_t( tb_chol * h, bool timed, std::vector<int> * kinds )
             default: break;
         }
         if( overlap && L.kind == tb::LaunchKind::Trsm ) { cudaEventRecord( h->ev_trsm, st ); }
+        if( overlap && L.kind == tb::LaunchKind::Gemm && L.part == 1 ) { cudaEventRecord( h->ev_soon, h->side ); }
         mark( static_cast<int>( L.kind == tb::LaunchKind::ExtendPull ? tb::LaunchKind::Extend : L.kind == tb::LaunchKind::Front ? tb::LaunchKind::Solve : L.kind ) );
         ++launches;
     }

@@ -42,9 +42,10 @@ void push_tiles( std::vector<GemmTask> & out, I64 a, I32 lda, I64 b, I32 ldb, I6
 
 // The tensor-core tiles of the fronts with an operand image (see TcTask):
 // kTcM x nt tiles (nt up to nmax <= kTcNMax) over C's M x N entries (symmetric: the
-// tiles on and right of the diagonal).  next_rows: the call updates the next
-// panel's rows, which the tiles of the first tile row contain.
-void push_tc( std::vector<TcTask> & out, std::vector<char> & next, bool next_rows, I64 blk, I32 tf,
+// tiles on and right of the diagonal).  soon: row bound of the tiles that the
+// panel steps up to the next full update read (0: none; see Launch::part): the
+// first tile row is class 2, further ones below `soon` 1, the rest 0.
+void push_tc( std::vector<TcTask> & out, std::vector<char> & next, I32 soon, I64 blk, I32 tf,
               I32 ta0, I32 tb0, I32 K, I64 c, I32 ldc, I32 M, I32 N, bool symmetric, I32 nmax )
 {
     for( I32 m0 = 0; m0 < M; m0 += kTcM )
@@ -59,7 +60,7 @@ void push_tc( std::vector<TcTask> & out, std::vector<char> & next, bool next_row
             t.nt = static_cast<I32>( std::min<I64>( nmax, ceil_div( N - c0, kImgRows ) * kImgRows ) );
             t.upper = symmetric ? 1 : 0;
             out.push_back( t );
-            next.push_back( next_rows && m0 == 0 ? 1 : 0 );
+            next.push_back( m0 >= soon ? 0 : m0 == 0 ? 2 : 1 );
         }
     }
 }
@@ -782,18 +783,20 @@ void Plan::build( const Symbolic & sym )
                         push_tiles( tiles, pa, ld0, front_u1[f] + static_cast<I64>(k0) * ld1, ld1,
                                     front_u1[f] + static_cast<I64>(r1) * ld1, ld1, K, rows, n1, false );
                     }
-                    // tiles of rows [r1, r1 + 64) feed the next panel
-                    for( size_t i = tfirst; i < tiles.size(); ++i ) { tile_next.push_back( tiles[i].m0 == 0 ? 1 : 0 ); }
+                    // tiles of rows [r1, r1 + 64) feed the next panel (class 2), those of the rows that
+                    // the steps up to the next full update read come next (1), the rest last (0)
+                    const I32 soon = kPanel * defer_steps;
+                    for( size_t i = tfirst; i < tiles.size(); ++i ) { tile_next.push_back( tiles[i].m0 >= soon ? 0 : tiles[i].m0 == 0 ? 2 : 1 ); }
                     if( front_img[f] >= 0 )
                     {
                         // r1 and k0 are multiples of 64: whole image column tiles and k-chunks
                         const I64 blk = front_img[f] + static_cast<I64>( k0 / kImgK ) * 2 * img_tf[f];
                         const I32 ta = r1 / kImgRows;
-                        push_tc( tct, tct_next, true, blk, img_tf[f], ta, ta, K,
+                        push_tc( tct, tct_next, soon, blk, img_tf[f], ta, ta, K,
                                  front_u0[f] + static_cast<I64>(r1) * ld0 + r1, ld0, rows, m, true, tc_nmax );
                         if( n1 > 0 )
                         {
-                            push_tc( tct, tct_next, true, blk, img_tf[f], ta, img_t0[f], K,
+                            push_tc( tct, tct_next, soon, blk, img_tf[f], ta, img_t0[f], K,
                                      front_u1[f] + static_cast<I64>(r1) * ld1, ld1, rows, n1, false, tc_nmax );
                         }
                     }
@@ -804,7 +807,7 @@ void Plan::build( const Symbolic & sym )
                     for( size_t i = tfirst; i < tiles.size(); ++i ) { tile_next.push_back( 0 ); }
                     if( front_img[f] >= 0 )
                     {
-                        push_tc( tct, tct_next, false, front_img[f], img_tf[f], img_t0[f], img_t0[f], n0,
+                        push_tc( tct, tct_next, 0, front_img[f], img_tf[f], img_t0[f], img_t0[f], n0,
                                  front_v[f], ld1, n1, n1, true, tc_nmax );
                     }
                 }
@@ -853,53 +856,49 @@ void Plan::build( const Symbolic & sym )
                 // the previous step's tiles of the front update the same C blocks
                 if( prev >= 0 ) { add_wait( d, kGemmDone, prev, panel_tiles[static_cast<size_t>(prev)] ); }
                 d.signal[0] = { kGemmDone, pi };
-                if( tile_next[i] ) { d.signal[1] = { kNextDone, pi }; ++panel_next[static_cast<size_t>(pi)]; }
-                (tile_next[i] ? next_tiles[q] : rest_tiles[q]).push_back( d );
+                if( tile_next[i] == 2 ) { d.signal[1] = { kNextDone, pi }; ++panel_next[static_cast<size_t>(pi)]; }
+                (tile_next[i] == 2 ? next_tiles[q] : rest_tiles[q]).push_back( d );
                 gemm.push_back( t );
             }
             for( size_t i : order ) { ++panel_tiles[static_cast<size_t>( tile_panel[i] )]; }
 
             const I32 oc = static_cast<I32>( static_cast<I64>(potrf.size()) - ofirst );
             const I32 pc = static_cast<I32>( static_cast<I64>(panel.size()) - pfirst );
-            const I32 gc = static_cast<I32>( static_cast<I64>(gemm.size()) - gfirst );
             if( oc > 0 ) { factor_launches.push_back( { LaunchKind::Potrf, oc, ofirst, h, q } ); }
             if( pc > 0 ) { factor_launches.push_back( { LaunchKind::Trsm, pc, pfirst, h, q } ); }
             if( large_potrf > 0 ) { whole_launches.push_back( { LaunchKind::Potrf, large_potrf, ofirst, h, q } ); }
             if( large_trsm > 0 ) { whole_launches.push_back( { LaunchKind::Trsm, large_trsm, pfirst, h, q } ); }
             {
-                // the step's tiles are in the order of `order`: the next panel's rows first,
-                // within each part the tiles of fronts without an operand image first
-                I32 gn = 0, sn0 = 0, sn1 = 0, before = 0, large = 0;
-                for( size_t i : order )
-                {
-                    gn += tile_next[i] ? 1 : 0;
-                    if( tile_small[i] >= 2 ) { (tile_next[i] ? sn0 : sn1) += 1; }
-                    if( tile_small[i] == 3 ) { ++before; }
-                    if( !tile_next[i] && (tile_small[i] == 1 || tile_small[i] == 2) ) { ++large; }
-                }
-                // the same updates as tensor-core tiles: next-row tiles first, deepest first
+                // the same updates as tensor-core tiles: by class, deepest first
                 std::vector<size_t> tord( tct.size() );
                 for( size_t i = 0; i < tord.size(); ++i ) { tord[i] = i; }
                 std::stable_sort( tord.begin(), tord.end(), [&]( size_t x, size_t y ) {
                     if( tct_next[x] != tct_next[y] ) { return tct_next[x] > tct_next[y]; }
                     return tct[x].K > tct[y].K;
                 } );
-                const I64 tfirst = static_cast<I64>( tc.size() );
-                I32 tn = 0;
-                for( size_t i : tord ) { tc.push_back( tct[i] ); tn += tct_next[i] ? 1 : 0; }
-                const I32 tcount = static_cast<I32>( tct.size() );
-                if( gn > 0 )
+                I64 tfirst = static_cast<I64>( tc.size() );
+                for( size_t i : tord ) { tc.push_back( tct[i] ); }
+                // the step's tiles are in the order of `order`: by class, within each class the tiles of
+                // fronts without an operand image first; one launch per class
+                I64 first = gfirst;
+                for( int part = 0; part < 3; ++part )
                 {
-                    Launch L{ LaunchKind::Gemm, gn, gfirst, h, q, 0 };
-                    L.small_count = sn0; L.tc_first = tfirst; L.tc_count = tn;
-                    factor_launches.push_back( L );
-                    whole_launches.push_back( L );              // (small fronts have one panel: no next rows)
-                }
-                if( gc > gn )
-                {
-                    Launch L{ LaunchKind::Gemm, gc - gn, gfirst + gn, h, q, 1 };
-                    L.small_count = sn1; L.tc_first = tfirst + tn; L.tc_count = tcount - tn;
-                    factor_launches.push_back( L );
+                    const char cls = static_cast<char>( 2 - part );
+                    Launch L{ LaunchKind::Gemm, 0, first, h, q, part };
+                    I32 before = 0, large = 0;
+                    for( size_t i : order )
+                    {
+                        if( tile_next[i] != cls ) { continue; }
+                        ++L.count;
+                        if( tile_small[i] >= 2 ) { ++L.small_count; }
+                        if( tile_small[i] == 3 ) { ++before; }
+                        if( tile_small[i] == 1 || tile_small[i] == 2 ) { ++large; }
+                    }
+                    L.tc_first = tfirst;
+                    for( size_t i : tord ) { L.tc_count += tct_next[i] == cls ? 1 : 0; }
+                    tfirst += L.tc_count;
+                    first += L.count;
+                    if( L.count > 0 || L.tc_count > 0 ) { factor_launches.push_back( L ); }
                     L.first += before; L.count = large;
                     if( large > 0 ) { whole_launches.push_back( L ); }
                 }

@@ -298,9 +298,13 @@ struct SuperSolveTask
 };
 
 // One launch: `count` tasks starting at `first` in the array of its kind.
-// A panel step's GEMM tiles come as two launches: part 0 updates the next
-// panel's rows (the next potrf / trsm wait for it), part 1 the rest of the
-// trailing matrix and the update matrices (it may overlap the next panel).
+// A panel step's GEMM tiles come as up to three launches: part 0 updates the
+// next panel's rows (the next potrf / trsm wait for it); part 1 the rows of the
+// panels after it up to the next full update, whose steps' part 0 wait for it;
+// part 2 the rest of the trailing matrix and the update matrices, which only
+// the next full update and the level's end wait for, so that it overlaps
+// defer_steps panel steps.  (128-row tensor-core tiles may reach a part's rows
+// early: a tile belongs to the part of its first row.)
 struct Launch
 {
     LaunchKind   kind;

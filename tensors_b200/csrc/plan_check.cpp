@@ -517,7 +517,7 @@ std::string check_plan( const Symbolic & sym, const Plan & pl )
     {
         for( const Launch & L : *list )
         {
-            if( L.count <= 0 || L.first < 0 || L.first + L.count > size_of( L.kind ) ) { return "launch task range out of bounds"; }
+            if( L.count < 0 || (L.count == 0 && L.kind != LaunchKind::Gemm) || L.first < 0 || L.first + L.count > size_of( L.kind ) ) { return "launch task range out of bounds"; }
         }
     }
     // task graph: every task index in range, and every wait reached by
