@@ -826,9 +826,11 @@ __global__ __launch_bounds__(kPotrfThreads, 1) void potrf_kernel( const PanelTas
                                                                const double * __restrict__ pivot_floor,
                                                                double * __restrict__ tinv )
 {
-    pdl_allow_next();
     const PanelTask t = tasks[blockIdx.x];
     pdl_wait();
+    // only now: the trsm reads the rest columns before its own wait, so everything before this
+    // launch must be complete when it starts
+    pdl_allow_next();
     potrf_body<T, kPotrfThreads>( t, arena, status, pivot_floor, tinv );
 }
 
@@ -1062,12 +1064,16 @@ void front_kernel( const FrontTask * __restrict__ tasks, const ExtendTask * __re
     }
 }
 
-// X = D^{-T} U for the rest columns [c0, c0 + kRestChunk) of a panel (trsm of
+// X = D^{-T} U for the rest columns [c0, c0 + cw) of a panel (trsm of
 // FactorizeSupernode, Multifrontal.hpp:452-466) as the product X = T^T U with
 // the inverse T = D^{-1} that the panel's potrf left in tinv: X row block rb
-// takes the K blocks 0..rb.  Warp w computes the output tiles (rb, ct) with
-// rb = (w + ct) mod 8, one of every block row, so every warp does the same
-// 36 8 x 8 x 8 DMMA steps (when nb = 64); no step waits on another.
+// takes the K blocks 0..rb.  A chunk lies in U0 or in U1, so that its rows are
+// read and written in aligned vectors.  Warp w takes the chunk's column tile w
+// with all eight row blocks' sums in registers: 72 independent-by-eight DMMAs
+// follow 88 fragment loads, and the results go to global memory from the
+// registers.  Bound: the launch's latency (load, 72 DMMAs a warp, store) on
+// the panel chain, so the rest columns are loaded before the wait on the
+// potrf, which writes only the diagonal block and T.
 // Operand-image entry of U row k, rest column `col` of a panel whose rest
 // columns start at U0 column r1 (m of them in U0, the rest U1 columns).
 __device__ __forceinline__ std::int64_t img_offset( const PanelTask & t, int k, int col, int r1, int m )
@@ -1078,7 +1084,7 @@ __device__ __forceinline__ std::int64_t img_offset( const PanelTask & t, int k, 
     return blk * (kImgRows * kImgK) + (ucol % kImgRows) * kImgK + (k % kImgK);
 }
 
-template<typename T>
+template<typename T, bool kPdl>
 __device__ __forceinline__ void trsm_body( const PanelTask & t, T * __restrict__ arena, const double * __restrict__ tinv,
                                            double * tsm, float * __restrict__ img = nullptr )
 {
@@ -1091,10 +1097,23 @@ __device__ __forceinline__ void trsm_body( const PanelTask & t, T * __restrict__
     const int r1 = t.r0 + nb;
     const int m = t.n0 - r1;
     const int rest = m + t.n1;
-    const int cw = min( kRestChunk, rest - t.c0 );
-    T * U0 = arena + t.u0;
-    T * U1 = arena + t.u1;
-    static_assert( kRestChunk == kPanel, "trsm assumes square blocks" );
+    const bool in0 = t.c0 < m;                            // the chunk's columns: U0's or U1's
+    const int cw = min( kRestChunk, (in0 ? m : rest) - t.c0 );
+    const int ld = in0 ? t.ld0 : t.ld1;
+    T * U = (in0 ? arena + t.u0 + r1 + t.c0 : arena + t.u1 + (t.c0 - m)) + (std::int64_t)t.r0 * ld;
+    static_assert( kRestChunk == kPanel && kTrsmThreads / 32 == kRestChunk / kSub, "trsm assumes square blocks and a warp per column tile" );
+    constexpr int kV = 16 / static_cast<int>( sizeof(T) );
+    constexpr int kPieces = kPanel * kRestChunk / kV / kTrsmThreads;
+    [[maybe_unused]] float4 xf[sizeof(T) == 4 ? kPieces : 1];
+#pragma unroll
+    for( int u = 0; u < kPieces; ++u )
+    {
+        const int idx = kV * (tid + u * kTrsmThreads), r = idx / kRestChunk, c = idx % kRestChunk;
+        const bool in = r < nb && c < cw;
+        if constexpr ( sizeof(T) == 8 ) { cp_async_16( &X[r][c], in ? U + (std::int64_t)r * ld + c : U, in ? (c + 1 < cw ? 16 : 8) : 0 ); }
+        else { xf[u] = in ? *reinterpret_cast<const float4 *>( U + (std::int64_t)r * ld + c ) : make_float4( 0.f, 0.f, 0.f, 0.f ); }
+    }
+    if constexpr ( kPdl ) { pdl_wait(); }
     {
         // only the leading (nb rounded up to 8)^2 block of T is read
         const double * Tg = tinv + (std::int64_t)t.panel * (kPanel * kPanel);
@@ -1103,76 +1122,77 @@ __device__ __forceinline__ void trsm_body( const PanelTask & t, T * __restrict__
         for( int u = 0; u < kPanel * kPanel / (2 * kTrsmThreads); ++u )
         {
             const int idx = 2 * (tid + u * kTrsmThreads);
-            const bool used = (idx >> 6) < nbp && (idx & 63) < nbp;
-            cp_async_16( &Ti[idx >> 6][idx & 63], used ? Tg + idx : Tg, used ? 16 : 0 );
+            if( (idx >> 6) < nbp && (idx & 63) < nbp ) { cp_async_16( &Ti[idx >> 6][idx & 63], Tg + idx, 16 ); }
         }
-    }
-    auto stage_src = [&]( int idx, double & ) -> const T *
-    {
-        const int r = idx / kPanel, c = idx % kPanel;
-        const int col = t.c0 + c;
-        if( r >= nb || c >= cw ) { return nullptr; }
-        return (col < m) ? U0 + (std::int64_t)(t.r0 + r) * t.ld0 + r1 + col
-                         : U1 + (std::int64_t)(t.r0 + r) * t.ld1 + (col - m);
-    };
-    auto stage_dst = [&]( int idx ) { return &X[idx / kPanel][idx % kPanel]; };
-    stage_block<T, kPanel * kRestChunk / kTrsmThreads, kTrsmThreads>( U0, stage_src, stage_dst );
-    cp_async_wait_all();
-    stage_finish<T, kPanel * kRestChunk / kTrsmThreads, kTrsmThreads>( stage_src, stage_dst );
-    __syncthreads();
-    const int nct = (cw + kSub - 1) / kSub;
-    double res[kRestChunk / kSub][2];
-#pragma unroll
-    for( int ct = 0; ct < kRestChunk / kSub; ++ct )
-    {
-        res[ct][0] = 0.0; res[ct][1] = 0.0;
-        const int rb = (warp + ct) & (kSubs - 1);
-        if( rb >= nbb || ct >= nct ) { continue; }
-        for( int kb = 0; kb <= rb; ++kb )
-        {
-            dmma_8x8x8( res[ct], [&]( int i, int k ) { return Ti[kSub * kb + k][kSub * rb + i]; },
-                                 [&]( int k, int j ) { return X[kSub * kb + k][kSub * ct + j]; } );
-        }
-    }
-    // the products are done: the results replace the staged block, then go out coalesced
-    __syncthreads();
-#pragma unroll
-    for( int ct = 0; ct < kRestChunk / kSub; ++ct )
-    {
-        const int rb = (warp + ct) & (kSubs - 1);
-        if( rb >= nbb || ct >= nct ) { continue; }
-        const int r = kSub * rb + (lane >> 2), cc = kSub * ct + 2 * (lane & 3);
-        X[r][cc] = static_cast<double>( static_cast<T>( res[ct][0] ) );
-        X[r][cc + 1] = static_cast<double>( static_cast<T>( res[ct][1] ) );
-    }
-    __syncthreads();
-    // U rows: consecutive threads, consecutive columns
-    for( int idx = tid; idx < kPanel * kRestChunk; idx += kTrsmThreads )
-    {
-        const int r = idx >> 6, cc = idx & 63;
-        if( r >= nb || cc >= cw ) { continue; }
-        const int col = t.c0 + cc;
-        const T v = static_cast<T>( X[r][cc] );
-        if( col < m ) { U0[(std::int64_t)(t.r0 + r) * t.ld0 + r1 + col] = v; }
-        else          { U1[(std::int64_t)(t.r0 + r) * t.ld1 + (col - m)] = v; }
     }
     if constexpr ( sizeof(T) == 4 )
     {
-        if( img != nullptr && t.img >= 0 )
+#pragma unroll
+        for( int u = 0; u < kPieces; ++u )
         {
-            // the stored FP32 values split into TF32 hi + lo, for the tensor-core tiles: the
-            // image is K-major, so a warp writes one column's 32 k values of a k-chunk at once
-            // (128 contiguous bytes per part)
-            const std::int64_t lo_off = static_cast<std::int64_t>( t.img_tf ) * (kImgRows * kImgK);
-            for( int pair = warp; pair < 2 * cw; pair += kTrsmThreads / 32 )
+            const int idx = kV * (tid + u * kTrsmThreads), r = idx / kRestChunk, c = idx % kRestChunk;
+            // (a row's padding beyond cw may hold anything: zero)
+            const double x[4] = { xf[u].x, c + 1 < cw ? xf[u].y : 0.0, c + 2 < cw ? xf[u].z : 0.0, c + 3 < cw ? xf[u].w : 0.0 };
+            *reinterpret_cast<double2 *>( &X[r][c] ) = make_double2( x[0], x[1] );
+            *reinterpret_cast<double2 *>( &X[r][c + 2] ) = make_double2( x[2], x[3] );
+        }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    const int c = kSub * warp;                            // this warp's column tile
+    if( c < cw )
+    {
+        const int fi = lane >> 2, fj = 2 * (lane & 3);
+        double acc[kSubs][2];
+#pragma unroll
+        for( int rb = 0; rb < kSubs; ++rb ) { acc[rb][0] = 0.0; acc[rb][1] = 0.0; }
+#pragma unroll
+        for( int kb = 0; kb < kSubs; ++kb )
+        {
+            if( kb >= nbb ) { break; }
+#pragma unroll
+            for( int q = 0; q < 2; ++q )
             {
-                const int cc = pair >> 1, r = 32 * (pair & 1) + lane;
-                if( r >= nb ) { continue; }
-                const float v = static_cast<float>( X[r][cc] );
-                const unsigned hi = to_tf32( v );
-                const std::int64_t o = img_offset( t, t.r0 + r, t.c0 + cc, r1, m );
-                img[o] = __uint_as_float( hi );
-                img[o + lo_off] = __uint_as_float( to_tf32( v - __uint_as_float( hi ) ) );
+                const int k = kSub * kb + (lane & 3) + 4 * q;
+                const double b = X[k][c + fi];
+                const double * Tk = Ti[k] + fi;
+#pragma unroll
+                for( int rb = kb; rb < kSubs; ++rb ) { dmma_8x8x4( acc[rb], Tk[kSub * rb], b ); }   // (rb >= nbb: unused sums)
+            }
+        }
+#pragma unroll
+        for( int rb = 0; rb < kSubs; ++rb )
+        {
+            const int r = kSub * rb + fi;
+            if( r >= nb || c + fj >= cw ) { continue; }
+            T * dst = U + (std::int64_t)r * ld + c + fj;
+            const bool two = c + fj + 1 < cw;
+            const T v0 = static_cast<T>( acc[rb][0] ), v1 = static_cast<T>( acc[rb][1] );
+            if constexpr ( sizeof(T) == 8 )
+            {
+                if( two ) { *reinterpret_cast<double2 *>( dst ) = make_double2( v0, v1 ); }
+                else { dst[0] = v0; }
+            }
+            else
+            {
+                if( two ) { *reinterpret_cast<float2 *>( dst ) = make_float2( v0, v1 ); }
+                else { dst[0] = v0; }
+                if( img != nullptr && t.img >= 0 )
+                {
+                    // the stored FP32 values split into TF32 hi + lo, for the tensor-core tiles: the image
+                    // is K-major, so eight lanes write eight consecutive k of a column (one 32-byte sector)
+                    const std::int64_t lo_off = static_cast<std::int64_t>( t.img_tf ) * (kImgRows * kImgK);
+#pragma unroll
+                    for( int e = 0; e < 2; ++e )
+                    {
+                        if( e == 1 && !two ) { continue; }
+                        const float v = e == 0 ? v0 : v1;
+                        const unsigned hi = to_tf32( v );
+                        const std::int64_t o = img_offset( t, t.r0 + r, t.c0 + c + fj + e, r1, m );
+                        img[o] = __uint_as_float( hi );
+                        img[o + lo_off] = __uint_as_float( to_tf32( v - __uint_as_float( hi ) ) );
+                    }
+                }
             }
         }
     }
@@ -1201,9 +1221,7 @@ __global__ __launch_bounds__(kTrsmThreads) void trsm_kernel( const PanelTask * _
 {
     extern __shared__ __align__(16) double tsm[];
     pdl_allow_next();
-    const PanelTask t = tasks[blockIdx.x];
-    pdl_wait();
-    trsm_body( t, arena, tinv, tsm, img );
+    trsm_body<T, true>( tasks[blockIdx.x], arena, tinv, tsm, img );
 }
 
 // ------------------------------------------------------------------- gemm
@@ -2048,7 +2066,7 @@ __global__ __launch_bounds__(kDagThreads, 3) void factor_dag_kernel( const DagAr
             case LaunchKind::Zero:   zero_body( a.zero[t.index], arena ); break;
             case LaunchKind::Extend: extend_body( a.extend[t.index], a.lut, arena ); break;
             case LaunchKind::Potrf:  potrf_body<T, kDagThreads>( a.potrf[t.index], arena, a.status, a.pivot_floor, a.tinv ); break;
-            case LaunchKind::Trsm:   trsm_body( a.panel[t.index], arena, a.tinv, dsm ); break;
+            case LaunchKind::Trsm:   trsm_body<T, false>( a.panel[t.index], arena, a.tinv, dsm ); break;
             case LaunchKind::Gemm:
                 if constexpr ( sizeof(T) == 4 ) { gemm_body( a.gemm[t.index], arena, dsm, tc, a.status ); }
                 else { gemm_body( a.gemm[t.index], arena, dsm ); }

@@ -739,7 +739,7 @@ void Plan::build( const Symbolic & sym )
                 t.panel = pi;                   // == sdiag.size(): one potrf task and one SolveDiagTask per panel
                 t.img = front_img[f]; t.img_t0 = img_t0[f]; t.img_tf = img_tf[f];
                 if( small ) { fronts[static_cast<size_t>( front_task[at - n_large] )].p = t; }
-                else { ++large_potrf; large_trsm += static_cast<I32>( ceil_div( rest, kRestChunk ) ); }
+                else { ++large_potrf; large_trsm += static_cast<I32>( ceil_div( n0 - r1, kRestChunk ) + ceil_div( n1, kRestChunk ) ); }
                 {
                     PendingTask d = make( LaunchKind::Potrf, static_cast<I64>(potrf.size()) );
                     // the first panel starts once the children's contributions are in and
@@ -750,7 +750,8 @@ void Plan::build( const Symbolic & sym )
                     step_potrf[q].push_back( d );
                 }
                 potrf.push_back( t );
-                for( I32 c0 = 0; c0 < rest; c0 += kRestChunk )
+                // chunks end where U0's columns do
+                for( I32 c0 = 0; c0 < rest; c0 = std::min( c0 + kRestChunk, c0 < n0 - r1 ? n0 - r1 : rest ) )
                 {
                     t.c0 = c0;
                     PendingTask d = make( LaunchKind::Trsm, static_cast<I64>(panel.size()) );

@@ -74,8 +74,8 @@ struct GemmTask
 };
 
 // Panel [r0, r0+nb) of a front.  As a potrf task: factor the diagonal block
-// in place.  As a trsm task: solve the panel's rows for rest columns
-// [c0, c0 + kRestChunk) against the factored block: rest column j is U0
+// in place.  As a trsm task: solve the panel's rows for the (up to kRestChunk)
+// rest columns from c0 on, to the end of U0's or of U1's, against the factored block: rest column j is U0
 // column r0+nb+j when j < n0-r0-nb, else U1 column j-(n0-r0-nb).  row0 is
 // the front's first global row (failures report the failing global row);
 // bit r of single_rows marks panel rows that form a 1 x 1 reference

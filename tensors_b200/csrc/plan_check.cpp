@@ -266,6 +266,9 @@ std::string check_plan( const Symbolic & sym, const Plan & pl )
             const I32 nb = std::min( kPanel, t.n0 - t.r0 );
             const I32 rest = (t.n0 - t.r0 - nb) + t.n1;
             if( which == 1 && (t.c0 < 0 || t.c0 >= rest) ) { return "panel chunk out of range" + at(); }
+            // (16-byte pieces: chunks start on multiples of kRestChunk inside U0 and inside U1)
+            if( which == 1 && (t.c0 < t.n0 - t.r0 - nb ? t.c0 : t.c0 - (t.n0 - t.r0 - nb)) % kRestChunk != 0 ) { return "panel chunk not aligned" + at(); }
+            if( (t.u0 | t.u1) % 4 != 0 || (t.ld0 | t.ld1) % 4 != 0 || t.r0 % kPanel != 0 ) { return "panel not 16-byte aligned" + at(); }
             if( t.row0 < 0 || t.row0 + t.n0 > sym.n ) { return "panel rows out of range" + at(); }
             // the inverse diagonal block: one per panel, written by the panel's potrf task
             if( t.panel < 0 || t.panel >= static_cast<I32>( pl.sdiag.size() ) ) { return "panel index out of range" + at(); }
