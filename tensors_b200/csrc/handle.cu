@@ -115,7 +115,9 @@ struct tb_chol
     // second stream of the level schedule: the GEMM tiles of a panel step that
     // do not touch the next panel run there, overlapping the next potrf / trsm
     cudaStream_t side = nullptr;
-    cudaEvent_t ev_trsm = nullptr, ev_soon = nullptr, ev_rest = nullptr;
+    // third stream (FP64): the next panel's rows without their diagonal block, beside its potrf
+    cudaStream_t row = nullptr;
+    cudaEvent_t ev_trsm = nullptr, ev_row = nullptr, ev_soon = nullptr, ev_rest = nullptr;
 
     // input pattern (copied, CholeskyDecomposition.hpp:313-371)
     std::int32_t n = 0;
@@ -247,6 +249,8 @@ struct tb_chol
         if( factor_graph ) { cudaGraphExecDestroy( factor_graph ); }
         if( own_stream && stream ) { cudaStreamDestroy( stream ); }
         if( side ) { cudaStreamDestroy( side ); }
+        if( row ) { cudaStreamDestroy( row ); }
+        if( ev_row ) { cudaEventDestroy( ev_row ); }
         if( ev_trsm ) { cudaEventDestroy( ev_trsm ); }
         if( ev_soon ) { cudaEventDestroy( ev_soon ); }
         if( ev_rest ) { cudaEventDestroy( ev_rest ); }
@@ -356,6 +360,8 @@ int ensure_device( tb_chol * h )
     {
         TB_CUDA( cudaStreamCreateWithFlags( &h->side, cudaStreamNonBlocking ) );
         TB_CUDA( cudaEventCreateWithFlags( &h->ev_trsm, cudaEventDisableTiming ) );
+        TB_CUDA( cudaStreamCreateWithFlags( &h->row, cudaStreamNonBlocking ) );
+        TB_CUDA( cudaEventCreateWithFlags( &h->ev_row, cudaEventDisableTiming ) );
         TB_CUDA( cudaEventCreateWithFlags( &h->ev_soon, cudaEventDisableTiming ) );
         TB_CUDA( cudaEventCreateWithFlags( &h->ev_rest, cudaEventDisableTiming ) );
     }
@@ -520,7 +526,7 @@ std::int64_t issue_factor_t( tb_chol * h, bool timed, std::vector<int> * kinds )
                     tb::launch_extend_pull( h->extend_pull.ptr + L.first, L.count, h->extend_segs.ptr, h->lut.ptr, A, st );
                     break;
                 case tb::LaunchKind::Potrf:  tb::launch_potrf( h->potrf.ptr + L.first, L.count, A, h->status.ptr, floor, h->tinv.ptr, st ); break;
-                case tb::LaunchKind::Trsm:   tb::launch_trsm( h->panel.ptr + L.first, L.count, A, h->tinv.ptr, st, img ); break;
+                case tb::LaunchKind::Trsm:   tb::launch_trsm( h->panel.ptr + L.first, L.count, A, h->tinv.ptr, st, img, true ); break;
                 case tb::LaunchKind::Gemm:   issue_gemm( h, L, A, st ); break;
                 default: break;
             }
@@ -546,32 +552,44 @@ std::int64_t issue_factor_t( tb_chol * h, bool timed, std::vector<int> * kinds )
         }
         return launches;
     }
-    // Look-ahead over two streams (the profiled path keeps one, so that every
-    // launch is timed alone).  Main stream: potrf(q), trsm(q), the tiles of
-    // step q that update panel q+1's rows (part 0).  Side stream: the other
-    // tiles of step q, after trsm(q): first the rows of the panels up to the
+    // Look-ahead over three streams (the profiled path keeps one, so that every
+    // launch is timed alone).  Main stream: potrf(q), trsm(q).  Row stream,
+    // after trsm(q): the tiles of step q that update panel q+1's rows (part 0;
+    // FP64: without the diagonal block, which potrf(q+1) updates itself, so that
+    // only trsm(q+1) waits for it; FP32: on the main stream).  Side stream, after
+    // trsm(q): the other tiles of step q, first the rows of the panels up to the
     // next full update (part 1), then the rest (part 2), which runs while the
-    // main stream goes through the next defer_steps panels.  Part 0 of a step
-    // waits for the part 1 of the last full update; part 0 of a full update for
-    // its part 2, which wrote panel q+1's rows last.  Each C tile keeps the
+    // main stream goes through the next defer_steps panels.  What panel q+1's
+    // rows wait for besides: the part 1 of the last full update, at a full
+    // update also its part 2, which wrote them last.  Each C tile keeps the
     // order of its updates, so the factor is the same bit for bit.  Levels join
-    // the side stream at their boundaries (the next extend-adds read the update
-    // matrices the part-2 tiles write).
+    // the other streams at their boundaries (the next extend-adds read the
+    // update matrices the part-2 tiles write).
     const bool overlap = !timed && h->side != nullptr;
-    bool soon_busy = false, rest_busy = false;       // side-stream work of parts 1 / 2 the main stream has not waited for
+    const bool row_stream = overlap && sizeof(T) == 8;
+    // work of parts 0 / 1 / 2 on the other streams that the main stream has not waited for
+    bool row_busy = false, soon_busy = false, rest_busy = false;
     std::int32_t level = -1;
-    auto join = [&]()
+    auto wait_row = [&]()
     {
-        if( rest_busy || soon_busy )
-        {
-            cudaEventRecord( h->ev_rest, h->side );
-            cudaStreamWaitEvent( st, h->ev_rest, 0 );
-        }
-        soon_busy = rest_busy = false;
+        if( row_busy ) { cudaStreamWaitEvent( st, h->ev_row, 0 ); }
+        row_busy = false;
     };
+    auto wait_side = [&]( bool all )
+    {
+        if( all && rest_busy )
+        {
+            cudaStreamWaitEvent( st, h->ev_rest, 0 );
+            rest_busy = false;
+        }
+        if( soon_busy ) { cudaStreamWaitEvent( st, h->ev_soon, 0 ); }
+        soon_busy = false;
+    };
+    auto join = [&]() { wait_row(); wait_side( true ); };
     for( const tb::Launch & L : level_launches( h ) )
     {
         cudaStream_t s = st;
+        bool after_potrf = true;                     // a trsm that waits for its potrf alone
         if( overlap )
         {
             if( L.level != level ) { join(); level = L.level; }
@@ -581,21 +599,16 @@ std::int64_t issue_factor_t( tb_chol * h, bool timed, std::vector<int> * kinds )
                 cudaEventRecord( h->ev_trsm, st );
                 cudaStreamWaitEvent( h->side, h->ev_trsm, 0 );
                 s = h->side;
-                rest_busy = true;
             }
-            if( L.kind == tb::LaunchKind::Gemm )
+            if( L.kind == tb::LaunchKind::Trsm )
             {
-                if( L.part == 0 )
-                {
-                    if( L.step % pl.defer_steps == pl.defer_steps - 1 ) { join(); }
-                    else if( soon_busy ) { cudaStreamWaitEvent( st, h->ev_soon, 0 ); soon_busy = false; }
-                }
-                else
-                {
-                    cudaStreamWaitEvent( h->side, h->ev_trsm, 0 );
-                    s = h->side;
-                    (L.part == 1 ? soon_busy : rest_busy) = true;
-                }
+                after_potrf = !row_busy;
+                wait_row();
+            }
+            if( L.kind == tb::LaunchKind::Gemm && (L.part > 0 || row_stream) )
+            {
+                s = L.part > 0 ? h->side : h->row;
+                cudaStreamWaitEvent( s, h->ev_trsm, 0 );
             }
         }
         switch( L.kind )
@@ -612,13 +625,25 @@ std::int64_t issue_factor_t( tb_chol * h, bool timed, std::vector<int> * kinds )
                                        h->tinv.ptr, s );
                 }
                 break;
-            case tb::LaunchKind::Potrf:  tb::launch_potrf( h->potrf.ptr + L.first, L.count, A, h->status.ptr, floor, h->tinv.ptr, s ); break;
-            case tb::LaunchKind::Trsm:   tb::launch_trsm( h->panel.ptr + L.first, L.count, A, h->tinv.ptr, s, img ); break;
+            case tb::LaunchKind::Potrf:
+                tb::launch_potrf( h->potrf.ptr + L.first, L.count, A, h->status.ptr, floor, h->tinv.ptr, s, sizeof(T) == 8 );
+                break;
+            case tb::LaunchKind::Trsm:   tb::launch_trsm( h->panel.ptr + L.first, L.count, A, h->tinv.ptr, s, img, after_potrf ); break;
             case tb::LaunchKind::Gemm:   issue_gemm( h, L, A, s ); break;
             default: break;
         }
-        if( overlap && L.kind == tb::LaunchKind::Trsm ) { cudaEventRecord( h->ev_trsm, st ); }
-        if( overlap && L.kind == tb::LaunchKind::Gemm && L.part == 1 ) { cudaEventRecord( h->ev_soon, h->side ); }
+        if( overlap && L.kind == tb::LaunchKind::Trsm )
+        {
+            wait_side( L.step % pl.defer_steps == pl.defer_steps - 1 );
+            cudaEventRecord( h->ev_trsm, st );
+        }
+        if( s != st && overlap )
+        {
+            const bool front = L.kind == tb::LaunchKind::Front;
+            if( !front && L.part == 0 ) { cudaEventRecord( h->ev_row, s ); row_busy = true; }
+            else if( !front && L.part == 1 ) { cudaEventRecord( h->ev_soon, s ); soon_busy = true; }
+            else { cudaEventRecord( h->ev_rest, s ); rest_busy = true; }
+        }
         mark( static_cast<int>( L.kind == tb::LaunchKind::ExtendPull ? tb::LaunchKind::Extend : L.kind == tb::LaunchKind::Front ? tb::LaunchKind::Solve : L.kind ) );
         ++launches;
     }

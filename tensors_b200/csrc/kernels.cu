@@ -757,7 +757,12 @@ __device__ __forceinline__ void potrf_core( const PotrfShared<kLd> & sh, const P
 }
 
 // The panel's diagonal block (64 x kPld cells of dynamic shared memory), then potrf_core.
-template<typename T, int kThreads>
+// kPend (FP64): the t.pend pending rows' update of the block comes first, D -= P^T P with P the rows
+// r0 - pend .. r0 - 1 of the block's columns, in chunks of 64 rows through T's and D's space; a warp
+// holds three of the 36 upper 8 x 8 tiles.  The panel chain is then trsm -> potrf, with the rest of
+// the row's update beside the potrf, instead of trsm -> GEMM -> potrf (a launch of 8-20 us).  The K
+// order and the single subtraction are the GEMM tile's: the same bits.
+template<typename T, int kThreads, bool kPend>
 __device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict__ arena, int * __restrict__ status,
                                             const double * __restrict__ pivot_floor, double * __restrict__ tinv )
 {
@@ -772,6 +777,76 @@ __device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict_
     sh.flags = reinterpret_cast<int *>( sh.floor_s + kPanel );
 
     T * U0 = arena + t.u0 + (std::int64_t)t.r0 * t.ld0 + t.r0;
+    if constexpr ( kPend )
+    {
+        static_assert( sizeof(T) == 8 && kThreads == 384, "12 warps hold 36 tiles" );
+        if( t.pend > 0 )
+        {
+            const int lane = tid & 31, warp = tid >> 5;
+            const int nch = t.pend / kPanel;
+            const T * P = arena + t.u0 + (std::int64_t)(t.r0 - t.pend) * t.ld0 + t.r0;
+            auto load_chunk = [&]( int ch )
+            {
+                double * dst = (ch & 1) ? sh.d : sh.ti;
+                for( int idx = 2 * tid; idx < kPanel * kPanel; idx += 2 * kThreads )
+                {
+                    const int r = idx / kPanel, c = idx % kPanel;
+                    cp_async_16( dst + r * kPld + c, c < nb ? P + (std::int64_t)(ch * kPanel + r) * t.ld0 + c : P, c + 1 < nb ? 16 : c < nb ? 8 : 0 );
+                }
+                cp_async_commit();
+            };
+            // tiles (ti, tj) of warp w: the w-th, 12 + w-th and 24 + w-th of the upper ones, by columns
+            int ti[3], tj[3];
+#pragma unroll
+            for( int e = 0; e < 3; ++e )
+            {
+                int left = warp + 12 * e, col = 0;
+                while( left > col ) { left -= col + 1; ++col; }
+                ti[e] = left;
+                tj[e] = col;
+            }
+            double acc[3][2];
+#pragma unroll
+            for( int e = 0; e < 3; ++e ) { acc[e][0] = 0.0; acc[e][1] = 0.0; }
+            load_chunk( 0 );
+            if( nch > 1 ) { load_chunk( 1 ); }
+            for( int ch = 0; ch < nch; ++ch )
+            {
+                if( ch + 1 < nch ) { cp_async_wait<1>(); } else { cp_async_wait<0>(); }
+                __syncthreads();
+                const double * src = ((ch & 1) ? sh.d : sh.ti) + (lane >> 2);
+#pragma unroll 4
+                for( int k = lane & 3; k < kPanel; k += 4 )
+                {
+#pragma unroll
+                    for( int e = 0; e < 3; ++e ) { dmma_8x8x4( acc[e], src[k * kPld + kSub * ti[e]], src[k * kPld + kSub * tj[e]] ); }
+                }
+                __syncthreads();
+                if( ch + 2 < nch ) { load_chunk( ch + 2 ); }
+            }
+#pragma unroll
+            for( int e = 0; e < 3; ++e )
+            {
+                const int r = kSub * ti[e] + (lane >> 2), c = kSub * tj[e] + 2 * (lane & 3);
+                double2 v = make_double2( r == c ? 1.0 : 0.0, r == c + 1 ? 1.0 : 0.0 );   // identity beyond nb
+                if( r < nb )
+                {
+                    // (below the diagonal of a diagonal tile: zeros, never used)
+                    v = make_double2( 0.0, 0.0 );
+                    const T * src = U0 + (std::int64_t)r * t.ld0 + c;
+                    if( c + 1 < nb ) { v = *reinterpret_cast<const double2 *>( src ); }
+                    else if( c < nb ) { v.x = src[0]; }
+                    if( c < nb ) { v.x -= acc[e][0]; }
+                    if( c + 1 < nb ) { v.y -= acc[e][1]; }
+                }
+                *reinterpret_cast<double2 *>( &sh.D( r, c ) ) = v;
+            }
+            if( tid == 0 ) { sh.fail() = -1; sh.redo() = 0; sh.raised() = 0; }
+            __syncthreads();
+            potrf_core<T, kThreads>( sh, t, nb, arena, status, pivot_floor, tinv );
+            return;
+        }
+    }
     // 16-byte pieces of the rows (16-byte aligned: offsets and leading dimensions are multiples of
     // kLdAlign entries), all of a thread's in flight together; pieces below the diagonal are not read
     // later and not loaded; identity padding beyond nb
@@ -820,7 +895,7 @@ __device__ __forceinline__ void potrf_body( const PanelTask & t, T * __restrict_
     potrf_core<T, kThreads>( sh, t, nb, arena, status, pivot_floor, tinv );
 }
 
-template<typename T>
+template<typename T, bool kPend>
 __global__ __launch_bounds__(kPotrfThreads, 1) void potrf_kernel( const PanelTask * __restrict__ tasks,
                                                                T * __restrict__ arena, int * __restrict__ status,
                                                                const double * __restrict__ pivot_floor,
@@ -828,10 +903,10 @@ __global__ __launch_bounds__(kPotrfThreads, 1) void potrf_kernel( const PanelTas
 {
     const PanelTask t = tasks[blockIdx.x];
     pdl_wait();
-    // only now: the trsm reads the rest columns before its own wait, so everything before this
-    // launch must be complete when it starts
+    // only now: the trsm may read the rest columns before its own wait (kPrefetch), so everything
+    // before this launch must be complete when it starts
     pdl_allow_next();
-    potrf_body<T, kPotrfThreads>( t, arena, status, pivot_floor, tinv );
+    potrf_body<T, kPotrfThreads, kPend>( t, arena, status, pivot_floor, tinv );
 }
 
 // ------------------------------------------------------------ small fronts
@@ -1072,8 +1147,7 @@ void front_kernel( const FrontTask * __restrict__ tasks, const ExtendTask * __re
 // with all eight row blocks' sums in registers: 72 independent-by-eight DMMAs
 // follow 88 fragment loads, and the results go to global memory from the
 // registers.  Bound: the launch's latency (load, 72 DMMAs a warp, store) on
-// the panel chain, so the rest columns are loaded before the wait on the
-// potrf, which writes only the diagonal block and T.
+// the panel chain.
 // Operand-image entry of U row k, rest column `col` of a panel whose rest
 // columns start at U0 column r1 (m of them in U0, the rest U1 columns).
 __device__ __forceinline__ std::int64_t img_offset( const PanelTask & t, int k, int col, int r1, int m )
@@ -1084,7 +1158,11 @@ __device__ __forceinline__ std::int64_t img_offset( const PanelTask & t, int k, 
     return blk * (kImgRows * kImgK) + (ucol % kImgRows) * kImgK + (k % kImgK);
 }
 
-template<typename T, bool kPdl>
+// kPrefetch: the launch before is the potrf, which let this one start only
+// after its own wait, and nothing else is waited for: the rest columns are
+// loaded before the wait.  (FP64 level launches: their update runs on another
+// stream, so that the wait comes first.)
+template<typename T, bool kPdl, bool kPrefetch>
 __device__ __forceinline__ void trsm_body( const PanelTask & t, T * __restrict__ arena, const double * __restrict__ tinv,
                                            double * tsm, float * __restrict__ img = nullptr )
 {
@@ -1105,6 +1183,7 @@ __device__ __forceinline__ void trsm_body( const PanelTask & t, T * __restrict__
     constexpr int kV = 16 / static_cast<int>( sizeof(T) );
     constexpr int kPieces = kPanel * kRestChunk / kV / kTrsmThreads;
     [[maybe_unused]] float4 xf[sizeof(T) == 4 ? kPieces : 1];
+    if constexpr ( kPdl && !kPrefetch ) { pdl_wait(); }
 #pragma unroll
     for( int u = 0; u < kPieces; ++u )
     {
@@ -1113,7 +1192,7 @@ __device__ __forceinline__ void trsm_body( const PanelTask & t, T * __restrict__
         if constexpr ( sizeof(T) == 8 ) { cp_async_16( &X[r][c], in ? U + (std::int64_t)r * ld + c : U, in ? (c + 1 < cw ? 16 : 8) : 0 ); }
         else { xf[u] = in ? *reinterpret_cast<const float4 *>( U + (std::int64_t)r * ld + c ) : make_float4( 0.f, 0.f, 0.f, 0.f ); }
     }
-    if constexpr ( kPdl ) { pdl_wait(); }
+    if constexpr ( kPdl && kPrefetch ) { pdl_wait(); }
     {
         // only the leading (nb rounded up to 8)^2 block of T is read
         const double * Tg = tinv + (std::int64_t)t.panel * (kPanel * kPanel);
@@ -1214,14 +1293,14 @@ __device__ __forceinline__ void trsm_body( const PanelTask & t, T * __restrict__
     }
 }
 
-template<typename T>
+template<typename T, bool kPrefetch>
 __global__ __launch_bounds__(kTrsmThreads) void trsm_kernel( const PanelTask * __restrict__ tasks,
                                                              T * __restrict__ arena, const double * __restrict__ tinv,
                                                              float * __restrict__ img )
 {
     extern __shared__ __align__(16) double tsm[];
     pdl_allow_next();
-    trsm_body<T, true>( tasks[blockIdx.x], arena, tinv, tsm, img );
+    trsm_body<T, true, kPrefetch>( tasks[blockIdx.x], arena, tinv, tsm, img );
 }
 
 // ------------------------------------------------------------------- gemm
@@ -2065,8 +2144,8 @@ __global__ __launch_bounds__(kDagThreads, 3) void factor_dag_kernel( const DagAr
         {
             case LaunchKind::Zero:   zero_body( a.zero[t.index], arena ); break;
             case LaunchKind::Extend: extend_body( a.extend[t.index], a.lut, arena ); break;
-            case LaunchKind::Potrf:  potrf_body<T, kDagThreads>( a.potrf[t.index], arena, a.status, a.pivot_floor, a.tinv ); break;
-            case LaunchKind::Trsm:   trsm_body<T, false>( a.panel[t.index], arena, a.tinv, dsm ); break;
+            case LaunchKind::Potrf:  potrf_body<T, kDagThreads, false>( a.potrf[t.index], arena, a.status, a.pivot_floor, a.tinv ); break;
+            case LaunchKind::Trsm:   trsm_body<T, false, false>( a.panel[t.index], arena, a.tinv, dsm ); break;
             case LaunchKind::Gemm:
                 if constexpr ( sizeof(T) == 4 ) { gemm_body( a.gemm[t.index], arena, dsm, tc, a.status ); }
                 else { gemm_body( a.gemm[t.index], arena, dsm ); }
@@ -2714,9 +2793,13 @@ void launch_fronts( const FrontTask * tasks, int count, int threads, int smem, c
 
 template<typename T>
 void launch_potrf( const PanelTask * tasks, int count, T * arena, int * status, const double * pivot_floor, double * tinv,
-                   cudaStream_t st )
+                   cudaStream_t st, bool pending )
 {
-    if( count > 0 ) { launch_pdl( potrf_kernel<T>, count, kPotrfThreads, kPotrfSmemBytes, st, tasks, arena, status, pivot_floor, tinv ); }
+    if constexpr ( sizeof(T) == 8 )
+    {
+        if( count > 0 && pending ) { launch_pdl( potrf_kernel<T, true>, count, kPotrfThreads, kPotrfSmemBytes, st, tasks, arena, status, pivot_floor, tinv ); return; }
+    }
+    if( count > 0 ) { launch_pdl( potrf_kernel<T, false>, count, kPotrfThreads, kPotrfSmemBytes, st, tasks, arena, status, pivot_floor, tinv ); }
 }
 
 // floor[i] = rel * |diagonal entry of row i| after assembly (FP32 storage).
@@ -2749,9 +2832,11 @@ void launch_pivot_floor( const std::int64_t * offsets, const float * arena, doub
 }
 
 template<typename T>
-void launch_trsm( const PanelTask * tasks, int count, T * arena, const double * tinv, cudaStream_t st, float * img )
+void launch_trsm( const PanelTask * tasks, int count, T * arena, const double * tinv, cudaStream_t st, float * img, bool after_potrf )
 {
-    if( count > 0 ) { launch_pdl( trsm_kernel<T>, count, kTrsmThreads, kTrsmSmemBytes, st, tasks, arena, tinv, img ); }
+    if( count <= 0 ) { return; }
+    if( after_potrf ) { launch_pdl( trsm_kernel<T, true>, count, kTrsmThreads, kTrsmSmemBytes, st, tasks, arena, tinv, img ); }
+    else { launch_pdl( trsm_kernel<T, false>, count, kTrsmThreads, kTrsmSmemBytes, st, tasks, arena, tinv, img ); }
 }
 
 template<typename T>
@@ -2922,8 +3007,8 @@ void launch_gather_diag( const std::int64_t * offsets, const T * arena, double *
                                     cudaStream_t );                                                                \
     template void launch_extend<T>( const ExtendTask *, int, const std::int32_t *, T *, cudaStream_t );             \
     template void launch_extend_pull<T>( const ExtendPullTask *, int, const ExtendTask *, const std::int32_t *, T *, cudaStream_t ); \
-    template void launch_potrf<T>( const PanelTask *, int, T *, int *, const double *, double *, cudaStream_t );     \
-    template void launch_trsm<T>( const PanelTask *, int, T *, const double *, cudaStream_t, float * );              \
+    template void launch_potrf<T>( const PanelTask *, int, T *, int *, const double *, double *, cudaStream_t, bool );     \
+    template void launch_trsm<T>( const PanelTask *, int, T *, const double *, cudaStream_t, float *, bool );              \
     template void launch_gemm<T>( const GemmTask *, int, T *, int *, cudaStream_t );                                 \
     template void launch_solve_dag<T>( const SolveDagArgs &, int, const T *, double *, double *, int, int, cudaStream_t );                                        \
     template void launch_factor_dag<T>( const DagArgs &, int, cudaStream_t );                                        \
@@ -2975,10 +3060,13 @@ cudaError_t configure_kernels()
         { reinterpret_cast<const void *>( front_kernel<128> ), kFrontSmemSmall },
         { reinterpret_cast<const void *>( front_kernel<256> ), kFrontSmemMid },
         { reinterpret_cast<const void *>( front_kernel<384> ), kFrontSmemMax },
-        { reinterpret_cast<const void *>( potrf_kernel<double> ), kPotrfSmemBytes },
-        { reinterpret_cast<const void *>( potrf_kernel<float> ), kPotrfSmemBytes },
-        { reinterpret_cast<const void *>( trsm_kernel<double> ), kTrsmSmemBytes },
-        { reinterpret_cast<const void *>( trsm_kernel<float> ), kTrsmSmemBytes },
+        { reinterpret_cast<const void *>( potrf_kernel<double, false> ), kPotrfSmemBytes },
+        { reinterpret_cast<const void *>( potrf_kernel<double, true> ), kPotrfSmemBytes },
+        { reinterpret_cast<const void *>( potrf_kernel<float, false> ), kPotrfSmemBytes },
+        { reinterpret_cast<const void *>( trsm_kernel<double, false> ), kTrsmSmemBytes },
+        { reinterpret_cast<const void *>( trsm_kernel<double, true> ), kTrsmSmemBytes },
+        { reinterpret_cast<const void *>( trsm_kernel<float, false> ), kTrsmSmemBytes },
+        { reinterpret_cast<const void *>( trsm_kernel<float, true> ), kTrsmSmemBytes },
         { reinterpret_cast<const void *>( gemm_tn_kernel ), kGemmSmemBytes },
         { reinterpret_cast<const void *>( gemm_tc_kernel ), kGemmSmemBytesF },
         { reinterpret_cast<const void *>( factor_dag_kernel<double> ), kDagSmemBytes },

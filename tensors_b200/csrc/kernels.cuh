@@ -36,15 +36,18 @@ void launch_fronts( const FrontTask * tasks, int count, int threads, int smem, c
 // element 1 + i the value a non-positive or lost pivot of permuted row i is
 // raised to instead of failing; status[2] counts them.
 // tinv: per panel (PanelTask::panel) the 64 x 64 inverse of its diagonal block, written here.
+// pending (FP64): the tasks' pending rows (PanelTask::pend) update the block first.
 template<typename T> void launch_potrf( const PanelTask * tasks, int count, T * arena, int * status,
-                                        const double * pivot_floor, double * tinv, cudaStream_t st );
+                                        const double * pivot_floor, double * tinv, cudaStream_t st, bool pending = false );
 // out (n + 1 doubles): the pivot floors in the layout of launch_potrf's pivot_floor.
 void launch_pivot_floor( const std::int64_t * offsets, const float * arena, double rel, double * out, int n, cudaStream_t st );
 // Uses the inverse diagonal blocks the panels' potrf wrote to tinv.  img
 // (FP32 path, else null): the operand image the trsm also writes its panel
 // rows into, split into TF32 hi and lo (tasks with PanelTask::img >= 0).
+// after_potrf: the only thing the launch waits for is the panels' potrf, the
+// launch before it on the stream (the rest columns are then loaded early).
 template<typename T> void launch_trsm( const PanelTask * tasks, int count, T * arena, const double * tinv, cudaStream_t st,
-                                       float * img = nullptr );
+                                       float * img, bool after_potrf );
 // status[0] gets kStatusTcTimeout (2) when a tensor-core completion wait of
 // the FP32 path ran out (its tile is then not updated).
 template<typename T> void launch_gemm( const GemmTask * tasks, int count, T * arena, int * status, cudaStream_t st );

@@ -736,6 +736,7 @@ void Plan::build( const Symbolic & sym )
                 t.ld0 = ld0; t.ld1 = ld1;
                 t.row0 = front_row0[f];
                 t.single_rows = singles;
+                t.pend = q > 0 ? kPanel * ((q - 1) % defer_steps + 1) : 0;
                 t.panel = pi;                   // == sdiag.size(): one potrf task and one SolveDiagTask per panel
                 t.img = front_img[f]; t.img_t0 = img_t0[f]; t.img_tf = img_tf[f];
                 if( small ) { fronts[static_cast<size_t>( front_task[at - n_large] )].p = t; }
@@ -812,9 +813,14 @@ void Plan::build( const Symbolic & sym )
                                  front_v[f], ld1, n1, n1, true, tc_nmax );
                     }
                 }
-                // the order of a step's tiles (within a part): taken whole without an image, others
+                // the order of a step's tiles (within a part): fronts taken whole without an image, others
                 // without, others with, taken whole with an image
-                for( size_t i = tfirst; i < tiles.size(); ++i ) { tile_small.push_back( front_img[f] < 0 ? (small ? 3 : 2) : (small ? 0 : 1) ); }
+                // (left out with them: the next panel's diagonal block, PanelTask::pend)
+                for( size_t i = tfirst; i < tiles.size(); ++i )
+                {
+                    const bool out = small || (tile_next[i] == 2 && tiles[i].upper && tiles[i].m0 == 0 && tiles[i].c0 == 0);
+                    tile_small.push_back( front_img[f] < 0 ? (out ? 3 : 2) : (out ? 0 : 1) );
+                }
                 for( size_t i = tfirst; i < tiles.size(); ++i ) { tile_panel.push_back( pi ); tile_prev.push_back( prev ); }
                 {
                     SolveRestTask t{};

@@ -91,6 +91,9 @@ struct PanelTask
     std::int64_t single_rows;      // bit r set: panel row r is a 1 x 1 reference supernode
     std::int64_t img;              // FP32 path: the front's first operand-image block (see TcTask)
     std::int32_t img_t0, img_tf;   // its U0 column tiles, and U0 + U1 column tiles per k-chunk segment
+    std::int32_t pend;             // potrf, FP64 level launches: rows r0 - pend .. r0 - 1 whose update of the diagonal
+                                   // block the potrf applies itself (the other launches have a GEMM tile for it)
+    std::int32_t pad;
 };
 
 // The FP32 path's Schur-complement tiles on the 5th-generation tensor cores
@@ -299,8 +302,11 @@ struct SuperSolveTask
 
 // One launch: `count` tasks starting at `first` in the array of its kind.
 // A panel step's GEMM tiles come as up to three launches: part 0 updates the
-// next panel's rows (the next potrf / trsm wait for it); part 1 the rows of the
-// panels after it up to the next full update, whose steps' part 0 wait for it;
+// next panel's rows (the next potrf / trsm wait for it; in the FP64 level
+// launches without the diagonal block, which the potrf updates itself, so that
+// only the trsm waits and the potrf runs beside it); part 1 the rows of the
+// panels after it up to the next full update, whose steps' part 0 (and, FP64,
+// potrf) wait for it;
 // part 2 the rest of the trailing matrix and the update matrices, which only
 // the next full update and the level's end wait for, so that it overlaps
 // defer_steps panel steps.  (128-row tensor-core tiles may reach a part's rows

@@ -226,7 +226,10 @@ std::string check_plan( const Symbolic & sym, const Plan & pl )
                 }
                 case LaunchKind::Gemm:
                 {
-                    // (a small front's only tiles are those of its update matrix)
+                    // (a small front's only tiles are those of its update matrix; the diagonal block of the
+                    // next panel's rows is the potrf's, like a small front's task)
+                    const GemmTask & g = pl.gemm[static_cast<size_t>( k )];
+                    if( L.part == 0 && g.upper && g.m0 == 0 && g.c0 == 0 ) { return 1; }
                     const auto v = by_v.find( { L.level, pl.gemm[static_cast<size_t>( k )].c } );
                     return v == by_v.end() ? 0 : pl.front_small[static_cast<size_t>( v->second )];
                 }
@@ -273,6 +276,7 @@ std::string check_plan( const Symbolic & sym, const Plan & pl )
             // the inverse diagonal block: one per panel, written by the panel's potrf task
             if( t.panel < 0 || t.panel >= static_cast<I32>( pl.sdiag.size() ) ) { return "panel index out of range" + at(); }
             if( which == 0 && t.panel != static_cast<I32>( k ) ) { return "potrf task is not its panel's" + at(); }
+            if( which == 0 && t.pend != (t.r0 > 0 ? kPanel * ((t.r0 / kPanel - 1) % pl.defer_steps + 1) : 0) ) { return "potrf task's pending rows" + at(); }
             if( which == 1 && (pl.potrf[static_cast<size_t>( t.panel )].r0 != t.r0 || pl.potrf[static_cast<size_t>( t.panel )].u0 != t.u0) )
             {
                 return "trsm task names another panel" + at();
