@@ -547,7 +547,7 @@ std::int64_t issue_factor_t( tb_chol * h, bool timed, std::vector<int> * kinds )
         launches += pl.dag.empty() ? 0 : 1;
         for( const tb::Launch & L : pl.sinv_launches )
         {
-            tb::launch_super_inv( h->sinv.ptr + L.first, L.count, h->spanels.ptr, A, h->tinv.ptr, h->tsuper.ptr, st );
+            tb::launch_super_inv( h->sinv.ptr + L.first, L.count, L.part, h->spanels.ptr, A, h->tinv.ptr, h->tsuper.ptr, st );
             ++launches;
         }
         return launches;
@@ -651,7 +651,7 @@ std::int64_t issue_factor_t( tb_chol * h, bool timed, std::vector<int> * kinds )
     // the large fronts' super-panel inverses for the solves (after every panel inverse exists)
     for( const tb::Launch & L : pl.sinv_launches )
     {
-        tb::launch_super_inv( h->sinv.ptr + L.first, L.count, h->spanels.ptr, A, h->tinv.ptr, h->tsuper.ptr, st );
+        tb::launch_super_inv( h->sinv.ptr + L.first, L.count, L.part, h->spanels.ptr, A, h->tinv.ptr, h->tsuper.ptr, st );
         mark( static_cast<int>( tb::LaunchKind::Invert ) );
         ++launches;
     }

@@ -2463,108 +2463,153 @@ int grid_for( std::int64_t work, int threads )
 constexpr int kSld = kPanel + 1;                        // padded smem row of a 64 x 64 block
 // Doubles of shared memory a 64 x kSld block of T takes (rounded up to 16 bytes).
 template<typename T> __host__ __device__ constexpr int super_block_doubles() { return ((kPanel * kSld * static_cast<int>( sizeof(T) ) + 15) / 16) * 2; }
-constexpr size_t kSuperInvSmem = sizeof(double) * 2 * kPanel * kSld;
 
 __device__ __forceinline__ int super_block_rows( const SuperPanel & sp, int b ) { return min( kPanel, sp.rows - b * kPanel ); }
 
-// acc[ct] (this warp's rows of 8 x 8 tile ct) += A(64 x 64) B(64 x 64) with A through a(i, k), B through b(k, j).
-template<typename FA, typename FB>
-__device__ __forceinline__ void block_product_64( double (&acc)[8][2], FA a, FB b )
-{
-    const int warp = threadIdx.x >> 5;
-    for( int kb = 0; kb < kSubs; ++kb )
-    {
-#pragma unroll
-        for( int ct = 0; ct < 8; ++ct )
-        {
-            dmma_8x8x8( acc[ct], [&]( int i, int k ) { return a( 8 * warp + i, 8 * kb + k ); },
-                                 [&]( int k, int j ) { return b( 8 * kb + k, 8 * ct + j ); } );
-        }
-    }
-}
+// One 64 x 64 block product of a super-panel's inverse (SuperInvTask): part 0
+// W_ij = sum_k U_ik T_kj, part 1 T_ij = -sum_k T_ik W_kj, or the copy of panel
+// i's inverse.  The sum over k streams through two stages of 32 columns of the
+// left and 32 rows of the right blocks.  Doubling needs 14 block products in a
+// row where the back substitution by distance from the diagonal needed 35
+// (C2: 370 us in eight launches); diagonal blocks are read from the panels'
+// inverses.
+constexpr int kInvK = 32;
+constexpr int kInvLda = kInvK + 4;                      // (conflict-free DMMA fragments, as kPld)
+constexpr int kInvStage = kPanel * kInvLda + kInvK * kPld;
+constexpr size_t kSuperInvSmem = sizeof(double) * 2 * kInvStage;
 
-// One block (i, j) of a super-panel's inverse (round j - i; rounds run in
-// order, so the blocks T_kj with k > i are complete): T_ii is panel i's
-// inverse (its nb x nb part), T_ij = -T_ii sum_{k=i+1..j} U_ik T_kj.
 template<typename T>
-__global__ __launch_bounds__(256) void super_inv_kernel( const SuperInvTask * __restrict__ tasks, const SuperPanel * __restrict__ sps,
+__global__ __launch_bounds__(256) void super_inv_kernel( const SuperInvTask * __restrict__ tasks, int part, const SuperPanel * __restrict__ sps,
                                                          const T * __restrict__ arena, const double * __restrict__ tinv,
                                                          double * __restrict__ tbuf )
 {
     extern __shared__ __align__(16) double ism[];
     pdl_allow_next();
     const SuperInvTask task = tasks[blockIdx.x];
-    const SuperPanel sp = sps[task.sp];
-    pdl_wait();
-    // two 64 x 64 blocks: the products' operands, then S (in A's place) and T_ii (in Bm's)
-    double (*A)[kSld] = reinterpret_cast<double (*)[kSld]>( ism );
-    double (*Bm)[kSld] = A + kPanel;
-    double (*S)[kSld] = A;
-    double (*Tii)[kSld] = Bm;
+    const SuperPanel & sp = sps[task.sp];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int i = task.i, j = task.j;
+    const int ldt = sp.ldt;
+    double * Tb = tbuf + sp.t;
+    auto block = [&]( int r, int c ) { return Tb + (std::int64_t)(kPanel * r) * ldt + kPanel * c; };
+    auto panel_inverse = [&]( int b ) { return tinv + (std::int64_t)sp.panel[b] * (kPanel * kPanel); };
     const int nbi = super_block_rows( sp, i );
-    double * out = tbuf + sp.t + (std::int64_t)(kPanel * i) * sp.ldt + kPanel * j;
-    auto load_tinv = [&]( double (*D)[kSld], int b, int nbb )
-    {
-        const double * src = tinv + (std::int64_t)sp.panel[b] * (kPanel * kPanel);
-#pragma unroll 4
-        for( int idx = tid; idx < kPanel * kPanel; idx += 256 )
-        {
-            const int r = idx >> 6, c = idx & 63;
-            const bool valid = r < nbb && c < nbb;
-            cp_async_8( &D[r][c], valid ? src + idx : src, valid );
-        }
-        cp_async_wait_all();
-    };
+    pdl_wait();
     if( i == j )
     {
-        load_tinv( Tii, i, nbi );
-        __syncthreads();
-        for( int idx = tid; idx < kPanel * kPanel; idx += 256 ) { out[(idx >> 6) * sp.ldt + (idx & 63)] = Tii[idx >> 6][idx & 63]; }
+        const double * src = panel_inverse( i );
+        double * out = block( i, i );
+        for( int idx = 2 * tid; idx < kPanel * kPanel; idx += 512 )
+        {
+            const int r = idx >> 6, c = idx & 63;
+            double2 v = make_double2( 0.0, 0.0 );
+            if( r < nbi && c < nbi )
+            {
+                v.x = src[idx];
+                if( c + 1 < nbi ) { v.y = src[idx + 1]; }
+            }
+            *reinterpret_cast<double2 *>( out + (std::int64_t)r * ldt + c ) = v;
+        }
         return;
     }
+    const int k0 = part == 0 ? task.mid : i, k1 = part == 0 ? j + 1 : task.mid;      // blocks of the sum
+    const int steps = (k1 - k0) * (kPanel / kInvK);
+    constexpr int kV = 16 / static_cast<int>( sizeof(T) );
+    [[maybe_unused]] float4 uf[2];
+    // stage st <- step q: columns [c0, c0 + 32) of the left block (i, k), rows [c0, c0 + 32) of the right one
+    auto load = [&]( int q )
+    {
+        const int k = k0 + q / (kPanel / kInvK), c0 = (q % (kPanel / kInvK)) * kInvK;
+        double * As = ism + (q & 1) * kInvStage;
+        double * Bs = As + kPanel * kInvLda;
+        const int nbk = super_block_rows( sp, k );
+        if( part == 0 )
+        {
+            const T * U = arena + sp.u0 + (std::int64_t)(sp.r0 + kPanel * i) * sp.ld0 + sp.r0 + kPanel * k + c0;
+#pragma unroll
+            for( int u = 0; u < kPanel * kInvK / kV / 256; ++u )
+            {
+                const int idx = kV * (tid + 256 * u), r = idx / kInvK, c = idx % kInvK;
+                const int left = r < nbi ? nbk - c0 - c : 0;                          // valid columns from c on
+                if constexpr ( sizeof(T) == 8 ) { cp_async_16( As + r * kInvLda + c, left > 0 ? U + (std::int64_t)r * sp.ld0 + c : U, left > 1 ? 16 : left > 0 ? 8 : 0 ); }
+                else
+                {
+                    uf[u] = left > 0 ? *reinterpret_cast<const float4 *>( U + (std::int64_t)r * sp.ld0 + c ) : make_float4( 0.f, 0.f, 0.f, 0.f );
+                    if( left < 4 ) { uf[u].w = 0.f; if( left < 3 ) { uf[u].z = 0.f; } if( left < 2 ) { uf[u].y = 0.f; } }
+                }
+            }
+        }
+        else
+        {
+            const bool diag = k == i;
+            const double * A = diag ? panel_inverse( i ) + c0 : block( i, k ) + c0;
+            const int lda = diag ? kPanel : ldt;
+#pragma unroll
+            for( int u = 0; u < kPanel * kInvK / 512; ++u )
+            {
+                const int idx = 2 * (tid + 256 * u), r = idx / kInvK, c = idx % kInvK;
+                const int left = diag ? (r < nbi ? nbi - c0 - c : 0) : 2;
+                cp_async_16( As + r * kInvLda + c, left > 0 ? A + (std::int64_t)r * lda + c : A, left > 1 ? 16 : left > 0 ? 8 : 0 );
+            }
+        }
+        {
+            const bool diag = part == 0 && k == j;
+            const double * B = (diag ? panel_inverse( j ) : part == 0 ? block( k, j ) : block( j, k )) + (std::int64_t)c0 * (diag ? kPanel : ldt);
+            const int ldb = diag ? kPanel : ldt;
+#pragma unroll
+            for( int u = 0; u < kPanel * kInvK / 512; ++u )
+            {
+                const int idx = 2 * (tid + 256 * u), r = idx / kPanel, c = idx % kPanel;
+                const int left = diag ? (c0 + r < nbk ? nbk - c : 0) : 2;
+                cp_async_16( Bs + r * kPld + c, left > 0 ? B + (std::int64_t)r * ldb + c : B, left > 1 ? 16 : left > 0 ? 8 : 0 );
+            }
+        }
+        cp_async_commit();
+    };
+    // FP32 storage: the left block's values, loaded a step ahead, widened into their stage
+    auto widen = [&]( int q )
+    {
+        if constexpr ( sizeof(T) == 4 )
+        {
+            if( part != 0 ) { return; }
+            double * As = ism + (q & 1) * kInvStage;
+#pragma unroll
+            for( int u = 0; u < 2; ++u )
+            {
+                const int idx = 4 * (tid + 256 * u), r = idx / kInvK, c = idx % kInvK;
+                *reinterpret_cast<double2 *>( As + r * kInvLda + c ) = make_double2( uf[u].x, uf[u].y );
+                *reinterpret_cast<double2 *>( As + r * kInvLda + c + 2 ) = make_double2( uf[u].z, uf[u].w );
+            }
+        }
+    };
     double acc[8][2];
 #pragma unroll
     for( int ct = 0; ct < 8; ++ct ) { acc[ct][0] = 0.0; acc[ct][1] = 0.0; }
-    const T * U0 = arena + sp.u0;
-    for( int k = i + 1; k <= j; ++k )
+    load( 0 );
+    widen( 0 );
+    for( int q = 0; q < steps; ++q )
     {
-        const int nbk = super_block_rows( sp, k );
-        const double * tk = tbuf + sp.t + (std::int64_t)(kPanel * k) * sp.ldt + kPanel * j;
-        auto src = [&]( int idx, double & fill ) -> const T *
+        cp_async_wait<0>();
+        __syncthreads();                                 // stage q complete; the other stage is free
+        if( q + 1 < steps ) { load( q + 1 ); }
+        const double * As = ism + (q & 1) * kInvStage + (8 * warp + (lane >> 2)) * kInvLda + (lane & 3);
+        const double * Bs = ism + (q & 1) * kInvStage + kPanel * kInvLda + (lane & 3) * kPld + (lane >> 2);
+#pragma unroll
+        for( int kk = 0; kk < kInvK; kk += 4 )
         {
-            fill = 0.0;
-            const int r = idx >> 6, c = idx & 63;
-            return (r < nbi && c < nbk) ? U0 + (std::int64_t)(sp.r0 + kPanel * i + r) * sp.ld0 + sp.r0 + kPanel * k + c : nullptr;
-        };
-        auto dst = [&]( int idx ) { return &A[idx >> 6][idx & 63]; };
-        stage_block<T, kPanel * kPanel / 256, 256>( U0, src, dst );
-        // T_kj is zero outside its valid rows and columns
-#pragma unroll 4
-        for( int idx = tid; idx < kPanel * kPanel; idx += 256 ) { cp_async_8( &Bm[idx >> 6][idx & 63], tk + (idx >> 6) * sp.ldt + (idx & 63), true ); }
-        cp_async_wait_all();
-        stage_finish<T, kPanel * kPanel / 256, 256>( src, dst );
-        __syncthreads();
-        block_product_64( acc, [&]( int r, int c ) { return A[r][c]; }, [&]( int r, int c ) { return Bm[r][c]; } );
-        __syncthreads();
+            const double a = As[kk];
+#pragma unroll
+            for( int ct = 0; ct < 8; ++ct ) { dmma_8x8x4( acc[ct], a, Bs[kk * kPld + 8 * ct] ); }
+        }
+        if( q + 1 < steps ) { widen( q + 1 ); }
     }
+    double * out = part == 0 ? block( j, i ) : block( i, j );
+    const double sign = part == 0 ? 1.0 : -1.0;
 #pragma unroll
     for( int ct = 0; ct < 8; ++ct )
     {
-        S[8 * warp + (lane >> 2)][8 * ct + 2 * (lane & 3)] = acc[ct][0];
-        S[8 * warp + (lane >> 2)][8 * ct + 2 * (lane & 3) + 1] = acc[ct][1];
-        acc[ct][0] = 0.0; acc[ct][1] = 0.0;
-    }
-    load_tinv( Tii, i, nbi );
-    __syncthreads();
-    block_product_64( acc, [&]( int r, int c ) { return Tii[r][c]; }, [&]( int r, int c ) { return S[r][c]; } );
-#pragma unroll
-    for( int ct = 0; ct < 8; ++ct )
-    {
-        const int r = 8 * warp + (lane >> 2), c = 8 * ct + 2 * (lane & 3);
-        out[r * sp.ldt + c] = -acc[ct][0];
-        out[r * sp.ldt + c + 1] = -acc[ct][1];
+        *reinterpret_cast<double2 *>( out + (std::int64_t)(8 * warp + (lane >> 2)) * ldt + 8 * ct + 2 * (lane & 3) )
+            = make_double2( sign * acc[ct][0], sign * acc[ct][1] );
     }
 }
 
@@ -2944,10 +2989,10 @@ void launch_solve_step( const SolveRestTask * tasks, int count, bool upper, cons
 }
 
 template<typename T>
-void launch_super_inv( const SuperInvTask * tasks, int count, const SuperPanel * sps, const T * arena, const double * tinv,
+void launch_super_inv( const SuperInvTask * tasks, int count, int part, const SuperPanel * sps, const T * arena, const double * tinv,
                        double * tbuf, cudaStream_t st )
 {
-    if( count > 0 ) { launch_pdl( super_inv_kernel<T>, count, 256, kSuperInvSmem, st, tasks, sps, arena, tinv, tbuf ); }
+    if( count > 0 ) { launch_pdl( super_inv_kernel<T>, count, 256, kSuperInvSmem, st, tasks, part, sps, arena, tinv, tbuf ); }
 }
 
 static size_t super_solve_smem( int k )
@@ -3015,7 +3060,7 @@ void launch_gather_diag( const std::int64_t * offsets, const T * arena, double *
     template void launch_solve_step<T>( const SolveRestTask *, int, bool, const T *, const double *,                \
                                         const std::int32_t *, double *, double *, int, int, cudaStream_t );         \
     template void launch_gather_diag<T>( const std::int64_t *, const T *, double *, int, cudaStream_t );          \
-    template void launch_super_inv<T>( const SuperInvTask *, int, const SuperPanel *, const T *, const double *,      \
+    template void launch_super_inv<T>( const SuperInvTask *, int, int, const SuperPanel *, const T *, const double *,      \
                                        double *, cudaStream_t );                                                    \
     template void launch_super_rest<T>( const SuperSolveTask *, int, const SuperPanel *, const T *,                 \
                                         const std::int32_t *, bool, double *, double *, const double *, int, int,   \

@@ -133,12 +133,12 @@ void launch_solve_dag( const SolveDagArgs & args, int grid, const T * arena, dou
 // Resident CTAs per SM of the persistent solve kernel for k right-hand sides (0 on error).
 int solve_dag_blocks_per_sm( int k );
 
-// Super-panel solve (plan.hpp, SuperPanel): the inverses' round launches
+// Super-panel solve (plan.hpp, SuperPanel): the inverses' product launches (part 0: W and the copies, 1: T)
 // (after the factorization; tbuf: Plan::super_inv_size doubles), and the diag
 // and rest steps of the sweeps (zbuf: n x ld doubles, zero before the back
 // sweep; in / out as launch_solve_step's).
 template<typename T>
-void launch_super_inv( const SuperInvTask * tasks, int count, const SuperPanel * sps, const T * arena, const double * tinv,
+void launch_super_inv( const SuperInvTask * tasks, int count, int part, const SuperPanel * sps, const T * arena, const double * tinv,
                        double * tbuf, cudaStream_t st );
 void launch_super_diag( const SuperSolveTask * tasks, int count, const SuperPanel * sps, const double * tbuf, bool upper,
                         const double * in, const double * zbuf, double * out, int ld, int k, cudaStream_t st );

@@ -1043,17 +1043,34 @@ void Plan::build_super( const std::vector<std::vector<I32>> & front_panels, Rang
         }
     }
     if( spanels.empty() ) { return; }
-    // the inverses: round d forms the blocks at distance d from the diagonal
-    for( I32 d = 0; d < kSuperPanels; ++d )
+    // the inverses: the copies of the panels' with the first products, then per doubling step two
+    // launches over the same blocks (Launch::part 0: W, 1: T)
+    for( I32 half = 1; half < kSuperPanels; half *= 2 )
     {
         const I64 first = static_cast<I64>( sinv.size() );
         for( I32 p = 0; p < static_cast<I32>( spanels.size() ); ++p )
         {
             const I32 nblk = static_cast<I32>( ceil_div( spanels[static_cast<size_t>(p)].rows, kPanel ) );
-            for( I32 i = 0; i + d < nblk; ++i ) { sinv.push_back( { p, i, i + d, 0 } ); }
+            for( I32 mid = half; mid < nblk; mid += 2 * half )
+            {
+                for( I32 i = mid - half; i < mid; ++i )
+                {
+                    for( I32 j = mid; j < std::min( mid + half, nblk ); ++j ) { sinv.push_back( { p, i, j, mid } ); }
+                }
+            }
         }
         const I32 count = static_cast<I32>( static_cast<I64>( sinv.size() ) - first );
-        if( count > 0 ) { sinv_launches.push_back( { LaunchKind::SuperInv, count, first, levels, d } ); }
+        I32 copies = 0;
+        if( half == 1 )
+        {
+            for( I32 p = 0; p < static_cast<I32>( spanels.size() ); ++p )
+            {
+                const I32 nblk = static_cast<I32>( ceil_div( spanels[static_cast<size_t>(p)].rows, kPanel ) );
+                for( I32 i = 0; i < nblk; ++i, ++copies ) { sinv.push_back( { p, i, i, 0 } ); }
+            }
+        }
+        if( count + copies > 0 ) { sinv_launches.push_back( { LaunchKind::SuperInv, count + copies, first, levels, half, 0 } ); }
+        if( count > 0 ) { sinv_launches.push_back( { LaunchKind::SuperInv, count, first, levels, half, 1 } ); }
     }
     // srest ranges: the large fronts' tasks last
     // (a task's front is large exactly when its n0 is: the criterion is the front's pivot-row count)

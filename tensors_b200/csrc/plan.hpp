@@ -282,11 +282,16 @@ struct SuperPanel
     std::int32_t ldt;              // the inverse's edge: rows rounded up to 64
 };
 
-// Block (i, j = i + d) of a super-panel's inverse, formed in round d:
-// d = 0 copies panel i's inverse; d > 0: T_ij = -T_ii sum_{k=i+1..j} U_ik T_kj.
+// Block (i, j) of a super-panel's inverse T, formed by doubling: with the
+// inverses of two adjacent diagonal blocks of 2^s panels known, the block
+// between them is -T_1 U_12 T_2, for s = 0, 1, 2 two launches of 64 x 64 block
+// products each: W_ij = sum_{k=mid..j} U_ik T_kj (kept at block (j, i), which the
+// solves never read), then T_ij = -sum_{k=i..mid-1} T_ik W_kj.  mid: the first
+// panel of the second diagonal block; i == j: panel i's inverse is copied (in
+// the first launch).
 struct SuperInvTask
 {
-    std::int32_t sp, i, j, pad;
+    std::int32_t sp, i, j, mid;
 };
 
 // A super-panel solve task.  Diag: the pair (blk, c0) of 64-row blocks, one

@@ -593,18 +593,47 @@ std::string check_plan( const Symbolic & sym, const Plan & pl )
                 else if( sp.panel[b] != -1 ) { return "super-panel panel beyond its rows" + at; }
             }
         }
-        for( size_t t = 0; t < pl.sinv.size(); ++t )
-        {
-            const SuperInvTask & v = pl.sinv[t];
-            if( v.sp < 0 || v.sp >= nsp || v.i < 0 || v.j < v.i || v.j >= nblk[static_cast<size_t>( v.sp )] ) { return "super-panel inverse task out of range"; }
-        }
+        // the inverses: tasks inside their super-panels; in launch order every block's operands are
+        // complete (T_kj of the second diagonal block, T_ik of the first, W of the same step) and every
+        // upper block is formed once
+        std::vector<std::vector<char>> t_done( static_cast<size_t>( nsp ), std::vector<char>( kSuperPanels * kSuperPanels, 0 ) ), w_done = t_done;
         for( const Launch & L : pl.sinv_launches )
         {
             if( L.kind != LaunchKind::SuperInv || L.count <= 0 || L.first < 0 || L.first + L.count > static_cast<I64>( pl.sinv.size() ) )
             {
                 return "super-panel inverse launch out of bounds";
             }
-            for( I64 t = L.first; t < L.first + L.count; ++t ) { if( pl.sinv[static_cast<size_t>( t )].j - pl.sinv[static_cast<size_t>( t )].i != L.step ) { return "super-panel inverse round mismatch"; } }
+            std::vector<std::pair<size_t, size_t>> formed;
+            for( I64 t = L.first; t < L.first + L.count; ++t )
+            {
+                const SuperInvTask & v = pl.sinv[static_cast<size_t>( t )];
+                if( v.sp < 0 || v.sp >= nsp || v.i < 0 || v.j < v.i || v.j >= nblk[static_cast<size_t>( v.sp )] ) { return "super-panel inverse task out of range"; }
+                const size_t p = static_cast<size_t>( v.sp );
+                auto at = [&]( I32 i, I32 j ) { return static_cast<size_t>( i * kSuperPanels + j ); };
+                if( v.i != v.j && (v.mid <= v.i || v.mid > v.j) ) { return "super-panel inverse task's blocks"; }
+                if( v.i == v.j ? L.part != 0 : false ) { return "super-panel inverse copy in a product launch"; }
+                if( v.i == v.j ) { if( t_done[p][at( v.i, v.i )] ) { return "super-panel inverse block formed twice"; } formed.push_back( { p, at( v.i, v.j ) } ); continue; }
+                // (diagonal blocks are read from the panels' inverses)
+                if( L.part == 0 )
+                {
+                    for( I32 k = v.mid; k < v.j; ++k ) { if( !t_done[p][at( k, v.j )] ) { return "super-panel inverse product before its operand"; } }
+                    w_done[p][at( v.i, v.j )] = 1;
+                }
+                else
+                {
+                    for( I32 k = v.i; k < v.mid; ++k ) { if( !w_done[p][at( k, v.j )] || (k > v.i && !t_done[p][at( v.i, k )]) ) { return "super-panel inverse product before its operand"; } }
+                    if( t_done[p][at( v.i, v.j )] ) { return "super-panel inverse block formed twice"; }
+                    formed.push_back( { p, at( v.i, v.j ) } );
+                }
+            }
+            for( const auto & f : formed ) { t_done[f.first][f.second] = 1; }
+        }
+        for( I64 p = 0; p < nsp; ++p )
+        {
+            for( I32 i = 0; i < nblk[static_cast<size_t>( p )]; ++i )
+            {
+                for( I32 j = i; j < nblk[static_cast<size_t>( p )]; ++j ) { if( !t_done[static_cast<size_t>( p )][static_cast<size_t>( i * kSuperPanels + j )] ) { return "super-panel inverse incomplete"; } }
+            }
         }
         // each sweep: every other front's tasks once, every super-panel's diag blocks and rest rows once
         for( const std::vector<Launch> * list : { &pl.lower_launches_sp, &pl.upper_launches_sp } )
