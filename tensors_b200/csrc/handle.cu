@@ -183,6 +183,7 @@ struct tb_chol
     DeviceArray<unsigned long long> solve_trace_buf; // with `trace`: forward then back sweep of the first RHS chunk
     int solve_schedule = TB_SCHEDULE_LEVELS;
     int dag_grid = 0;                            // CTAs of the persistent factorization launch
+    bool dag_ready = false;                      // the task graph is ordered and on the device
     bool use_dag = false;                        // persistent task-graph launch (else one launch per step)
     int schedule = TB_SCHEDULE_LEVELS;
     int precision = TB_PRECISION_FP64;
@@ -373,14 +374,13 @@ int ensure_device( tb_chol * h )
     }
     if( h->device_ready ) { return TB_OK; }
     {
-        // the persistent launch's CTA count, and the task order for it
+        // the persistent launch's CTA count (the task order for it: ensure_task_graph)
         int sms = 0;
         TB_CUDA( cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, h->device ) );
         const int per_sm = tb::factor_dag_blocks_per_sm();
         if( per_sm <= 0 ) { return fail( TB_ERR_CUDA, "persistent factorization kernel cannot be resident" ); }
         h->dag_grid = static_cast<int>( std::min<std::int64_t>( static_cast<std::int64_t>( per_sm ) * sms,
                                                                 static_cast<std::int64_t>( h->plan.dag.size() ) ) );
-        tb::schedule_task_graph( h->plan, h->dag_grid );
     }
     {
         const std::string msg = tb::check_plan( h->sym, h->plan );
@@ -432,8 +432,6 @@ int ensure_device( tb_chol * h )
         }
     }
     TB_TRY( h->tinv.reserve( static_cast<std::int64_t>( pl.sdiag.size() ) * tb::kPanel * tb::kPanel ) );
-    TB_TRY( h->dag.upload( pl.dag, st_ ) );
-    TB_TRY( h->dag_state.reserve( static_cast<std::int64_t>( pl.dag_counters ) + 2 ) );
     TB_TRY( h->solve_fwd_order.upload( pl.solve_fwd_order, st_ ) );
     TB_TRY( h->solve_bwd_order.upload( pl.solve_bwd_order, st_ ) );
     TB_TRY( h->solve_targets.upload( pl.solve_targets, st_ ) );
@@ -447,7 +445,24 @@ int ensure_device( tb_chol * h )
     TB_CUDA( cudaStreamSynchronize( st_ ) );
     if( h->factor_graph ) { cudaGraphExecDestroy( h->factor_graph ); h->factor_graph = nullptr; }
     h->drop_solve_graphs();
+    h->dag_ready = false;
     h->device_ready = true;
+    return TB_OK;
+}
+
+// Orders the factorization's task graph for the persistent launch, checks the order and uploads
+// it: only for the schedules that run it (the level schedule's first pass spent 21 of its 120 ms
+// here for the 64^3 Laplacian).
+int ensure_task_graph( tb_chol * h )
+{
+    if( h->dag_ready ) { return TB_OK; }
+    tb::schedule_task_graph( h->plan, h->dag_grid );
+    const std::string msg = tb::check_task_graph( h->plan );
+    if( !msg.empty() ) { return fail( TB_ERR_INVALID_ARGUMENT, "plan check: " + msg ); }
+    TB_TRY( h->dag.upload( h->plan.dag, h->stream ) );
+    TB_TRY( h->dag_state.reserve( static_cast<std::int64_t>( h->plan.dag_counters ) + 2 ) );
+    TB_CUDA( cudaStreamSynchronize( h->stream ) );
+    h->dag_ready = true;
     return TB_OK;
 }
 
@@ -668,6 +683,7 @@ int run_factor( tb_chol * h, double reg )
 {
     tb::TraceRange range( "Sparse::CholeskyDecomposition::NumericFactorization_Multifrontal" );
     cudaStream_t st = h->stream;
+    if( h->use_dag && !h->profiling ) { TB_TRY( ensure_task_graph( h ) ); }
     TB_TRY( h->pin_small.reserve( 64 ) );
     double * pr = h->pin_small.as<double>();
     pr[0] = reg;
@@ -2173,6 +2189,7 @@ int tb_chol_plan_stats( tb_chol * h, std::int64_t * out, std::int32_t cap )
     TB_TRY( check_handle( h ) );
     if( out == nullptr || cap < 0 ) { return fail( TB_ERR_INVALID_ARGUMENT, "null output" ); }
     TB_TRY( ensure_symbolic( h ) );
+    if( h->device_ready ) { TB_TRY( ensure_task_graph( h ) ); }     // (the ordered graph's duration)
     const tb::Plan & pl = h->plan;
     const std::int64_t v[] = {
         pl.arena_size(), pl.v_size, pl.levels, static_cast<std::int64_t>( level_launches( h ).size() ) + 2,
