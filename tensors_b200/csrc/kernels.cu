@@ -2433,7 +2433,7 @@ __global__ void init_status_kernel( int * status )
 
 // Launch with programmatic stream serialization (see pdl_allow_next).
 template<typename... KArgs, typename... Args>
-void launch_pdl( void (*kernel)( KArgs... ), unsigned grid, unsigned block, size_t smem, cudaStream_t st, Args... args )
+void launch( bool programmatic, void (*kernel)( KArgs... ), unsigned grid, unsigned block, size_t smem, cudaStream_t st, Args... args )
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3( grid );
@@ -2444,8 +2444,14 @@ void launch_pdl( void (*kernel)( KArgs... ), unsigned grid, unsigned block, size
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = programmatic ? 1 : 0;
     cudaLaunchKernelEx( &cfg, kernel, static_cast<KArgs>( args )... );
+}
+
+template<typename... KArgs, typename... Args>
+void launch_pdl( void (*kernel)( KArgs... ), unsigned grid, unsigned block, size_t smem, cudaStream_t st, Args... args )
+{
+    launch( true, kernel, grid, block, smem, st, args... );
 }
 
 int grid_for( std::int64_t work, int threads )
@@ -2885,13 +2891,13 @@ void launch_trsm( const PanelTask * tasks, int count, T * arena, const double * 
 }
 
 template<typename T>
-void launch_gemm( const GemmTask * tasks, int count, T * arena, int * status, cudaStream_t st )
+void launch_gemm( const GemmTask * tasks, int count, T * arena, int * status, cudaStream_t st, bool programmatic )
 {
     if( count <= 0 ) { return; }
     if constexpr ( sizeof(T) == 8 )
     {
         (void)status;
-        launch_pdl( gemm_tn_kernel, count, kGemmThreads, kGemmSmemBytes, st, tasks, arena );
+        launch( programmatic, gemm_tn_kernel, count, kGemmThreads, kGemmSmemBytes, st, tasks, arena );
     }
     else
     {
@@ -2899,7 +2905,7 @@ void launch_gemm( const GemmTask * tasks, int count, T * arena, int * status, cu
         cudaGetDevice( &dev );
         cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
         const int grid = std::min( count, 3 * std::max( sms, 1 ) );
-        launch_pdl( gemm_tc_kernel, grid, kGemmThreads, kGemmSmemBytesF, st, tasks, count, arena, status );
+        launch( programmatic, gemm_tc_kernel, grid, kGemmThreads, kGemmSmemBytesF, st, tasks, count, arena, status );
     }
 }
 
@@ -3054,7 +3060,7 @@ void launch_gather_diag( const std::int64_t * offsets, const T * arena, double *
     template void launch_extend_pull<T>( const ExtendPullTask *, int, const ExtendTask *, const std::int32_t *, T *, cudaStream_t ); \
     template void launch_potrf<T>( const PanelTask *, int, T *, int *, const double *, double *, cudaStream_t, bool );     \
     template void launch_trsm<T>( const PanelTask *, int, T *, const double *, cudaStream_t, float *, bool );              \
-    template void launch_gemm<T>( const GemmTask *, int, T *, int *, cudaStream_t );                                 \
+    template void launch_gemm<T>( const GemmTask *, int, T *, int *, cudaStream_t, bool );                                 \
     template void launch_solve_dag<T>( const SolveDagArgs &, int, const T *, double *, double *, int, int, cudaStream_t );                                        \
     template void launch_factor_dag<T>( const DagArgs &, int, cudaStream_t );                                        \
     template void launch_solve_step<T>( const SolveRestTask *, int, bool, const T *, const double *,                \

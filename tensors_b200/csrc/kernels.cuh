@@ -50,7 +50,8 @@ template<typename T> void launch_trsm( const PanelTask * tasks, int count, T * a
                                        float * img, bool after_potrf );
 // status[0] gets kStatusTcTimeout (2) when a tensor-core completion wait of
 // the FP32 path ran out (its tile is then not updated).
-template<typename T> void launch_gemm( const GemmTask * tasks, int count, T * arena, int * status, cudaStream_t st );
+// programmatic: may start while the kernel before it in the stream drains (it waits for its end by itself)
+template<typename T> void launch_gemm( const GemmTask * tasks, int count, T * arena, int * status, cudaStream_t st, bool programmatic );
 
 // The tensor map (CUtensorMap, 128 bytes) of the operand image, held by the
 // host and passed to the tile kernel by value.
