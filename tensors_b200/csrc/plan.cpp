@@ -1018,7 +1018,13 @@ void Plan::build_super( const std::vector<std::vector<I32>> & front_panels, Rang
     std::vector<std::vector<I32>> front_sp( static_cast<size_t>(F) );
     if( use_super )
     {
-        for( I32 f = 0; f < F; ++f ) { big[static_cast<size_t>(f)] = front_n0[f] >= kSuperMinRows ? 1 : 0; }
+        for( const std::vector<I32> & fronts_of_level : by_level )
+        {
+            I32 most = 0;
+            for( I32 f : fronts_of_level ) { most = std::max( most, front_n0[f] ); }
+            if( most < kSuperMinRows ) { continue; }
+            for( I32 f : fronts_of_level ) { big[static_cast<size_t>(f)] = front_n0[f] > kPanel ? 1 : 0; }
+        }
     }
     for( I32 f = 0; f < F; ++f )
     {
@@ -1073,8 +1079,9 @@ void Plan::build_super( const std::vector<std::vector<I32>> & front_panels, Rang
         if( count > 0 ) { sinv_launches.push_back( { LaunchKind::SuperInv, count, first, levels, half, 1 } ); }
     }
     // srest ranges: the large fronts' tasks last
-    // (a task's front is large exactly when its n0 is: the criterion is the front's pivot-row count)
-    auto is_big_task = [&]( const SolveRestTask & t ) { return use_super && t.n0 >= kSuperMinRows; };
+    std::vector<char> big_panel( sdiag.size(), 0 );
+    for( const SuperPanel & sp : spanels ) { for( I32 q : sp.panel ) { if( q >= 0 ) { big_panel[static_cast<size_t>(q)] = 1; } } }
+    auto is_big_task = [&]( const SolveRestTask & t ) { return big_panel[static_cast<size_t>( t.panel )] != 0; };
     std::vector<std::vector<I32>> regular( static_cast<size_t>(levels) );
     for( I32 h = 0; h < levels; ++h )
     {

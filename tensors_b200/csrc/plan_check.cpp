@@ -636,6 +636,7 @@ std::string check_panels( const Symbolic & sym, const Plan & pl )
         // panel inverses they start from belong to their rows
         const I64 nsp = static_cast<I64>( pl.spanels.size() );
         std::vector<I32> nblk( static_cast<size_t>( nsp ) ), nrest( static_cast<size_t>( nsp ) );
+        std::vector<char> big_panel( pl.sdiag.size(), 0 );                    // panels solved by super-panels, each in one
         for( I64 p = 0; p < nsp; ++p )
         {
             const SuperPanel & sp = pl.spanels[static_cast<size_t>( p )];
@@ -658,6 +659,7 @@ std::string check_panels( const Symbolic & sym, const Plan & pl )
                     if( q < 0 || q >= static_cast<I32>( pl.sdiag.size() ) ) { return "super-panel panel out of range" + at; }
                     const SolveDiagTask & d = pl.sdiag[static_cast<size_t>( q )];
                     if( d.u0 != sp.u0 || d.r0 != sp.r0 + b * kPanel || d.n0 != sp.n0 ) { return "super-panel panel mismatch" + at; }
+                    if( big_panel[static_cast<size_t>( q )]++ ) { return "super-panel panel in two super-panels" + at; }
                 }
                 else if( sp.panel[b] != -1 ) { return "super-panel panel beyond its rows" + at; }
             }
@@ -715,7 +717,7 @@ std::string check_panels( const Symbolic & sym, const Plan & pl )
                 if( L.kind == LaunchKind::Solve )
                 {
                     if( L.count <= 0 || L.first < 0 || L.first + L.count > static_cast<I64>( pl.srest.size() ) ) { return "super solve list: step launch out of bounds"; }
-                    for( I64 t = L.first; t < L.first + L.count; ++t ) { if( pl.srest[static_cast<size_t>( t )].n0 >= kSuperMinRows ) { return "super solve list: a large front's panel step"; } }
+                    for( I64 t = L.first; t < L.first + L.count; ++t ) { if( big_panel[static_cast<size_t>( pl.srest[static_cast<size_t>( t )].panel )] ) { return "super solve list: a large front's panel step"; } }
                     regular += L.count;
                     continue;
                 }
@@ -744,7 +746,7 @@ std::string check_panels( const Symbolic & sym, const Plan & pl )
                 }
             }
             I64 small = 0;
-            for( const SolveRestTask & t : pl.srest ) { small += t.n0 >= kSuperMinRows ? 0 : 1; }
+            for( const SolveRestTask & t : pl.srest ) { small += big_panel[static_cast<size_t>( t.panel )] ? 0 : 1; }
             if( regular != small ) { return "super solve list: the other fronts' steps are not covered once"; }
             for( I64 p = 0; p < nsp; ++p )
             {
