@@ -826,7 +826,11 @@ std::int64_t issue_sweeps( tb_chol * h, int which, double * W, double * Y, std::
         begin();
         if( L.kind == tb::LaunchKind::SuperDiag )
         {
-            tb::launch_super_diag( h->ssolve.ptr + L.first, L.count, h->spanels.ptr, h->tsuper.ptr, upper, in, Z + c0, out, k, kc, st );
+            const tb::SolveRestTask * steps = h->srest.ptr + L.tc_first;
+            if( mixed ) { tb::launch_super_diag( h->ssolve.ptr + L.first, L.count, steps, L.tc_count, h->spanels.ptr, h->tsuper.ptr,
+                                                 arena_as<float>( h ), h->tinv.ptr, h->sn_inner.ptr, upper, in, Z + c0, out, k, kc, st ); }
+            else        { tb::launch_super_diag( h->ssolve.ptr + L.first, L.count, steps, L.tc_count, h->spanels.ptr, h->tsuper.ptr,
+                                                 arena_as<double>( h ), h->tinv.ptr, h->sn_inner.ptr, upper, in, Z + c0, out, k, kc, st ); }
         }
         else if( L.kind == tb::LaunchKind::SuperRest )
         {
@@ -845,7 +849,7 @@ std::int64_t issue_sweeps( tb_chol * h, int which, double * W, double * Y, std::
             tb::launch_solve_step( h->srest.ptr + L.first, L.count, upper, arena_as<double>( h ), h->tinv.ptr,
                                    h->sn_inner.ptr, in, out, k, kc, st );
         }
-        end( L.level, L.step, L.count, upper ? 1 : 0 );
+        end( L.level, L.step, L.count + (L.kind == tb::LaunchKind::SuperDiag ? L.tc_count : 0), upper ? 1 : 0 );
         ++launches;
     };
     auto persistent = [&]( bool upper, double * in, double * out, std::int32_t kc, std::int32_t c0 )

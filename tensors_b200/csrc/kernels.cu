@@ -1727,6 +1727,35 @@ __device__ __forceinline__ void warp_rows_product( double (&acc)[NCT][2], int kb
     }
 }
 
+// Stages rows row(0..nr) (leading dimension ld, k columns) of a sweep vector x
+// into V (64 x KP, leading dimension KP + 4); cells outside nr x k are zero.
+// 16-byte copies where every row starts on a 16-byte boundary (x does).
+template<int KP, typename RowOf>
+__device__ __forceinline__ void stage_rows( double * V, const double * x, RowOf row, int nr, int ld, int k )
+{
+    constexpr int ldv = KP + 4;
+    if( ((ld | k) & 1) == 0 )
+    {
+#pragma unroll
+        for( int u = 0; u < kPanel * KP / 512; ++u )
+        {
+            const int idx = 2 * (threadIdx.x + 256 * u), r = idx / KP, c = idx % KP;
+            const bool ok = r < nr && c < k;
+            cp_async_16( V + r * ldv + c, ok ? x + row( r ) * ld + c : x, ok ? 16 : 0 );
+        }
+    }
+    else
+    {
+#pragma unroll 4
+        for( int idx = threadIdx.x; idx < kPanel * KP; idx += 256 )
+        {
+            const int r = idx / KP, c = idx % KP;
+            const bool ok = r < nr && c < k;
+            cp_async_8( V + r * ldv + c, ok ? x + row( r ) * ld + c : x, ok );
+        }
+    }
+}
+
 // One solve step.  Forward (U^T y = b): every task forms x_q = T_q^T y_q for
 // the panel's rows of `in`; the owner writes x_q to `out`, and a task with
 // rest rows subtracts P^T x_q from its (up to) 64 rest rows of `in` (rows of
@@ -1824,25 +1853,10 @@ __device__ __forceinline__ void solve_step_body( const SolveRestTask & t, int up
     if constexpr ( kPdl ) { pdl_wait(); }
     // y_q: the panel's rows of `in` (forward: every task; backward: the owner)
     const bool need_y = !upper || owner;
-#pragma unroll 4
-    for( int idx = tid; idx < (kPanel << lkp); idx += kSolveThreads )
-    {
-        const int i = idx >> lkp, c = idx & (kp - 1);
-        const bool valid = need_y && i < nb && c < k;
-        cp_async_8( &sY[i * ldv + c], valid ? in + (prow + i) * ld + c : in, valid );
-    }
+    stage_rows<KP>( sY, in, [&]( int i ) { return prow + i; }, need_y ? nb : 0, ld, k );
     __syncthreads();
-    if( upper )
-    {
-        // x_r: the rest rows of `out`, final
-#pragma unroll 4
-        for( int idx = tid; idx < (kPanel << lkp); idx += kSolveThreads )
-        {
-            const int i = idx >> lkp, c = idx & (kp - 1);
-            const bool valid = i < cw && c < k;
-            cp_async_8( &sX[i * ldv + c], valid ? out + trow[i] * ld + c : out, valid );
-        }
-    }
+    // x_r: the rest rows of `out`, final
+    if( upper ) { stage_rows<KP>( sX, out, [&]( int i ) { return trow[i]; }, cw, ld, k ); }
     cp_async_wait_all();
     __syncthreads();
 
@@ -2466,9 +2480,8 @@ int grid_for( std::int64_t work, int threads )
 // from the 64-row panel inverses, replaces eight sequential panel steps by
 // one product with T.  64 x 64 blocks throughout; warp w owns output rows
 // 8w..8w+7 as 8 x 8 DMMA tiles.
-constexpr int kSld = kPanel + 1;                        // padded smem row of a 64 x 64 block
-// Doubles of shared memory a 64 x kSld block of T takes (rounded up to 16 bytes).
-template<typename T> __host__ __device__ constexpr int super_block_doubles() { return ((kPanel * kSld * static_cast<int>( sizeof(T) ) + 15) / 16) * 2; }
+// Doubles of shared memory a padded 64 x 64 block of T takes (see super_rest_kernel).
+template<typename T> __host__ __device__ constexpr int super_block_doubles() { return sizeof(T) == 4 ? kPanel * (kPanel + 8) / 2 : kPanel * kPld; }
 
 __device__ __forceinline__ int super_block_rows( const SuperPanel & sp, int b ) { return min( kPanel, sp.rows - b * kPanel ); }
 
@@ -2619,22 +2632,6 @@ __global__ __launch_bounds__(256) void super_inv_kernel( const SuperInvTask * __
     }
 }
 
-// Stages x rows [row, row + nr) (leading dimension ld, k columns) of a sweep
-// vector into V (64 x KP, leading dimension KP + 4) with 8-byte asynchronous
-// copies; cells outside nr x k are zero.
-template<int KP>
-__device__ __forceinline__ void stage_rows( double * V, const double * x, std::int64_t row, int nr, int ld, int k )
-{
-    constexpr int ldv = KP + 4;
-#pragma unroll 4
-    for( int idx = threadIdx.x; idx < kPanel * KP; idx += 256 )
-    {
-        const int r = idx / KP, c = idx % KP;
-        const bool ok = r < nr && c < k;
-        cp_async_8( V + r * ldv + c, ok ? x + (row + r) * ld + c : x, ok );
-    }
-}
-
 // One block pair of a super-panel's diag step.  Forward (task (o, b), b <= o):
 // x_o += T_bo^T y_b; back (b >= o): x_o += T_ob (y_b + z_b).  y: `in`, z: the
 // rest steps' sums in `zbuf`, x: `out`, whose block rows are zero before the
@@ -2642,35 +2639,39 @@ __device__ __forceinline__ void stage_rows( double * V, const double * x, std::i
 // of two >= 8.  One 64 x 64 block of T and one 64 x k block of vectors per
 // CTA, all copies in flight together.
 template<int KP>
-__global__ __launch_bounds__(256) void super_diag_kernel( const SuperSolveTask * __restrict__ tasks, const SuperPanel * __restrict__ sps,
-                                                          const double * __restrict__ tbuf, int upper, const double * in,
-                                                          const double * zbuf, double * out, int ld, int k )
+__device__ __forceinline__ void super_diag_body( const SuperSolveTask & task, const SuperPanel * __restrict__ sps,
+                                                 const double * __restrict__ tbuf, int upper, const double * in,
+                                                 const double * zbuf, double * out, int ld, int k, double * dsm )
 {
-    extern __shared__ __align__(16) double dsm[];
-    pdl_allow_next();
-    const SuperSolveTask task = tasks[blockIdx.x];
-    const SuperPanel sp = sps[task.sp];
+    const SuperPanel & sp = sps[task.sp];
     constexpr int nct = KP / 8;
     constexpr int ldv = KP + 4;
-    double (*Tb)[kSld] = reinterpret_cast<double (*)[kSld]>( dsm );
-    double * V = dsm + kPanel * kSld;                  // [64][ldv]
+    double (*Tb)[kPld] = reinterpret_cast<double (*)[kPld]>( dsm );
+    double * V = dsm + kPanel * kPld;                  // [64][ldv]
     double * Z = V + kPanel * ldv;                     // [64][ldv], back sweep only
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int o = task.blk, b = task.c0;
     const int nbb = super_block_rows( sp, b );
     const std::int64_t brow = (std::int64_t)sp.row0 + sp.r0;
+    const int ldt = sp.ldt;
     // forward: block (b, o) of T, read transposed; back: block (o, b).  The
     // blocks are zero outside their valid rows and columns.
-    const double * tb = upper ? tbuf + sp.t + (std::int64_t)(kPanel * o) * sp.ldt + kPanel * b
-                              : tbuf + sp.t + (std::int64_t)(kPanel * b) * sp.ldt + kPanel * o;
-#pragma unroll 4
-    for( int idx = tid; idx < kPanel * kPanel; idx += 256 ) { cp_async_8( &Tb[idx >> 6][idx & 63], tb + (idx >> 6) * sp.ldt + (idx & 63), true ); }
+    const double * tb = upper ? tbuf + sp.t + (std::int64_t)(kPanel * o) * ldt + kPanel * b
+                              : tbuf + sp.t + (std::int64_t)(kPanel * b) * ldt + kPanel * o;
+#pragma unroll
+    for( int u = 0; u < kPanel * kPanel / 512; ++u )
+    {
+        const int idx = 2 * (tid + 256 * u);
+        cp_async_16( &Tb[idx >> 6][idx & 63], tb + (idx >> 6) * ldt + (idx & 63), 16 );
+    }
     pdl_wait();
-    stage_rows<KP>( V, in, brow + kPanel * b, nbb, ld, k );
-    if( upper ) { stage_rows<KP>( Z, zbuf, brow + kPanel * b, nbb, ld, k ); }
+    auto rows = [&]( int r ) { return brow + kPanel * b + r; };
+    stage_rows<KP>( V, in, rows, nbb, ld, k );
+    if( upper ) { stage_rows<KP>( Z, zbuf, rows, nbb, ld, k ); }
     cp_async_wait_all();
     if( upper )
     {
+        __syncthreads();
         for( int idx = tid; idx < kPanel * KP; idx += 256 ) { V[(idx / KP) * ldv + idx % KP] += Z[(idx / KP) * ldv + idx % KP]; }
     }
     __syncthreads();
@@ -2703,6 +2704,30 @@ __global__ __launch_bounds__(256) void super_diag_kernel( const SuperSolveTask *
     }
 }
 
+// A diag step and, in the level's first one, the level's panel steps beside it
+// (its one-panel fronts; the two touch different fronts' rows, ancestor rows by
+// reductions): one launch less on the level's chain.  With the 16-byte copies
+// and padded rows of this and the rest step: C2 with 16 right-hand sides 1.56
+// -> 1.22 ms, 56^3 with 64 2.93 -> 2.01 ms.
+template<typename T, int KP>
+__global__ __launch_bounds__(256) void super_diag_kernel( const SuperSolveTask * __restrict__ tasks, int ndiag,
+                                                          const SolveRestTask * __restrict__ steps, const SuperPanel * __restrict__ sps,
+                                                          const double * __restrict__ tbuf, const T * __restrict__ arena,
+                                                          const double * __restrict__ tinv, const std::int32_t * __restrict__ sn_inner,
+                                                          int upper, double * in, const double * zbuf, double * out, int ld, int k )
+{
+    extern __shared__ __align__(16) double dsm[];
+    pdl_allow_next();
+    if( static_cast<int>( blockIdx.x ) < ndiag )
+    {
+        super_diag_body<KP>( tasks[blockIdx.x], sps, tbuf, upper, in, zbuf, out, ld, k, dsm );
+    }
+    else
+    {
+        solve_step_body<T, KP, true>( steps[blockIdx.x - ndiag], upper, arena, tinv, sn_inner, in, out, ld, k, false, dsm );
+    }
+}
+
 // One (block, rest chunk) pair of a super-panel's rest step, rest columns
 // [c0, c1) of block b.  Forward: y_rest -= U_{b,rest}^T x_b (x_b: `out`, final
 // after the diag step; y: `in`, every row by reductions, as the eight blocks
@@ -2720,8 +2745,10 @@ __global__ __launch_bounds__(256) void super_rest_kernel( const SuperSolveTask *
     constexpr int nct = KP / 8;
     constexpr int ldv = KP + 4;
     __shared__ std::int64_t trow[kSolveRest];
-    // the factor block in the factor's type (FP32 storage: half the shared memory), widened as read
-    T (*P)[kSld] = reinterpret_cast<T (*)[kSld]>( rsm );
+    // the factor block in the factor's type (FP32 storage: half the shared memory), widened as read;
+    // leading dimensions without bank conflicts in the fragment reads (FP32: 68 by rows, 72 by columns)
+    T * Ps = reinterpret_cast<T *>( rsm );
+    const int ldp = sizeof(T) == 4 && !upper ? kPanel + 8 : kPld;
     double * V = rsm + super_block_doubles<T>();        // [64][ldv]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int r1 = sp.r0 + sp.rows;
@@ -2738,31 +2765,23 @@ __global__ __launch_bounds__(256) void super_rest_kernel( const SuperSolveTask *
     // P: rows of block b (U rows r0 + 64 b + rr), the chunk's rest columns
     const T * U0 = arena + sp.u0;
     const T * U1 = arena + sp.u1;
-#pragma unroll 4
-    for( int idx = tid; idx < kPanel * kPanel; idx += 256 )
+    // (a chunk lies in U0 or in U1 alone, both 16-byte aligned there)
+    constexpr int kV = 16 / static_cast<int>( sizeof(T) );
+    const T * src0 = task.c0 < m ? U0 + (std::int64_t)(sp.r0 + kPanel * b) * sp.ld0 + r1 + task.c0
+                                 : U1 + (std::int64_t)(sp.r0 + kPanel * b) * sp.ld1 + (task.c0 - m);
+    const int lds = task.c0 < m ? sp.ld0 : sp.ld1;
+#pragma unroll
+    for( int u = 0; u < kPanel * kPanel / kV / 256; ++u )
     {
-        const int rr = idx >> 6, jj = idx & 63;
-        const bool valid = rr < nbb && jj < cw;
-        const int col = task.c0 + jj;
-        const std::int64_t urow = sp.r0 + kPanel * b + rr;
-        const T * src = !valid ? U0 : col < m ? U0 + urow * sp.ld0 + r1 + col : U1 + urow * sp.ld1 + (col - m);
-        if constexpr ( sizeof(T) == 8 ) { cp_async_8( reinterpret_cast<double *>( &P[rr][jj] ), reinterpret_cast<const double *>( src ), valid ); }
-        else { cp_async_4( &P[rr][jj], src, valid ); }
+        const int idx = kV * (tid + 256 * u), rr = idx >> 6, jj = idx & 63;
+        const int left = rr < nbb ? min( cw - jj, kV ) : 0;
+        cp_async_16( Ps + rr * ldp + jj, left > 0 ? src0 + (std::int64_t)rr * lds + jj : src0, left > 0 ? left * static_cast<int>( sizeof(T) ) : 0 );
     }
     pdl_wait();
     __syncthreads();                                    // trow
-    if( upper )
-    {
-        // x_rest: the chunk's rows of `out`
-#pragma unroll 4
-        for( int idx = tid; idx < kPanel * KP; idx += 256 )
-        {
-            const int r = idx / KP, c = idx % KP;
-            const bool ok = r < cw && c < k;
-            cp_async_8( V + r * ldv + c, ok ? out + trow[r] * ld + c : out, ok );
-        }
-    }
-    else { stage_rows<KP>( V, out, brow + kPanel * b, nbb, ld, k ); }
+    // x_rest: the chunk's rows of `out`; x_b
+    if( upper ) { stage_rows<KP>( V, out, [&]( int r ) { return trow[r]; }, cw, ld, k ); }
+    else { stage_rows<KP>( V, out, [&]( int r ) { return brow + kPanel * b + r; }, nbb, ld, k ); }
     cp_async_wait_all();
     __syncthreads();
     double acc[nct][2];
@@ -2774,9 +2793,9 @@ __global__ __launch_bounds__(256) void super_rest_kernel( const SuperSolveTask *
         for( int ct = 0; ct < nct; ++ct )
         {
             // forward: acc(jj, c) = sum_rr P[rr][jj] x_b[rr][c]; back: acc(rr, c) = sum_jj P[rr][jj] x_rest[jj][c]
-            if( upper ) { dmma_8x8x8( acc[ct], [&]( int i, int kk ) { return static_cast<double>( P[8 * warp + i][8 * kb + kk] ); },
+            if( upper ) { dmma_8x8x8( acc[ct], [&]( int i, int kk ) { return static_cast<double>( Ps[(8 * warp + i) * ldp + 8 * kb + kk] ); },
                                                [&]( int kk, int j ) { return V[(8 * kb + kk) * ldv + 8 * ct + j]; } ); }
-            else        { dmma_8x8x8( acc[ct], [&]( int i, int kk ) { return static_cast<double>( P[8 * kb + kk][8 * warp + i] ); },
+            else        { dmma_8x8x8( acc[ct], [&]( int i, int kk ) { return static_cast<double>( Ps[(8 * kb + kk) * ldp + 8 * warp + i] ); },
                                                [&]( int kk, int j ) { return V[(8 * kb + kk) * ldv + 8 * ct + j]; } ); }
         }
     }
@@ -3001,9 +3020,10 @@ void launch_super_inv( const SuperInvTask * tasks, int count, int part, const Su
     if( count > 0 ) { launch_pdl( super_inv_kernel<T>, count, 256, kSuperInvSmem, st, tasks, part, sps, arena, tinv, tbuf ); }
 }
 
-static size_t super_solve_smem( int k )
+template<typename T>
+static size_t super_diag_smem( int k )
 {
-    return sizeof(double) * (kPanel * kSld + 2 * kPanel * ((1 << solve_lkp( k )) + 4));
+    return std::max( solve_smem_bytes<T>( k ), sizeof(double) * (kPanel * kPld + 2 * kPanel * ((1 << solve_lkp( k )) + 4)) );
 }
 
 template<typename T>
@@ -3012,18 +3032,20 @@ static size_t super_rest_smem( int k )
     return sizeof(double) * (super_block_doubles<T>() + kPanel * ((1 << solve_lkp( k )) + 4));
 }
 
-void launch_super_diag( const SuperSolveTask * tasks, int count, const SuperPanel * sps, const double * tbuf, bool upper,
-                        const double * in, const double * zbuf, double * out, int ld, int k, cudaStream_t st )
+template<typename T>
+void launch_super_diag( const SuperSolveTask * tasks, int count, const SolveRestTask * steps, int nsteps, const SuperPanel * sps,
+                        const double * tbuf, const T * arena, const double * tinv, const std::int32_t * sn_inner, bool upper,
+                        double * in, const double * zbuf, double * out, int ld, int k, cudaStream_t st )
 {
-    if( count <= 0 ) { return; }
-    const size_t sm = super_solve_smem( k );
-    const int u = upper ? 1 : 0;
+    if( count + nsteps <= 0 ) { return; }
+    const size_t sm = super_diag_smem<T>( k );
+    const int u = upper ? 1 : 0, n = count + nsteps;
     switch( solve_lkp( k ) )
     {
-        case 3:  launch_pdl( super_diag_kernel<8>, count, 256, sm, st, tasks, sps, tbuf, u, in, zbuf, out, ld, k ); break;
-        case 4:  launch_pdl( super_diag_kernel<16>, count, 256, sm, st, tasks, sps, tbuf, u, in, zbuf, out, ld, k ); break;
-        case 5:  launch_pdl( super_diag_kernel<32>, count, 256, sm, st, tasks, sps, tbuf, u, in, zbuf, out, ld, k ); break;
-        default: launch_pdl( super_diag_kernel<64>, count, 256, sm, st, tasks, sps, tbuf, u, in, zbuf, out, ld, k ); break;
+        case 3:  launch_pdl( super_diag_kernel<T, 8>, n, 256, sm, st, tasks, count, steps, sps, tbuf, arena, tinv, sn_inner, u, in, zbuf, out, ld, k ); break;
+        case 4:  launch_pdl( super_diag_kernel<T, 16>, n, 256, sm, st, tasks, count, steps, sps, tbuf, arena, tinv, sn_inner, u, in, zbuf, out, ld, k ); break;
+        case 5:  launch_pdl( super_diag_kernel<T, 32>, n, 256, sm, st, tasks, count, steps, sps, tbuf, arena, tinv, sn_inner, u, in, zbuf, out, ld, k ); break;
+        default: launch_pdl( super_diag_kernel<T, 64>, n, 256, sm, st, tasks, count, steps, sps, tbuf, arena, tinv, sn_inner, u, in, zbuf, out, ld, k ); break;
     }
 }
 
@@ -3068,6 +3090,8 @@ void launch_gather_diag( const std::int64_t * offsets, const T * arena, double *
     template void launch_gather_diag<T>( const std::int64_t *, const T *, double *, int, cudaStream_t );          \
     template void launch_super_inv<T>( const SuperInvTask *, int, int, const SuperPanel *, const T *, const double *,      \
                                        double *, cudaStream_t );                                                    \
+    template void launch_super_diag<T>( const SuperSolveTask *, int, const SolveRestTask *, int, const SuperPanel *, const double *, const T *,   \
+                                        const double *, const std::int32_t *, bool, double *, const double *, double *, int, int, cudaStream_t ); \
     template void launch_super_rest<T>( const SuperSolveTask *, int, const SuperPanel *, const T *,                 \
                                         const std::int32_t *, bool, double *, double *, const double *, int, int,   \
                                         cudaStream_t );
@@ -3140,10 +3164,14 @@ cudaError_t configure_kernels()
         { reinterpret_cast<const void *>( solve_dag_kernel<float, 64> ), solve_smem_bytes<float>( 64 ) },
         { reinterpret_cast<const void *>( super_inv_kernel<double> ), kSuperInvSmem },
         { reinterpret_cast<const void *>( super_inv_kernel<float> ), kSuperInvSmem },
-        { reinterpret_cast<const void *>( super_diag_kernel<8> ), super_solve_smem( 8 ) },
-        { reinterpret_cast<const void *>( super_diag_kernel<16> ), super_solve_smem( 16 ) },
-        { reinterpret_cast<const void *>( super_diag_kernel<32> ), super_solve_smem( 32 ) },
-        { reinterpret_cast<const void *>( super_diag_kernel<64> ), super_solve_smem( 64 ) },
+        { reinterpret_cast<const void *>( super_diag_kernel<double, 8> ), super_diag_smem<double>( 8 ) },
+        { reinterpret_cast<const void *>( super_diag_kernel<float, 8> ), super_diag_smem<float>( 8 ) },
+        { reinterpret_cast<const void *>( super_diag_kernel<double, 16> ), super_diag_smem<double>( 16 ) },
+        { reinterpret_cast<const void *>( super_diag_kernel<float, 16> ), super_diag_smem<float>( 16 ) },
+        { reinterpret_cast<const void *>( super_diag_kernel<double, 32> ), super_diag_smem<double>( 32 ) },
+        { reinterpret_cast<const void *>( super_diag_kernel<float, 32> ), super_diag_smem<float>( 32 ) },
+        { reinterpret_cast<const void *>( super_diag_kernel<double, 64> ), super_diag_smem<double>( 64 ) },
+        { reinterpret_cast<const void *>( super_diag_kernel<float, 64> ), super_diag_smem<float>( 64 ) },
         { reinterpret_cast<const void *>( super_rest_kernel<double, 8> ), super_rest_smem<double>( 8 ) },
         { reinterpret_cast<const void *>( super_rest_kernel<double, 16> ), super_rest_smem<double>( 16 ) },
         { reinterpret_cast<const void *>( super_rest_kernel<double, 32> ), super_rest_smem<double>( 32 ) },

@@ -141,8 +141,10 @@ int solve_dag_blocks_per_sm( int k );
 template<typename T>
 void launch_super_inv( const SuperInvTask * tasks, int count, int part, const SuperPanel * sps, const T * arena, const double * tinv,
                        double * tbuf, cudaStream_t st );
-void launch_super_diag( const SuperSolveTask * tasks, int count, const SuperPanel * sps, const double * tbuf, bool upper,
-                        const double * in, const double * zbuf, double * out, int ld, int k, cudaStream_t st );
+template<typename T>
+void launch_super_diag( const SuperSolveTask * tasks, int count, const SolveRestTask * steps, int nsteps, const SuperPanel * sps,
+                        const double * tbuf, const T * arena, const double * tinv, const std::int32_t * sn_inner, bool upper,
+                        double * in, const double * zbuf, double * out, int ld, int k, cudaStream_t st );
 template<typename T>
 void launch_super_rest( const SuperSolveTask * tasks, int count, const SuperPanel * sps, const T * arena,
                         const std::int32_t * sn_inner, bool upper, double * in, double * zbuf, const double * out, int ld, int k,

@@ -1121,10 +1121,16 @@ void Plan::build_super( const std::vector<std::vector<I32>> & front_panels, Rang
             }
             else
             {
-                const I32 rest = (sp.n0 - sp.r0 - sp.rows) + sp.n1;
+                // chunks lie in U0 or in U1 alone (aligned vector copies)
+                const I32 m = sp.n0 - sp.r0 - sp.rows, rest = m + sp.n1;
                 for( I32 b = 0; b < nblk; ++b )
                 {
-                    for( I32 c0 = 0; c0 < rest; c0 += kSolveRest ) { ssolve.push_back( { p, b, c0, std::min( rest, c0 + kSolveRest ) } ); }
+                    for( I32 c0 = 0; c0 < rest; )
+                    {
+                        const I32 c1 = std::min( c0 < m ? m : rest, c0 + kSolveRest );
+                        ssolve.push_back( { p, b, c0, c1 } );
+                        c0 = c1;
+                    }
                 }
             }
         }
@@ -1136,9 +1142,17 @@ void Plan::build_super( const std::vector<std::vector<I32>> & front_panels, Rang
             list.push_back( L );
         }
     };
+    // (a level with super-panels has one panel step at most, that of its one-panel fronts: it runs
+    // in the level's first diag launch, its tasks [tc_first, tc_first + tc_count) of srest)
+    auto with_steps = [&]( I32 h, Launch & L )
+    {
+        if( ranges( h ) == 0 || regular[static_cast<size_t>(h)][0] == 0 ) { return; }
+        L.tc_first = range_of( h, 0 ).first;
+        L.tc_count = regular[static_cast<size_t>(h)][0];
+    };
     for( I32 h = 0; h < levels; ++h )
     {
-        for( size_t q = 0; q < ranges( h ); ++q )
+        for( size_t q = 0; q < ranges( h ) && super_steps( h ) == 0; ++q )
         {
             const auto r = range_of( h, q );
             const I32 nreg = regular[static_cast<size_t>(h)][q];
@@ -1147,6 +1161,7 @@ void Plan::build_super( const std::vector<std::vector<I32>> & front_panels, Rang
         for( size_t st = 0; st < super_steps( h ); ++st )
         {
             push_super( lower_launches_sp, h, st, true, true );
+            if( st == 0 ) { with_steps( h, lower_launches_sp.back() ); }
             push_super( lower_launches_sp, h, st, false, true );
         }
     }
@@ -1156,8 +1171,9 @@ void Plan::build_super( const std::vector<std::vector<I32>> & front_panels, Rang
         {
             push_super( upper_launches_sp, h, st, false, false );
             push_super( upper_launches_sp, h, st, true, false );
+            if( st + 1 == super_steps( h ) ) { with_steps( h, upper_launches_sp.back() ); }
         }
-        for( size_t q = ranges( h ); q-- > 0; )
+        for( size_t q = super_steps( h ) == 0 ? ranges( h ) : 0; q-- > 0; )
         {
             const auto r = range_of( h, q );
             const I32 nreg = regular[static_cast<size_t>(h)][q];

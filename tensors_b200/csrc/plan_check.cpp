@@ -726,6 +726,17 @@ std::string check_panels( const Symbolic & sym, const Plan & pl )
                 {
                     return "super solve list: launch out of bounds";
                 }
+                if( L.tc_count < 0 || L.tc_first < 0 || L.tc_first + L.tc_count > static_cast<I64>( pl.srest.size() ) || (L.tc_count > 0 && L.kind != LaunchKind::SuperDiag) )
+                {
+                    return "super solve list: panel steps out of bounds";
+                }
+                for( I64 t = L.tc_first; t < L.tc_first + L.tc_count; ++t )
+                {
+                    // (one-panel fronts: their step depends on no other one of the level)
+                    const SolveRestTask & r = pl.srest[static_cast<size_t>( t )];
+                    if( big_panel[static_cast<size_t>( r.panel )] || r.n0 > kPanel ) { return "super solve list: a large front's panel step"; }
+                }
+                regular += L.tc_count;
                 for( I64 t = L.first; t < L.first + L.count; ++t )
                 {
                     const SuperSolveTask & v = pl.ssolve[static_cast<size_t>( t )];
@@ -741,6 +752,10 @@ std::string check_panels( const Symbolic & sym, const Plan & pl )
                     else
                     {
                         if( v.c0 < 0 || v.c1 > nrest[p] || v.c0 >= v.c1 || v.c1 - v.c0 > kSolveRest ) { return "super solve rest rows out of range"; }
+                        // (16-byte pieces: inside U0 or U1, at a multiple of 4 entries there)
+                        const SuperPanel & sp = pl.spanels[p];
+                        const I32 m = sp.n0 - sp.r0 - sp.rows;
+                        if( (v.c0 < m && v.c1 > m) || (v.c0 < m ? sp.r0 + sp.rows + v.c0 : v.c0 - m) % 4 != 0 || (sp.u0 | sp.u1) % 4 != 0 || (sp.ld0 | sp.ld1) % 4 != 0 ) { return "super solve rest chunk alignment"; }
                         rest[p] += v.c1 - v.c0;
                     }
                 }
