@@ -841,12 +841,12 @@ std::int64_t issue_sweeps( tb_chol * h, int which, double * W, double * Y, std::
         }
         else if( mixed )
         {
-            tb::launch_solve_step( h->srest.ptr + L.first, L.count, upper, arena_as<float>( h ), h->tinv.ptr,
+            tb::launch_solve_step( h->srest.ptr + L.first, L.count, L.small_count, upper, arena_as<float>( h ), h->tinv.ptr,
                                    h->sn_inner.ptr, in, out, k, kc, st );
         }
         else
         {
-            tb::launch_solve_step( h->srest.ptr + L.first, L.count, upper, arena_as<double>( h ), h->tinv.ptr,
+            tb::launch_solve_step( h->srest.ptr + L.first, L.count, L.small_count, upper, arena_as<double>( h ), h->tinv.ptr,
                                    h->sn_inner.ptr, in, out, k, kc, st );
         }
         end( L.level, L.step, L.count + (L.kind == tb::LaunchKind::SuperDiag ? L.tc_count : 0), upper ? 1 : 0 );

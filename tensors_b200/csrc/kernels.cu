@@ -1973,9 +1973,203 @@ __device__ __forceinline__ void solve_step_body( const SolveRestTask & t, int up
     }
 }
 
-// One kernel per right-hand-side width KP, so that each gets the registers it needs.
+// The same step of a tiny front (Launch::small_count) by one warp: no shared
+// memory, every operand is loaded from global memory as the DMMA fragment it is
+// used as, 16 columns of the right-hand sides at a time, and the product with T
+// changes from accumulator to operand layout by shuffles.  A CTA per such front
+// spent its time on two block barriers and on occupancy (2 to 4 an SM); of a
+// grid's leaves half have one row and six rest rows.  C2 with 16 right-hand
+// sides 1.22 -> 1.11 ms, 56^3 with 64 2.01 -> 1.89 ms, 96 meshes 481 -> 404 us.
 template<typename T, int KP>
-__global__ __launch_bounds__(kSolveThreads) void solve_step_kernel( const SolveRestTask * __restrict__ tasks, int upper,
+__device__ __forceinline__ void solve_warp_body( const SolveRestTask & t, int upper, const T * __restrict__ arena,
+                                                 const double * __restrict__ tinv, const std::int32_t * __restrict__ sn_inner,
+                                                 double * in, double * out, int ld, int k )
+{
+    constexpr int NC = KP == 8 ? 1 : 2;                  // 8-column tiles at a time
+    constexpr int NT = kTinyRows / 8;
+    const int lane = threadIdx.x & 31, fq = lane >> 2, fr = lane & 3;
+    const int nb = t.n0, nt = (nb + 7) >> 3;             // (one panel: every rest column lies in U1)
+    const bool owner = t.c0 <= 0;
+    const int c0 = max( t.c0, 0 ), cw = t.c0 >= 0 ? t.c1 - t.c0 : 0;
+    const std::int64_t prow = t.row0;
+    const double * Tg = tinv + (std::int64_t)t.panel * (kPanel * kPanel);
+    const T * P = arena + t.u1 + c0;
+    const std::int32_t * rest = sn_inner + t.inner + c0;
+    // accumulator tile (row fq, columns 2 fr, 2 fr + 1) -> operand (row fr + 4 s, column fq)
+    auto turned = [&]( const double (&v)[2], int s )
+    {
+        const int src = 4 * (fr + 4 * s) + (fq >> 1);
+        const double a = __shfl_sync( 0xffffffffu, v[0], src ), b = __shfl_sync( 0xffffffffu, v[1], src );
+        return (fq & 1) ? b : a;
+    };
+    for( int cb = 0; cb < k; cb += 8 * NC )
+    {
+        double v[NT][2][NC];                             // operand: y, then x (forward); y - P x_r (back)
+        if( !upper )
+        {
+#pragma unroll
+            for( int kb = 0; kb < NT; ++kb )
+            {
+#pragma unroll
+                for( int s = 0; s < 2; ++s )
+                {
+#pragma unroll
+                    for( int ct = 0; ct < NC; ++ct )
+                    {
+                        const int r = 8 * kb + fr + 4 * s, c = cb + 8 * ct + fq;
+                        v[kb][s][ct] = r < nb && c < k ? in[(prow + r) * ld + c] : 0.0;
+                    }
+                }
+            }
+#pragma unroll
+            for( int rt = NT - 1; rt >= 0; --rt )
+            {
+                if( rt >= nt ) { continue; }
+                double acc[NC][2] = {};
+#pragma unroll
+                for( int kb = 0; kb <= rt; ++kb )
+                {
+#pragma unroll
+                    for( int s = 0; s < 2; ++s )
+                    {
+                        const double a = Tg[(8 * kb + fr + 4 * s) * kPanel + 8 * rt + fq];
+#pragma unroll
+                        for( int ct = 0; ct < NC; ++ct ) { dmma_8x8x4( acc[ct], a, v[kb][s][ct] ); }
+                    }
+                }
+#pragma unroll
+                for( int ct = 0; ct < NC; ++ct )
+                {
+                    const int r = 8 * rt + fq, c = cb + 8 * ct + 2 * fr;
+                    if( owner && r < nb )
+                    {
+                        if( c < k ) { out[(prow + r) * ld + c] = acc[ct][0]; }
+                        if( c + 1 < k ) { out[(prow + r) * ld + c + 1] = acc[ct][1]; }
+                    }
+#pragma unroll
+                    for( int s = 0; s < 2; ++s ) { v[rt][s][ct] = turned( acc[ct], s ); }
+                }
+            }
+#pragma unroll 1
+            for( int o = 0; o < cw; o += 8 )
+            {
+                const bool ok = o + fq < cw;
+                const std::int64_t row = ok ? rest[o + fq] : 0;
+                double a[NT][2];
+#pragma unroll
+                for( int kb = 0; kb < NT; ++kb )
+                {
+#pragma unroll
+                    for( int s = 0; s < 2; ++s )
+                    {
+                        const int r = 8 * kb + fr + 4 * s;
+                        a[kb][s] = ok && r < nb ? static_cast<double>( P[(std::int64_t)r * t.ld1 + o + fq] ) : 0.0;
+                    }
+                }
+                double acc[NC][2] = {};
+#pragma unroll
+                for( int kb = 0; kb < NT; ++kb )
+                {
+                    if( kb >= nt ) { break; }
+#pragma unroll
+                    for( int s = 0; s < 2; ++s )
+                    {
+#pragma unroll
+                        for( int ct = 0; ct < NC; ++ct ) { dmma_8x8x4( acc[ct], a[kb][s], v[kb][s][ct] ); }
+                    }
+                }
+                if( ok )
+                {
+#pragma unroll
+                    for( int ct = 0; ct < NC; ++ct )
+                    {
+                        const int c = cb + 8 * ct + 2 * fr;
+                        if( c < k ) { red_add_f64( in + row * ld + c, -acc[ct][0] ); }
+                        if( c + 1 < k ) { red_add_f64( in + row * ld + c + 1, -acc[ct][1] ); }
+                    }
+                }
+            }
+        }
+        else
+        {
+            double acc[NT][NC][2] = {};
+#pragma unroll 1
+            for( int o = 0; o < cw; o += 8 )
+            {
+#pragma unroll
+                for( int s = 0; s < 2; ++s )
+                {
+                    const int j = o + fr + 4 * s;
+                    const std::int64_t row = j < cw ? rest[j] : 0;
+                    double x[NC];
+#pragma unroll
+                    for( int ct = 0; ct < NC; ++ct )
+                    {
+                        const int c = cb + 8 * ct + fq;
+                        x[ct] = j < cw && c < k ? out[row * ld + c] : 0.0;
+                    }
+#pragma unroll
+                    for( int rt = 0; rt < NT; ++rt )
+                    {
+                        if( rt >= nt ) { break; }
+                        const int r = 8 * rt + fq;
+                        const double a = r < nb && j < cw ? static_cast<double>( P[(std::int64_t)r * t.ld1 + j] ) : 0.0;
+#pragma unroll
+                        for( int ct = 0; ct < NC; ++ct ) { dmma_8x8x4( acc[rt][ct], a, x[ct] ); }
+                    }
+                }
+            }
+#pragma unroll
+            for( int rt = 0; rt < NT; ++rt )
+            {
+#pragma unroll
+                for( int ct = 0; ct < NC; ++ct )
+                {
+                    const int r = 8 * rt + fq, c = cb + 8 * ct + 2 * fr;
+                    double d[2];
+#pragma unroll
+                    for( int e = 0; e < 2; ++e ) { d[e] = (owner && r < nb && c + e < k ? in[(prow + r) * ld + c + e] : 0.0) - acc[rt][ct][e]; }
+#pragma unroll
+                    for( int s = 0; s < 2; ++s ) { v[rt][s][ct] = turned( d, s ); }
+                }
+            }
+#pragma unroll
+            for( int rt = 0; rt < NT; ++rt )
+            {
+                if( rt >= nt ) { break; }
+                double z[NC][2] = {};
+#pragma unroll
+                for( int kb = rt; kb < NT; ++kb )
+                {
+                    if( kb >= nt ) { break; }
+#pragma unroll
+                    for( int s = 0; s < 2; ++s )
+                    {
+                        const double a = Tg[(8 * rt + fq) * kPanel + 8 * kb + fr + 4 * s];
+#pragma unroll
+                        for( int ct = 0; ct < NC; ++ct ) { dmma_8x8x4( z[ct], a, v[kb][s][ct] ); }
+                    }
+                }
+                const int r = 8 * rt + fq;
+                if( r < nb )
+                {
+#pragma unroll
+                    for( int ct = 0; ct < NC; ++ct )
+                    {
+                        const int c = cb + 8 * ct + 2 * fr;
+                        if( c < k ) { red_add_f64( out + (prow + r) * ld + c, z[ct][0] ); }
+                        if( c + 1 < k ) { red_add_f64( out + (prow + r) * ld + c + 1, z[ct][1] ); }
+                    }
+                }
+            }
+        }
+    }
+}
+
+// One kernel per right-hand-side width KP, so that each gets the registers it needs: a CTA for
+// each of the first `ctas` tasks, a warp for each of the others.
+template<typename T, int KP>
+__global__ __launch_bounds__(kSolveThreads) void solve_step_kernel( const SolveRestTask * __restrict__ tasks, int ctas, int count, int upper,
                                                                     const T * __restrict__ arena,
                                                                     const double * __restrict__ tinv,
                                                                     const std::int32_t * __restrict__ sn_inner,
@@ -1983,7 +2177,16 @@ __global__ __launch_bounds__(kSolveThreads) void solve_step_kernel( const SolveR
 {
     extern __shared__ __align__(16) double ssm[];
     pdl_allow_next();
-    solve_step_body<T, KP, true>( tasks[blockIdx.x], upper, arena, tinv, sn_inner, in, out, ld, k, false, ssm );
+    if( static_cast<int>( blockIdx.x ) < ctas )
+    {
+        solve_step_body<T, KP, true>( tasks[blockIdx.x], upper, arena, tinv, sn_inner, in, out, ld, k, false, ssm );
+        return;
+    }
+    const int i = ctas + (blockIdx.x - ctas) * (kSolveThreads / 32) + (threadIdx.x >> 5);
+    if( i >= count ) { return; }
+    const SolveRestTask t = tasks[i];
+    pdl_wait();
+    solve_warp_body<T, KP>( t, upper, arena, tinv, sn_inner, in, out, ld, k );
 }
 
 // The solve's task graph (Plan::solve_*) as one persistent launch per sweep:
@@ -2998,18 +3201,19 @@ int solve_dag_blocks_per_sm( int k )
 }
 
 template<typename T>
-void launch_solve_step( const SolveRestTask * tasks, int count, bool upper, const T * arena, const double * tinv,
+void launch_solve_step( const SolveRestTask * tasks, int count, int small_count, bool upper, const T * arena, const double * tinv,
                         const std::int32_t * sn_inner, double * in, double * out, int ld, int k, cudaStream_t st )
 {
     if( count <= 0 ) { return; }
-    const size_t sm = solve_smem_bytes<T>( k );
-    const int u = upper ? 1 : 0;
+    const size_t sm = small_count < count ? solve_smem_bytes<T>( k ) : 0;
+    constexpr int kWarps = kSolveThreads / 32;
+    const int u = upper ? 1 : 0, ctas = count - small_count, grid = ctas + (small_count + kWarps - 1) / kWarps;
     switch( solve_lkp( k ) )
     {
-        case 3:  launch_pdl( solve_step_kernel<T, 8>, count, kSolveThreads, sm, st, tasks, u, arena, tinv, sn_inner, in, out, ld, k ); break;
-        case 4:  launch_pdl( solve_step_kernel<T, 16>, count, kSolveThreads, sm, st, tasks, u, arena, tinv, sn_inner, in, out, ld, k ); break;
-        case 5:  launch_pdl( solve_step_kernel<T, 32>, count, kSolveThreads, sm, st, tasks, u, arena, tinv, sn_inner, in, out, ld, k ); break;
-        default: launch_pdl( solve_step_kernel<T, 64>, count, kSolveThreads, sm, st, tasks, u, arena, tinv, sn_inner, in, out, ld, k ); break;
+        case 3:  launch_pdl( solve_step_kernel<T, 8>, grid, kSolveThreads, sm, st, tasks, ctas, count, u, arena, tinv, sn_inner, in, out, ld, k ); break;
+        case 4:  launch_pdl( solve_step_kernel<T, 16>, grid, kSolveThreads, sm, st, tasks, ctas, count, u, arena, tinv, sn_inner, in, out, ld, k ); break;
+        case 5:  launch_pdl( solve_step_kernel<T, 32>, grid, kSolveThreads, sm, st, tasks, ctas, count, u, arena, tinv, sn_inner, in, out, ld, k ); break;
+        default: launch_pdl( solve_step_kernel<T, 64>, grid, kSolveThreads, sm, st, tasks, ctas, count, u, arena, tinv, sn_inner, in, out, ld, k ); break;
     }
 }
 
@@ -3085,7 +3289,7 @@ void launch_gather_diag( const std::int64_t * offsets, const T * arena, double *
     template void launch_gemm<T>( const GemmTask *, int, T *, int *, cudaStream_t, bool );                                 \
     template void launch_solve_dag<T>( const SolveDagArgs &, int, const T *, double *, double *, int, int, cudaStream_t );                                        \
     template void launch_factor_dag<T>( const DagArgs &, int, cudaStream_t );                                        \
-    template void launch_solve_step<T>( const SolveRestTask *, int, bool, const T *, const double *,                \
+    template void launch_solve_step<T>( const SolveRestTask *, int, int, bool, const T *, const double *,                \
                                         const std::int32_t *, double *, double *, int, int, cudaStream_t );         \
     template void launch_gather_diag<T>( const std::int64_t *, const T *, double *, int, cudaStream_t );          \
     template void launch_super_inv<T>( const SuperInvTask *, int, int, const SuperPanel *, const T *, const double *,      \

@@ -97,10 +97,11 @@ template<typename T> void launch_factor_dag( const DagArgs & args, int grid, cud
 // Resident CTAs per SM of the persistent kernel (0 on error).
 int factor_dag_blocks_per_sm();
 
-// One forward (upper = false) or backward solve step over `count` tasks;
+// One forward (upper = false) or backward solve step over `count` tasks, the last
+// small_count of them tiny fronts (kTinyRows), a warp each;
 // in / out row-major with leading dimension ld, k <= kSolveMaxRhs columns.
 template<typename T>
-void launch_solve_step( const SolveRestTask * tasks, int count, bool upper, const T * arena, const double * tinv,
+void launch_solve_step( const SolveRestTask * tasks, int count, int small_count, bool upper, const T * arena, const double * tinv,
                         const std::int32_t * sn_inner, double * in, double * out, int ld, int k, cudaStream_t st );
 
 // The levels of the solve task graph as one persistent launch per sweep

@@ -997,6 +997,24 @@ void Plan::build( const Symbolic & sym )
     build_super( front_panels, [&]( I32 h, size_t q ) { return std::make_pair( rest_ranges[static_cast<size_t>(h)][q].first,
                                                                               rest_ranges[static_cast<size_t>(h)][q].count ); },
                  [&]( I32 h ) { return rest_ranges[static_cast<size_t>(h)].size(); }, by_level );
+    // the tiny fronts' tasks behind the others (not in levels with super-panels,
+    // whose panel steps run beside other work)
+    std::vector<I32> tiny( static_cast<size_t>(levels), 0 );
+    std::vector<char> has_super( static_cast<size_t>(levels), 0 );
+    for( const Launch & L : lower_launches_sp ) { if( L.kind == LaunchKind::SuperDiag ) { has_super[static_cast<size_t>( L.level )] = 1; } }
+    for( I32 h = 0; h < levels; ++h )
+    {
+        if( rest_ranges[static_cast<size_t>(h)].empty() || has_super[static_cast<size_t>(h)] ) { continue; }
+        const auto r = rest_ranges[static_cast<size_t>(h)][0];
+        auto small = []( const SolveRestTask & t ) { return t.n0 <= kTinyRows && t.c1 - std::max( t.c0, 0 ) <= kTinyRest; };
+        auto b = srest.begin() + r.first, e = b + r.count;
+        std::stable_partition( b, e, [&]( const SolveRestTask & t ) { return !small( t ); } );
+        tiny[static_cast<size_t>(h)] = static_cast<I32>( std::count_if( b, e, small ) );
+    }
+    for( std::vector<Launch> * list : { &lower_launches, &upper_launches, &lower_launches_sp, &upper_launches_sp } )
+    {
+        for( Launch & L : *list ) { if( L.kind == LaunchKind::Solve && L.step == 0 ) { L.small_count = tiny[static_cast<size_t>( L.level )]; } }
+    }
     build_solve_graph( sym, solve_split );
 }
 

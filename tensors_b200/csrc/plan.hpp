@@ -261,6 +261,13 @@ constexpr std::int64_t front_smem_bytes( std::int64_t n0, std::int64_t n1 )
     return 8 * (a * (a + b + 4) + a * (a + 4) + 4 * b * (b / 8 + 1) + kPanel + 2);
 }
 
+// Solve steps of fronts of at most kTinyRows rows and kTinyRest rest rows run a warp each, the
+// others a CTA each.  A warp walks its rest rows eight at a
+// time: with 32 or 64 of them it is slower than a CTA (C2 1.11 ms at 16, 1.12 at 32, 1.16 at 64;
+// 56^3 with 64 right-hand sides 1.89, 1.94, 2.05), and so it is with up to 32 pivot rows (C2 1.55).
+constexpr int kTinyRows = 8;
+constexpr int kTinyRest = 16;
+
 // The solve of a large front steps through its pivot rows 512 at a time
 // (super-panels) instead of 64 at a time: the inverse of each 512 x 512
 // diagonal block of U0 (T, FP64, upper triangular, row-major, built from
@@ -335,6 +342,7 @@ struct Launch
     std::int64_t tc_first = 0;
     std::int32_t tc_count = 0;
     std::int32_t small_count = 0;
+    // Solve launches: the last small_count tasks are tiny fronts (kTinyRows), a warp each
     // Front launches: small_count = the launch's shared memory in bytes, tc_count = its threads; part 1: other
     // fronts of the level keep their launches (the two may run side by side)
     // ExtendPull launches: the level's extend tasks in pass order are

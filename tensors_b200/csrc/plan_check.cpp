@@ -628,6 +628,19 @@ std::string check_panels( const Symbolic & sym, const Plan & pl )
         }
     }
     { const std::string msg = check_task_graph( pl ); if( !msg.empty() ) { return msg; } }
+    for( const std::vector<Launch> * list : { &pl.lower_launches, &pl.upper_launches, &pl.lower_launches_sp, &pl.upper_launches_sp } )
+    {
+        for( const Launch & L : *list )
+        {
+            if( L.kind != LaunchKind::Solve ) { continue; }
+            if( L.count < 0 || L.first < 0 || L.first + L.count > static_cast<I64>( pl.srest.size() ) || L.small_count < 0 || L.small_count > L.count ) { return "solve launch out of bounds"; }
+            for( I64 t = L.first + L.count - L.small_count; t < L.first + L.count; ++t )
+            {
+                const SolveRestTask & r = pl.srest[static_cast<size_t>( t )];
+                if( r.n0 > kTinyRows || r.r0 != 0 || r.c1 - r.c0 > kTinyRest + (r.c0 < 0 ? 1 : 0) ) { return "solve launch: a front too large for a warp"; }
+            }
+        }
+    }
     for( const Launch & L : pl.lower_launches ) { if( L.kind != LaunchKind::Solve ) { return "unexpected launch kind in the forward solve"; } }
     for( const Launch & L : pl.upper_launches ) { if( L.kind != LaunchKind::Solve ) { return "unexpected launch kind in the back solve"; } }
     if( !pl.spanels.empty() )
