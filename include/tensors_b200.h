@@ -336,7 +336,8 @@ int tb_chol_solve_trace( tb_chol * h, int64_t * out, int64_t cap );
 /* Per-kernel timing: when enabled, factorizations run as direct launches
  * bracketed by CUDA events and tb_chol_kernel_profile reports, per launch
  * kind (0 zero, 1 extend-add, 2 panel trsm, 3 GEMM tiles, 4 inversion of
- * the diagonal blocks for the solves, 6 panel potrf, 7 clear + assembly),
+ * the diagonal blocks for the solves, 5 small fronts taken whole, 6 panel
+ * potrf, 7 clear + assembly),
  * the milliseconds and launches of the last factorization and the
  * algorithmic flops of the GEMM tiles (8 entries each). */
 int tb_chol_set_profiling( tb_chol * h, int32_t enabled );

@@ -2693,8 +2693,8 @@ __device__ __forceinline__ int super_block_rows( const SuperPanel & sp, int b ) 
 // i's inverse.  The sum over k streams through two stages of 32 columns of the
 // left and 32 rows of the right blocks.  Doubling needs 14 block products in a
 // row where the back substitution by distance from the diagonal needed 35
-// (C2: 370 us in eight launches); diagonal blocks are read from the panels'
-// inverses.
+// (C2: 0.37 ms of launches -> 0.18, timed one by one); diagonal blocks are read
+// from the panels' inverses.
 constexpr int kInvK = 32;
 constexpr int kInvLda = kInvK + 4;                      // (conflict-free DMMA fragments, as kPld)
 constexpr int kInvStage = kPanel * kInvLda + kInvK * kPld;
