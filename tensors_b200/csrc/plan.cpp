@@ -1018,7 +1018,7 @@ void Plan::build( const Symbolic & sym )
     build_solve_graph( sym, solve_split );
 }
 
-// The super-panel solve: super-panels of the large fronts, the rounds of their
+// The super-panel solve: super-panels of the large fronts, the products of their
 // inverses, and the solve launch lists in which their panel steps are replaced.
 // Within each (level, step) range of srest the tasks of the large fronts are
 // moved behind the others (the order inside a range is free: its tasks are

@@ -271,12 +271,13 @@ constexpr int kTinyRest = 16;
 // The solve of a large front steps through its pivot rows 512 at a time
 // (super-panels) instead of 64 at a time: the inverse of each 512 x 512
 // diagonal block of U0 (T, FP64, upper triangular, row-major, built from
-// the 64-row panel inverses after the factorization by block back
-// substitution) turns eight sequential panel steps into one.  A level uses
-// super-panels for every front of more than one panel when its largest front
-// has at least kSuperMinRows pivot rows: it then runs three launches where the
-// panel steps of its fronts below that size alone took up to four (56^3 grid, 64
-// right-hand sides: 3.15 -> 2.93 ms; 40^3 grid: 354 -> 295 us).  Lower lines
+// the 64-row panel inverses after the factorization by doubling) turns eight
+// sequential panel steps into one.  A level uses super-panels for every front of
+// more than one panel when its largest front has at least kSuperMinRows pivot
+// rows: it then runs two launches a super-panel step (its one-panel fronts in the
+// first) where the panel steps of its fronts below that size alone took up to
+// four (56^3 grid, 64 right-hand sides: 3.15 -> 2.93 ms; 40^3 grid: 354 -> 299
+// us, with the one-panel fronts still in a launch of their own).  Lower lines
 // cost more inverses than they save steps (the largest front at 193 rows:
 // 131^2 mesh factor 394 -> 418 us, solve 90 -> 78 us).
 constexpr int kSuperPanels  = 8;
