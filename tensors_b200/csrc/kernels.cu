@@ -463,6 +463,7 @@ __device__ __forceinline__ bool potrf_diag_tile( const PotrfShared<kLd> & sh, co
 #pragma unroll
         for( int c = r; c < kSub; ++c ) { a[r][c] = sh.D( o + r, o + c ); }
     }
+    __syncwarp();                                       // every lane has the tile before lane 0 writes rows over it
     auto store_row = [&]( int r, const double (&v)[kSub] )
     {
         if( lane != 0 ) { return; }
