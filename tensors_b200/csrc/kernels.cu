@@ -410,13 +410,27 @@ template<typename T> __device__ __forceinline__ double round_to( double v ) { re
 // triangle (A, overwritten by U tile row by tile row); Ti: the inverse
 // T = U^{-1}, upper 8 x 8 tiles (the diagonal tiles are zero below the
 // diagonal).  kLd: the leading dimension of both, 0: given at run time.
+//
+// kIllPivot (FP64): a diagonal tile with a pivot below 1 / kIllPivot of its
+// diagonal entry (a pivot's ratio does not change when rows and columns are
+// scaled) solves its row block by substitution.  The product with the tile's
+// inverse is exact to a few roundings only while the inverse stays small: with
+// every third row within 1e-10 (squared) of the one before, |U^T U - A| is 4
+// u |A| by substitution and 12,800 by the product, and from 1e-11 on the
+// product's errors make a later pivot negative.  The line lies where both
+// agree: with rows within 1e-2 every such tile is below it and the product
+// still as good.  A grid Laplacian's separator has no tile below it; the check
+// alone makes a factor 0 to 1.5% slower (31^3 grid 1450 -> 1468 us),
+// substitution in every tile 1 to 8%.
+constexpr double kIllPivot = 16.0;
+
 template<int kLd>
 struct PotrfShared
 {
     double * d;
     double * ti;
     int ldd, ldt;                                       // used when kLd == 0
-    double * floor_s;                                   // the panel's pivot floors (mixed precision)
+    double * floor_s;                                   // mixed precision: the panel's pivot floors; FP64: ill()'s place
     int * flags;                                        // first failing row (-1: none); a tile to factor again; bit q: tile
                                                         // q has raised pivots (the last two: mixed precision)
     __device__ __forceinline__ double & D( int r, int c ) const { return d[r * (kLd > 0 ? kLd : ldd) + c]; }
@@ -424,6 +438,7 @@ struct PotrfShared
     __device__ __forceinline__ int & fail() const { return flags[0]; }
     __device__ __forceinline__ int & redo() const { return flags[1]; }
     __device__ __forceinline__ int & raised() const { return flags[2]; }
+    __device__ __forceinline__ int & ill( int q ) const { return reinterpret_cast<int *>( floor_s )[q]; }   // FP64: see kIllPivot
 };
 
 // Cholesky of the diagonal tile q of D by one warp, and W = U_qq^{-1} into
@@ -463,6 +478,9 @@ __device__ __forceinline__ bool potrf_diag_tile( const PotrfShared<kLd> & sh, co
 #pragma unroll
         for( int c = r; c < kSub; ++c ) { a[r][c] = sh.D( o + r, o + c ); }
     }
+    // FP64: lane r (mod 8) keeps diagonal entry r and, below, its pivot
+    const double entry = sh.D( o + (lane & (kSub - 1)), o + (lane & (kSub - 1)) );
+    double pivot = entry;
     __syncwarp();                                       // every lane has the tile before lane 0 writes rows over it
     auto store_row = [&]( int r, const double (&v)[kSub] )
     {
@@ -506,6 +524,7 @@ __device__ __forceinline__ bool potrf_diag_tile( const PotrfShared<kLd> & sh, co
             else { if( o + r < nb && !(d > tau) ) { low |= 1u << r; } }
         }
         if( !(d > 0.0) ) { nonpos |= 1u << r; }
+        if( (lane & (kSub - 1)) == r ) { pivot = d; }
         const double iv = rsqrt( d );
         double us[kSub];
         a[r][r] = d * iv;
@@ -533,6 +552,11 @@ __device__ __forceinline__ bool potrf_diag_tile( const PotrfShared<kLd> & sh, co
     if constexpr ( sizeof(T) == 4 && !kFloored )
     {
         if( low != 0u && pivot_floor != nullptr ) { return false; }
+    }
+    if constexpr ( sizeof(T) == 8 )
+    {
+        const bool ill = __any_sync( 0xffffffffu, kIllPivot * pivot < entry );
+        if( lane == 0 ) { sh.ill( q ) = ill ? 1 : 0; }
     }
     nonpos &= ~singles;
     if( nb - o < kSub ) { nonpos &= (1u << (nb - o)) - 1u; }
@@ -577,7 +601,7 @@ __device__ __noinline__ void potrf_row_substitution( const PotrfShared<kLd> sh, 
 #pragma unroll
         for( int r = 0; r < kSub; ++r )
         {
-            x[r] *= sh.Ti( kPanel - kSub + r, o + r );      // the pivot's reciprocal
+            x[r] *= sh.Ti( (sizeof(T) == 4 ? kPanel - kSub : o) + r, o + r );      // the pivot's reciprocal
 #pragma unroll
             for( int r2 = r + 1; r2 < kSub; ++r2 ) { x[r2] -= sh.D( o + r, o + r2 ) * x[r]; }
         }
@@ -599,18 +623,15 @@ __device__ __forceinline__ void potrf_core( const PotrfShared<kLd> & sh, const P
     T * U0 = arena + t.u0 + (std::int64_t)t.r0 * t.ld0 + t.r0;
     const int nsub = (nb + kSub - 1) / kSub;
     const int i8 = lane >> 2, j8 = 2 * (lane & 3);        // this lane's entries of an 8 x 8 DMMA result
-    // U_bc = W_b^T A_bc in place (tile (b, c) of D), rounded to the storage type.  Mixed precision,
-    // tiles with raised pivots: by substitution, as a raised pivot next to large entries makes W_b's
-    // entries grow beyond what the product can cancel.
+    // U_bc = W_b^T A_bc in place (tile (b, c) of D), rounded to the storage type.  By substitution
+    // where W_b's entries may grow beyond what the product can cancel: FP64 tiles with a small pivot
+    // (kIllPivot), mixed precision tiles with raised pivots.
     auto row_tile = [&]( int o, int oc )
     {
-        if constexpr ( sizeof(T) == 4 )
+        if( sizeof(T) == 4 ? (sh.raised() >> (o / kSub)) & 1 : sh.ill( o / kSub ) )
         {
-            if( (sh.raised() >> (o / kSub)) & 1 )
-            {
-                potrf_row_substitution<T>( sh, o, oc );
-                return;
-            }
+            potrf_row_substitution<T>( sh, o, oc );
+            return;
         }
         const int ow = sizeof(T) == 4 ? kPanel - kSub : o;
         double acc[2] = { 0.0, 0.0 };
