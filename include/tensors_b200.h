@@ -154,7 +154,8 @@ int tb_chol_solve_device_ex( tb_chol * h, double alpha, const void * d_B, int32_
 
 /* NumericalFactorization_T (CholeskyDecomposition.hpp:132-201): a numeric
  * factor held apart from any handle (device memory: the factor storage, the
- * inverse diagonal blocks and the values it was computed from).  A new one is
+ * inverse diagonal blocks of its panels and super-panels, and the values it was
+ * computed from).  A new one is
  * empty (not factorized).  tb_factor_state: NumericallyFactorizedQ,
  * NumericallyGoodQ, AllocatedByteCount and the precision of the stored factor
  * (-1 when it never held one). */

@@ -2656,13 +2656,14 @@ int tb_chol_launch_counts( tb_chol * h, std::int64_t * factor_launches, std::int
 // NumericalFactorization_T (CholeskyDecomposition.hpp:132-201): a numeric
 // factor held apart from any handle.  Here it is the device state a
 // factorization leaves behind: the front storage (FP64, or FP32 in the
-// mixed-precision mode), the inverse diagonal blocks the solves use, the
+// mixed-precision mode), the inverse diagonal blocks of the panels and
+// super-panels, which the solves use, the
 // matrix values and shift the mixed mode's refinement needs, and the
 // factorized / good flags.
 struct tb_factor
 {
     int device = -1;
-    DeviceArray<double> arena, tinv, values;
+    DeviceArray<double> arena, tinv, tsuper, values;
     int precision = -1;                          // of the stored factor; -1: never held one
     double last_reg = 0.0;
     bool factorized = false, good = false, fell_back = false;
@@ -2710,7 +2711,7 @@ int tb_factor_state( tb_factor * f, std::int32_t * factorized, std::int32_t * go
     if( f == nullptr ) { return fail( TB_ERR_INVALID_ARGUMENT, "null factor" ); }
     if( factorized ) { *factorized = f->factorized ? 1 : 0; }
     if( good ) { *good = f->good ? 1 : 0; }
-    if( bytes ) { *bytes = 8 * (f->arena.size + f->tinv.size + f->values.size); }
+    if( bytes ) { *bytes = 8 * (f->arena.size + f->tinv.size + f->tsuper.size + f->values.size); }
     if( precision ) { *precision = f->precision; }
     return TB_OK;
 }
@@ -2731,6 +2732,7 @@ int tb_chol_swap_factor( tb_chol * h, tb_factor * f )
     const int incoming = f->precision;
     swap_arrays( h->arena, f->arena );
     swap_arrays( h->tinv, f->tinv );
+    swap_arrays( h->tsuper, f->tsuper );
     swap_arrays( h->values, f->values );
     std::swap( h->last_reg, f->last_reg );
     std::swap( h->factorized, f->factorized );
@@ -2751,7 +2753,7 @@ int tb_chol_swap_factor( tb_chol * h, tb_factor * f )
     if( h->factorized && !h->good ) { h->factorized = false; }
     const std::int64_t need_tinv = static_cast<std::int64_t>( h->plan.sdiag.size() ) * tb::kPanel * tb::kPanel;
     if( h->factorized && (h->arena.size < required_arena( h, h->precision ) || h->tinv.size < need_tinv
-                          || h->values.size < h->sym.nnz || h->arena.ptr == nullptr) )
+                          || h->tsuper.size < h->plan.super_inv_size || h->values.size < h->sym.nnz || h->arena.ptr == nullptr) )
     {
         h->factorized = false;
         h->good = false;
@@ -2764,6 +2766,7 @@ int tb_chol_swap_factor( tb_chol * h, tb_factor * f )
         // the device plan stays: storage too small for it is grown (its contents are then moot)
         TB_TRY( h->arena.reserve( required_arena( h, h->precision ) ) );
         TB_TRY( h->tinv.reserve( need_tinv ) );
+        if( h->plan.super_inv_size > 0 ) { TB_TRY( h->tsuper.reserve( h->plan.super_inv_size ) ); }
         TB_TRY( h->values.reserve( h->sym.nnz ) );
     }
     return TB_OK;
