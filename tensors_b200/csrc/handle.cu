@@ -164,6 +164,7 @@ struct tb_chol
     DeviceArray<tb::SuperInvTask>   sinv;
     DeviceArray<tb::SuperSolveTask> ssolve;
     DeviceArray<double>             tsuper;      // their 512 x 512 inverses
+    DeviceArray<int>                grown;       // their blocks that keep a guarded one from its inverse (SuperPanel::guard)
     DeviceArray<std::int64_t>       a_outer;     // caller-order pattern, for residuals
     DeviceArray<std::int32_t>       a_inner;
     DeviceArray<double>             values;      // caller-order values of the last factorization
@@ -345,6 +346,9 @@ int ensure_symbolic( tb_chol * h )
     return TB_OK;
 }
 
+// Ints of tb_chol::grown.
+std::int64_t grown_size( const tb_chol * h ) { return static_cast<std::int64_t>( tb::kGuardBlocks ) * static_cast<std::int64_t>( h->plan.spanels.size() ); }
+
 // Binds the handle's device and stream and uploads the plan (once per
 // symbolic analysis).  Everything before this point is host-only, so the
 // symbolic phase and its getters work without a GPU.
@@ -410,6 +414,7 @@ int ensure_device( tb_chol * h )
     TB_TRY( h->sinv.upload( pl.sinv, st_ ) );
     TB_TRY( h->ssolve.upload( pl.ssolve, st_ ) );
     if( pl.super_inv_size > 0 ) { TB_TRY( h->tsuper.reserve( pl.super_inv_size ) ); }
+    if( pl.super_inv_size > 0 ) { TB_TRY( h->grown.reserve( grown_size( h ) ) ); }
     TB_TRY( h->zero.upload( pl.zero, st_ ) );
     TB_TRY( h->exports.upload( pl.exports, st_ ) );
     TB_TRY( h->colmap.upload( pl.colmap, st_ ) );
@@ -562,7 +567,7 @@ std::int64_t issue_factor_t( tb_chol * h, bool timed, std::vector<int> * kinds )
         launches += pl.dag.empty() ? 0 : 1;
         for( const tb::Launch & L : pl.sinv_launches )
         {
-            tb::launch_super_inv( h->sinv.ptr + L.first, L.count, L.part, h->spanels.ptr, A, h->tinv.ptr, h->tsuper.ptr, st );
+            tb::launch_super_inv( h->sinv.ptr + L.first, L.count, L.part, h->spanels.ptr, A, h->tinv.ptr, h->tsuper.ptr, h->grown.ptr, st );
             ++launches;
         }
         return launches;
@@ -671,7 +676,7 @@ std::int64_t issue_factor_t( tb_chol * h, bool timed, std::vector<int> * kinds )
     // the large fronts' super-panel inverses for the solves (after every panel inverse exists)
     for( const tb::Launch & L : pl.sinv_launches )
     {
-        tb::launch_super_inv( h->sinv.ptr + L.first, L.count, L.part, h->spanels.ptr, A, h->tinv.ptr, h->tsuper.ptr, st );
+        tb::launch_super_inv( h->sinv.ptr + L.first, L.count, L.part, h->spanels.ptr, A, h->tinv.ptr, h->tsuper.ptr, h->grown.ptr, st );
         mark( static_cast<int>( tb::LaunchKind::Invert ) );
         ++launches;
     }
@@ -827,9 +832,9 @@ std::int64_t issue_sweeps( tb_chol * h, int which, double * W, double * Y, std::
         if( L.kind == tb::LaunchKind::SuperDiag )
         {
             const tb::SolveRestTask * steps = h->srest.ptr + L.tc_first;
-            if( mixed ) { tb::launch_super_diag( h->ssolve.ptr + L.first, L.count, steps, L.tc_count, h->spanels.ptr, h->tsuper.ptr,
+            if( mixed ) { tb::launch_super_diag( h->ssolve.ptr + L.first, L.count, steps, L.tc_count, h->spanels.ptr, h->tsuper.ptr, h->grown.ptr,
                                                  arena_as<float>( h ), h->tinv.ptr, h->sn_inner.ptr, upper, in, Z + c0, out, k, kc, st ); }
-            else        { tb::launch_super_diag( h->ssolve.ptr + L.first, L.count, steps, L.tc_count, h->spanels.ptr, h->tsuper.ptr,
+            else        { tb::launch_super_diag( h->ssolve.ptr + L.first, L.count, steps, L.tc_count, h->spanels.ptr, h->tsuper.ptr, h->grown.ptr,
                                                  arena_as<double>( h ), h->tinv.ptr, h->sn_inner.ptr, upper, in, Z + c0, out, k, kc, st ); }
         }
         else if( L.kind == tb::LaunchKind::SuperRest )
@@ -2664,6 +2669,7 @@ struct tb_factor
 {
     int device = -1;
     DeviceArray<double> arena, tinv, tsuper, values;
+    DeviceArray<int> grown;
     int precision = -1;                          // of the stored factor; -1: never held one
     double last_reg = 0.0;
     bool factorized = false, good = false, fell_back = false;
@@ -2711,7 +2717,7 @@ int tb_factor_state( tb_factor * f, std::int32_t * factorized, std::int32_t * go
     if( f == nullptr ) { return fail( TB_ERR_INVALID_ARGUMENT, "null factor" ); }
     if( factorized ) { *factorized = f->factorized ? 1 : 0; }
     if( good ) { *good = f->good ? 1 : 0; }
-    if( bytes ) { *bytes = 8 * (f->arena.size + f->tinv.size + f->tsuper.size + f->values.size); }
+    if( bytes ) { *bytes = 8 * (f->arena.size + f->tinv.size + f->tsuper.size + f->values.size) + 4 * f->grown.size; }
     if( precision ) { *precision = f->precision; }
     return TB_OK;
 }
@@ -2733,6 +2739,7 @@ int tb_chol_swap_factor( tb_chol * h, tb_factor * f )
     swap_arrays( h->arena, f->arena );
     swap_arrays( h->tinv, f->tinv );
     swap_arrays( h->tsuper, f->tsuper );
+    swap_arrays( h->grown, f->grown );
     swap_arrays( h->values, f->values );
     std::swap( h->last_reg, f->last_reg );
     std::swap( h->factorized, f->factorized );
@@ -2753,7 +2760,7 @@ int tb_chol_swap_factor( tb_chol * h, tb_factor * f )
     if( h->factorized && !h->good ) { h->factorized = false; }
     const std::int64_t need_tinv = static_cast<std::int64_t>( h->plan.sdiag.size() ) * tb::kPanel * tb::kPanel;
     if( h->factorized && (h->arena.size < required_arena( h, h->precision ) || h->tinv.size < need_tinv
-                          || h->tsuper.size < h->plan.super_inv_size || h->values.size < h->sym.nnz || h->arena.ptr == nullptr) )
+                          || h->tsuper.size < h->plan.super_inv_size || h->grown.size < grown_size( h ) || h->values.size < h->sym.nnz || h->arena.ptr == nullptr) )
     {
         h->factorized = false;
         h->good = false;
@@ -2767,6 +2774,7 @@ int tb_chol_swap_factor( tb_chol * h, tb_factor * f )
         TB_TRY( h->arena.reserve( required_arena( h, h->precision ) ) );
         TB_TRY( h->tinv.reserve( need_tinv ) );
         if( h->plan.super_inv_size > 0 ) { TB_TRY( h->tsuper.reserve( h->plan.super_inv_size ) ); }
+        if( h->plan.super_inv_size > 0 ) { TB_TRY( h->grown.reserve( grown_size( h ) ) ); }
         TB_TRY( h->values.reserve( h->sym.nnz ) );
     }
     return TB_OK;

@@ -2725,7 +2725,7 @@ constexpr size_t kSuperInvSmem = sizeof(double) * 2 * kInvStage;
 template<typename T>
 __global__ __launch_bounds__(256) void super_inv_kernel( const SuperInvTask * __restrict__ tasks, int part, const SuperPanel * __restrict__ sps,
                                                          const T * __restrict__ arena, const double * __restrict__ tinv,
-                                                         double * __restrict__ tbuf )
+                                                         double * __restrict__ tbuf, int * __restrict__ grown )
 {
     extern __shared__ __align__(16) double ism[];
     pdl_allow_next();
@@ -2753,6 +2753,27 @@ __global__ __launch_bounds__(256) void super_inv_kernel( const SuperInvTask * __
                 if( c + 1 < nbi ) { v.y = src[idx + 1]; }
             }
             *reinterpret_cast<double2 *>( out + (std::int64_t)r * ldt + c ) = v;
+        }
+        if( sp.guard )
+        {
+            // a column's entries of U over its diagonal entry, squared and summed over the block's rows
+            // so far, four threads a column
+            const int c = tid & 63;
+            const int diag = kPanel * i + min( c, nbi - 1 );
+            const T * U = arena + sp.u0 + (std::int64_t)sp.r0 * sp.ld0 + sp.r0 + diag;
+            const double inv = 1.0 / static_cast<double>( U[(std::int64_t)diag * sp.ld0] );
+            double sum = 0.0;
+#pragma unroll 16
+            for( int r = tid >> 6; r <= diag; r += 4 )
+            {
+                const double q = static_cast<double>( U[(std::int64_t)r * sp.ld0] ) * inv;
+                sum = fma( q, q, sum );
+            }
+            ism[tid] = sum;
+            __syncthreads();
+            if( tid < kPanel ) { sum = (ism[tid] + ism[tid + 64]) + (ism[tid + 128] + ism[tid + 192]); }
+            const int above = __syncthreads_or( tid < kPanel && !(sum <= kGuardGrowth) );
+            if( tid == 0 ) { grown[kGuardBlocks * task.sp + i] = above; }
         }
         return;
     }
@@ -2857,18 +2878,124 @@ __global__ __launch_bounds__(256) void super_inv_kernel( const SuperInvTask * __
     }
 }
 
+// The diag step of a guarded super-panel whose inverse is not used (kGuardGrowth), panel by panel in
+// one CTA: forward x_q = T_q^T (y_q - sum_{p<q} U_pq^T x_p), back x_q = T_q (y_q + z_q - sum_{p>q} U_qp x_p),
+// with the panels' own inverses T_q and the x_p read back from `out`.  Rare: plain loads.
+template<typename T, int KP>
+__device__ __noinline__ void super_diag_panels( const SuperPanel & sp, const T * __restrict__ arena, const double * __restrict__ tinv, int upper,
+                                                const double * in, const double * zbuf, double * out, int ld, int k, double * dsm )
+{
+    constexpr int nct = KP / 8;
+    constexpr int ldv = KP + 4;
+    double (*B)[kPld] = reinterpret_cast<double (*)[kPld]>( dsm );
+    double * V = dsm + kPanel * kPld;                  // [64][ldv]
+    double * X = V + kPanel * ldv;                     // [64][ldv]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nblk = (sp.rows + kPanel - 1) / kPanel;
+    const std::int64_t brow = (std::int64_t)sp.row0 + sp.r0;
+    const T * U = arena + sp.u0 + (std::int64_t)sp.r0 * sp.ld0 + sp.r0;
+    // this warp's rows of B^T S (forward) or B S (back)
+    auto product = [&]( double (&acc)[nct][2], const double * S )
+    {
+#pragma unroll
+        for( int ct = 0; ct < nct; ++ct ) { acc[ct][0] = 0.0; acc[ct][1] = 0.0; }
+        for( int kb = 0; kb < kSubs; ++kb )
+        {
+#pragma unroll
+            for( int ct = 0; ct < nct; ++ct )
+            {
+                if( upper ) { dmma_8x8x8( acc[ct], [&]( int i, int kk ) { return B[8 * warp + i][8 * kb + kk]; },
+                                                   [&]( int kk, int j ) { return S[(8 * kb + kk) * ldv + 8 * ct + j]; } ); }
+                else        { dmma_8x8x8( acc[ct], [&]( int i, int kk ) { return B[8 * kb + kk][8 * warp + i]; },
+                                                   [&]( int kk, int j ) { return S[(8 * kb + kk) * ldv + 8 * ct + j]; } ); }
+            }
+        }
+    };
+    double acc[nct][2];
+    for( int s = 0; s < nblk; ++s )
+    {
+        const int q = upper ? nblk - 1 - s : s;
+        const int nbq = super_block_rows( sp, q );
+        const std::int64_t qrow = brow + kPanel * q;
+        for( int idx = tid; idx < kPanel * KP; idx += 256 )
+        {
+            const int r = idx / KP, c = idx % KP;
+            double v = 0.0;
+            if( r < nbq && c < k ) { v = in[(qrow + r) * ld + c] + (upper ? zbuf[(qrow + r) * ld + c] : 0.0); }
+            V[r * ldv + c] = v;
+        }
+        for( int e = 0; e < s; ++e )
+        {
+            const int p = upper ? nblk - 1 - e : e, a = min( p, q ), b = max( p, q );
+            const int nba = super_block_rows( sp, a ), nbb = super_block_rows( sp, b ), nbp = super_block_rows( sp, p );
+            for( int idx = tid; idx < kPanel * kPanel; idx += 256 )
+            {
+                const int r = idx >> 6, c = idx & 63;
+                B[r][c] = r < nba && c < nbb ? static_cast<double>( U[(std::int64_t)(kPanel * a + r) * sp.ld0 + kPanel * b + c] ) : 0.0;
+            }
+            for( int idx = tid; idx < kPanel * KP; idx += 256 )
+            {
+                const int r = idx / KP, c = idx % KP;
+                X[r * ldv + c] = r < nbp && c < k ? out[(brow + kPanel * p + r) * ld + c] : 0.0;
+            }
+            __syncthreads();
+            product( acc, X );
+            double * v = V + (8 * warp + (lane >> 2)) * ldv + 2 * (lane & 3);
+#pragma unroll
+            for( int ct = 0; ct < nct; ++ct ) { v[8 * ct] -= acc[ct][0]; v[8 * ct + 1] -= acc[ct][1]; }
+            __syncthreads();
+        }
+        const double * tq = tinv + (std::int64_t)sp.panel[q] * (kPanel * kPanel);
+        for( int idx = tid; idx < kPanel * kPanel; idx += 256 )
+        {
+            const int r = idx >> 6, c = idx & 63;
+            B[r][c] = r < nbq && c < nbq ? tq[idx] : 0.0;
+        }
+        __syncthreads();
+        product( acc, V );
+        const int r = 8 * warp + (lane >> 2);
+        if( r < nbq )
+        {
+            double * dst = out + (qrow + r) * ld;
+#pragma unroll
+            for( int ct = 0; ct < nct; ++ct )
+            {
+                const int c = 8 * ct + 2 * (lane & 3);
+                if( c < k ) { dst[c] = acc[ct][0]; }
+                if( c + 1 < k ) { dst[c + 1] = acc[ct][1]; }
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // One block pair of a super-panel's diag step.  Forward (task (o, b), b <= o):
 // x_o += T_bo^T y_b; back (b >= o): x_o += T_ob (y_b + z_b).  y: `in`, z: the
 // rest steps' sums in `zbuf`, x: `out`, whose block rows are zero before the
 // step (the pairs of one block row add into it).  KP = k rounded up to a power
 // of two >= 8.  One 64 x 64 block of T and one 64 x k block of vectors per
-// CTA, all copies in flight together.
-template<int KP>
+// CTA, all copies in flight together.  A guarded super-panel that does not use
+// its inverse leaves its diag step to the CTA of its first pair.
+template<typename T, int KP>
 __device__ __forceinline__ void super_diag_body( const SuperSolveTask & task, const SuperPanel * __restrict__ sps,
-                                                 const double * __restrict__ tbuf, int upper, const double * in,
+                                                 const double * __restrict__ tbuf, const int * __restrict__ grown,
+                                                 const T * __restrict__ arena, const double * __restrict__ tinv, int upper, const double * in,
                                                  const double * zbuf, double * out, int ld, int k, double * dsm )
 {
     const SuperPanel & sp = sps[task.sp];
+    if( sp.guard )
+    {
+        static_assert( kGuardBlocks == 4, "one int4 a super-panel" );
+        const int4 g = *reinterpret_cast<const int4 *>( grown + kGuardBlocks * task.sp );
+        // (blocks beyond the super-panel's rows are never written)
+        if( (g.x | (sp.rows > kPanel ? g.y : 0) | (sp.rows > 2 * kPanel ? g.z : 0) | (sp.rows > 3 * kPanel ? g.w : 0)) != 0 )
+        {
+            if( task.blk != 0 || task.c0 != 0 ) { return; }
+            pdl_wait();
+            super_diag_panels<T, KP>( sp, arena, tinv, upper, in, zbuf, out, ld, k, dsm );
+            return;
+        }
+    }
     constexpr int nct = KP / 8;
     constexpr int ldv = KP + 4;
     double (*Tb)[kPld] = reinterpret_cast<double (*)[kPld]>( dsm );
@@ -2937,7 +3064,8 @@ __device__ __forceinline__ void super_diag_body( const SuperSolveTask & task, co
 template<typename T, int KP>
 __global__ __launch_bounds__(256) void super_diag_kernel( const SuperSolveTask * __restrict__ tasks, int ndiag,
                                                           const SolveRestTask * __restrict__ steps, const SuperPanel * __restrict__ sps,
-                                                          const double * __restrict__ tbuf, const T * __restrict__ arena,
+                                                          const double * __restrict__ tbuf, const int * __restrict__ grown,
+                                                          const T * __restrict__ arena,
                                                           const double * __restrict__ tinv, const std::int32_t * __restrict__ sn_inner,
                                                           int upper, double * in, const double * zbuf, double * out, int ld, int k )
 {
@@ -2945,7 +3073,7 @@ __global__ __launch_bounds__(256) void super_diag_kernel( const SuperSolveTask *
     pdl_allow_next();
     if( static_cast<int>( blockIdx.x ) < ndiag )
     {
-        super_diag_body<KP>( tasks[blockIdx.x], sps, tbuf, upper, in, zbuf, out, ld, k, dsm );
+        super_diag_body<T, KP>( tasks[blockIdx.x], sps, tbuf, grown, arena, tinv, upper, in, zbuf, out, ld, k, dsm );
     }
     else
     {
@@ -3241,9 +3369,9 @@ void launch_solve_step( const SolveRestTask * tasks, int count, int small_count,
 
 template<typename T>
 void launch_super_inv( const SuperInvTask * tasks, int count, int part, const SuperPanel * sps, const T * arena, const double * tinv,
-                       double * tbuf, cudaStream_t st )
+                       double * tbuf, int * grown, cudaStream_t st )
 {
-    if( count > 0 ) { launch_pdl( super_inv_kernel<T>, count, 256, kSuperInvSmem, st, tasks, part, sps, arena, tinv, tbuf ); }
+    if( count > 0 ) { launch_pdl( super_inv_kernel<T>, count, 256, kSuperInvSmem, st, tasks, part, sps, arena, tinv, tbuf, grown ); }
 }
 
 template<typename T>
@@ -3260,18 +3388,18 @@ static size_t super_rest_smem( int k )
 
 template<typename T>
 void launch_super_diag( const SuperSolveTask * tasks, int count, const SolveRestTask * steps, int nsteps, const SuperPanel * sps,
-                        const double * tbuf, const T * arena, const double * tinv, const std::int32_t * sn_inner, bool upper,
-                        double * in, const double * zbuf, double * out, int ld, int k, cudaStream_t st )
+                        const double * tbuf, const int * grown, const T * arena, const double * tinv, const std::int32_t * sn_inner,
+                        bool upper, double * in, const double * zbuf, double * out, int ld, int k, cudaStream_t st )
 {
     if( count + nsteps <= 0 ) { return; }
     const size_t sm = super_diag_smem<T>( k );
     const int u = upper ? 1 : 0, n = count + nsteps;
     switch( solve_lkp( k ) )
     {
-        case 3:  launch_pdl( super_diag_kernel<T, 8>, n, 256, sm, st, tasks, count, steps, sps, tbuf, arena, tinv, sn_inner, u, in, zbuf, out, ld, k ); break;
-        case 4:  launch_pdl( super_diag_kernel<T, 16>, n, 256, sm, st, tasks, count, steps, sps, tbuf, arena, tinv, sn_inner, u, in, zbuf, out, ld, k ); break;
-        case 5:  launch_pdl( super_diag_kernel<T, 32>, n, 256, sm, st, tasks, count, steps, sps, tbuf, arena, tinv, sn_inner, u, in, zbuf, out, ld, k ); break;
-        default: launch_pdl( super_diag_kernel<T, 64>, n, 256, sm, st, tasks, count, steps, sps, tbuf, arena, tinv, sn_inner, u, in, zbuf, out, ld, k ); break;
+        case 3:  launch_pdl( super_diag_kernel<T, 8>, n, 256, sm, st, tasks, count, steps, sps, tbuf, grown, arena, tinv, sn_inner, u, in, zbuf, out, ld, k ); break;
+        case 4:  launch_pdl( super_diag_kernel<T, 16>, n, 256, sm, st, tasks, count, steps, sps, tbuf, grown, arena, tinv, sn_inner, u, in, zbuf, out, ld, k ); break;
+        case 5:  launch_pdl( super_diag_kernel<T, 32>, n, 256, sm, st, tasks, count, steps, sps, tbuf, grown, arena, tinv, sn_inner, u, in, zbuf, out, ld, k ); break;
+        default: launch_pdl( super_diag_kernel<T, 64>, n, 256, sm, st, tasks, count, steps, sps, tbuf, grown, arena, tinv, sn_inner, u, in, zbuf, out, ld, k ); break;
     }
 }
 
@@ -3315,8 +3443,8 @@ void launch_gather_diag( const std::int64_t * offsets, const T * arena, double *
                                         const std::int32_t *, double *, double *, int, int, cudaStream_t );         \
     template void launch_gather_diag<T>( const std::int64_t *, const T *, double *, int, cudaStream_t );          \
     template void launch_super_inv<T>( const SuperInvTask *, int, int, const SuperPanel *, const T *, const double *,      \
-                                       double *, cudaStream_t );                                                    \
-    template void launch_super_diag<T>( const SuperSolveTask *, int, const SolveRestTask *, int, const SuperPanel *, const double *, const T *,   \
+                                       double *, int *, cudaStream_t );                                             \
+    template void launch_super_diag<T>( const SuperSolveTask *, int, const SolveRestTask *, int, const SuperPanel *, const double *, const int *, const T *, \
                                         const double *, const std::int32_t *, bool, double *, const double *, double *, int, int, cudaStream_t ); \
     template void launch_super_rest<T>( const SuperSolveTask *, int, const SuperPanel *, const T *,                 \
                                         const std::int32_t *, bool, double *, double *, const double *, int, int,   \

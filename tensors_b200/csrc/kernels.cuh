@@ -136,16 +136,18 @@ void launch_solve_dag( const SolveDagArgs & args, int grid, const T * arena, dou
 int solve_dag_blocks_per_sm( int k );
 
 // Super-panel solve (plan.hpp, SuperPanel): the inverses' product launches (part 0: W and the copies, 1: T)
-// (after the factorization; tbuf: Plan::super_inv_size doubles), and the diag
+// (after the factorization; tbuf: Plan::super_inv_size doubles; grown: kGuardBlocks
+// ints per super-panel, where the copies of a guarded super-panel's panel inverses
+// note the blocks with a pivot below kGuardGrowth's line), and the diag
 // and rest steps of the sweeps (zbuf: n x ld doubles, zero before the back
 // sweep; in / out as launch_solve_step's).
 template<typename T>
 void launch_super_inv( const SuperInvTask * tasks, int count, int part, const SuperPanel * sps, const T * arena, const double * tinv,
-                       double * tbuf, cudaStream_t st );
+                       double * tbuf, int * grown, cudaStream_t st );
 template<typename T>
 void launch_super_diag( const SuperSolveTask * tasks, int count, const SolveRestTask * steps, int nsteps, const SuperPanel * sps,
-                        const double * tbuf, const T * arena, const double * tinv, const std::int32_t * sn_inner, bool upper,
-                        double * in, const double * zbuf, double * out, int ld, int k, cudaStream_t st );
+                        const double * tbuf, const int * grown, const T * arena, const double * tinv, const std::int32_t * sn_inner,
+                        bool upper, double * in, const double * zbuf, double * out, int ld, int k, cudaStream_t st );
 template<typename T>
 void launch_super_rest( const SuperSolveTask * tasks, int count, const SuperPanel * sps, const T * arena,
                         const std::int32_t * sn_inner, bool upper, double * in, double * zbuf, const double * out, int ld, int k,

@@ -1056,6 +1056,7 @@ void Plan::build_super( const std::vector<std::vector<I32>> & front_panels, Rang
             sp.n0 = front_n0[f]; sp.n1 = front_n1[f]; sp.ld0 = front_ld0[f]; sp.ld1 = front_ld1[f];
             sp.r0 = r0; sp.rows = std::min( kSuperRows, front_n0[f] - r0 ); sp.row0 = front_row0[f];
             sp.ldt = kPanel * static_cast<I32>( ceil_div( sp.rows, kPanel ) );
+            sp.guard = front_n0[f] < kSuperMinRows ? 1 : 0;
             for( I32 b = 0; b < kSuperPanels; ++b )
             {
                 const size_t q = static_cast<size_t>( r0 / kPanel + b );

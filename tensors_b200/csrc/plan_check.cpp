@@ -661,6 +661,7 @@ std::string check_panels( const Symbolic & sym, const Plan & pl )
             if( sp.n1 > 0 && (sp.inner < 0 || sp.inner + sp.n1 > inner_size) ) { return "super-panel columns out of range" + at; }
             if( sp.row0 < 0 || sp.row0 + sp.n0 > sym.n ) { return "super-panel rows out of the matrix" + at; }
             if( sp.ldt != kPanel * ((sp.rows + kPanel - 1) / kPanel) ) { return "super-panel inverse edge" + at; }
+            if( sp.guard != (sp.n0 < kSuperMinRows ? 1 : 0) || (sp.guard && (sp.r0 != 0 || sp.rows != sp.n0 || sp.ldt > kGuardBlocks * kPanel)) ) { return "super-panel guard" + at; }
             if( sp.t < 0 || sp.t + static_cast<I64>( sp.ldt ) * sp.ldt > pl.super_inv_size ) { return "super-panel inverse out of range" + at; }
             nblk[static_cast<size_t>( p )] = (sp.rows + kPanel - 1) / kPanel;
             nrest[static_cast<size_t>( p )] = (sp.n0 - sp.r0 - sp.rows) + sp.n1;
