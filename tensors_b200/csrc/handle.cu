@@ -184,7 +184,8 @@ struct tb_chol
     DeviceArray<unsigned long long> solve_trace_buf; // with `trace`: forward then back sweep of the first RHS chunk
     int solve_schedule = TB_SCHEDULE_LEVELS;
     int dag_grid = 0;                            // CTAs of the persistent factorization launch
-    bool dag_ready = false;                      // the task graph is ordered and on the device
+    bool dag_ordered = false;                    // the task graph is ordered (host)
+    bool dag_ready = false;                      // and on the device
     bool use_dag = false;                        // persistent task-graph launch (else one launch per step)
     int schedule = TB_SCHEDULE_LEVELS;
     int precision = TB_PRECISION_FP64;
@@ -450,18 +451,28 @@ int ensure_device( tb_chol * h )
     TB_CUDA( cudaStreamSynchronize( st_ ) );
     if( h->factor_graph ) { cudaGraphExecDestroy( h->factor_graph ); h->factor_graph = nullptr; }
     h->drop_solve_graphs();
+    h->dag_ordered = false;
     h->dag_ready = false;
     h->device_ready = true;
     return TB_OK;
 }
 
-// Orders the factorization's task graph for the persistent launch, checks the order and uploads
-// it: only for the schedules that run it (the level schedule's first pass spent 21 of its 120 ms
-// here for the 64^3 Laplacian).
+// Orders the factorization's task graph for the persistent launch (host work: 21 ms for the 64^3
+// Laplacian, of a first pass of 120 when every schedule did it): on first use by a schedule that
+// runs the graph, or by the statistics that report its duration.
+void order_task_graph( tb_chol * h )
+{
+    if( h->dag_ordered ) { return; }
+    tb::schedule_task_graph( h->plan, h->dag_grid );
+    h->dag_ordered = true;
+}
+
+// The ordered task graph, checked and on the handle's device: only for the schedules that run it.
 int ensure_task_graph( tb_chol * h )
 {
     if( h->dag_ready ) { return TB_OK; }
-    tb::schedule_task_graph( h->plan, h->dag_grid );
+    TB_CUDA( cudaSetDevice( h->device ) );
+    order_task_graph( h );
     const std::string msg = tb::check_task_graph( h->plan );
     if( !msg.empty() ) { return fail( TB_ERR_INVALID_ARGUMENT, "plan check: " + msg ); }
     TB_TRY( h->dag.upload( h->plan.dag, h->stream ) );
@@ -2203,7 +2214,7 @@ int tb_chol_plan_stats( tb_chol * h, std::int64_t * out, std::int32_t cap )
     TB_TRY( check_handle( h ) );
     if( out == nullptr || cap < 0 ) { return fail( TB_ERR_INVALID_ARGUMENT, "null output" ); }
     TB_TRY( ensure_symbolic( h ) );
-    if( h->device_ready ) { TB_TRY( ensure_task_graph( h ) ); }     // (the ordered graph's duration)
+    if( h->device_ready ) { order_task_graph( h ); }     // (the ordered graph's duration; no device work)
     const tb::Plan & pl = h->plan;
     const std::int64_t v[] = {
         pl.arena_size(), pl.v_size, pl.levels, static_cast<std::int64_t>( level_launches( h ).size() ) + 2,
