@@ -2,7 +2,9 @@
 #pragma once
 
 #include <algorithm>
+#include <cstddef>
 #include <cstdint>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -25,10 +27,13 @@ void parallel_rows( std::int64_t count, Body && body, std::int64_t max_threads =
     const std::int64_t threads = std::min<std::int64_t>( host_threads( max_threads ), std::max<std::int64_t>( 1, count / 65536 ) );
     if( threads <= 1 ) { body( std::int64_t(0), count ); return; }
     std::vector<std::thread> pool;
+    pool.reserve( static_cast<std::size_t>( threads ) );
     for( std::int64_t t = 0; t < threads; ++t )
     {
         const std::int64_t b = count * t / threads, e = count * (t + 1) / threads;
-        pool.emplace_back( [&body, b, e]() { body( b, e ); } );
+        // a range whose thread cannot be created runs here
+        try { pool.emplace_back( [&body, b, e]() { body( b, e ); } ); }
+        catch( const std::system_error & ) { body( b, e ); }
     }
     for( auto & th : pool ) { th.join(); }
 }

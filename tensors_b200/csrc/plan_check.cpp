@@ -17,6 +17,7 @@
 #include <future>
 #include <map>
 #include <string>
+#include <system_error>
 #include <vector>
 
 namespace tb
@@ -855,12 +856,17 @@ std::string check_panels( const Symbolic & sym, const Plan & pl )
 // (Two threads for large plans: 64^3 Laplacian 78 -> 41 ms of its first pass.)
 std::string check_plan( const Symbolic & sym, const Plan & pl )
 {
-    const bool two = host_threads( pl.threads ) > 1 && pl.lut.size() > 65536;
-    std::future<std::string> children = std::async( two ? std::launch::async : std::launch::deferred, [&]() { return check_children( sym, pl ); } );
+    std::future<std::string> children;
+    if( host_threads( pl.threads ) > 1 && pl.lut.size() > 65536 )
+    {
+        // (without a second thread to be had, one after the other)
+        try { children = std::async( std::launch::async, [&]() { return check_children( sym, pl ); } ); }
+        catch( const std::system_error & ) {}
+    }
     std::string msg;
-    if( !two ) { msg = children.get(); if( !msg.empty() ) { return msg; } }
+    if( !children.valid() ) { msg = check_children( sym, pl ); if( !msg.empty() ) { return msg; } }
     const std::string panels = check_panels( sym, pl );
-    if( two ) { msg = children.get(); }
+    if( children.valid() ) { msg = children.get(); }
     return msg.empty() ? panels : msg;
 }
 
