@@ -2244,17 +2244,15 @@ int tb_chol_check_plan( tb_chol * h )
 int tb_chol_device_bytes( tb_chol * h, std::int64_t * out )
 {
     if( h == nullptr || out == nullptr ) { return fail( TB_ERR_INVALID_ARGUMENT, "null argument" ); }
-    std::int64_t b = 0;
-    b += h->arena.size * 8 + h->asm_src.size * 8 + h->asm_dst.size * 8 + h->diag_off.size * 8;
-    b += (h->lut.size + h->sn_inner.size + h->p.size + h->p_inv.size + h->a_inner.size) * 4;
-    b += h->gemm.size * (std::int64_t)sizeof(tb::GemmTask) + (h->panel.size + h->potrf.size) * (std::int64_t)sizeof(tb::PanelTask);
-    b += (h->extend.size + h->extend_segs.size) * (std::int64_t)sizeof(tb::ExtendTask) + h->sdiag.size * (std::int64_t)sizeof(tb::SolveDiagTask);
-    b += h->extend_pull.size * (std::int64_t)sizeof(tb::ExtendPullTask);
-    b += h->srest.size * (std::int64_t)sizeof(tb::SolveRestTask) + h->a_outer.size * 8;
-    b += h->zero.size * (std::int64_t)sizeof(tb::ZeroTask) + h->exports.size * (std::int64_t)sizeof(tb::ExportTask);
-    b += h->colmap.size * 4 + h->exported.size * 8;
-    b += (h->values.size + h->work.size + h->work2.size + h->in.size + h->out.size + h->diag_vals.size + h->tinv.size) * 8;
-    *out = b;
+    auto sum = []( const auto & ... a ) { return (std::int64_t{ 0 } + ... + (a.size * static_cast<std::int64_t>( sizeof(*a.ptr) ))); };
+    *out = sum( h->arena, h->tinv, h->tsuper, h->grown, h->values, h->reg, h->status, h->pivot_floor, h->exported, h->diag_vals )
+         + sum( h->asm_src, h->asm_dst, h->diag_off, h->lut, h->sn_inner, h->p, h->p_inv, h->colmap, h->a_outer, h->a_inner )
+         + sum( h->zero, h->exports, h->gemm, h->tc, h->img, h->potrf, h->panel, h->extend, h->extend_pull, h->extend_segs, h->fronts )
+         + sum( h->sdiag, h->srest, h->spanels, h->sinv, h->ssolve, h->dag, h->dag_state, h->trace_buf )
+         + sum( h->solve_fwd_order, h->solve_bwd_order, h->solve_targets, h->solve_fwd_expected, h->solve_panel_tasks,
+                h->solve_target_ptr, h->solve_state, h->solve_trace_buf )
+         + sum( h->work, h->work2, h->work3, h->in, h->out, h->ir_x, h->ir_r, h->ir_norms, h->cg_buf, h->cg_scal, h->cg_host,
+                h->gm_buf, h->gm_scal );
     return TB_OK;
 }
 
