@@ -386,7 +386,21 @@ void Plan::build( const Symbolic & sym )
     front_small.assign( static_cast<size_t>(F), 0 );
     for( I32 h = 0; h < levels; ++h )
     {
-        auto fits = [&]( I32 f ) { return front_n0[f] <= kPanel && front_smem_bytes( front_n0[f], front_n1[f] ) <= kFrontSmemMax; };
+        auto shape_fits = [&]( I32 f ) { return front_n0[f] <= kPanel && front_smem_bytes( front_n0[f], front_n1[f] ) <= kFrontSmemMax; };
+        auto wide_parent = [&]( I32 f )
+        {
+            if( front_n0[f] + front_n1[f] <= kFrontWide ) { return false; }
+            I64 entries = 0;
+            for( I32 c = child_ptr[f]; c < child_ptr[f+1]; ++c )
+            {
+                const I64 m1 = front_n1[child_idx[static_cast<size_t>(c)]];
+                entries += m1 * (m1 + 1) / 2;
+            }
+            return entries > kFrontChildEntries;
+        };
+        I64 wide = 0;
+        for( I32 f : by_level[h] ) { wide += shape_fits( f ) && wide_parent( f ) ? 1 : 0; }
+        auto fits = [&]( I32 f ) { return shape_fits( f ) && (wide >= kFrontSpread || !wide_parent( f )); };
         I64 count = 0;
         for( I32 f : by_level[h] ) { count += fits( f ) ? 1 : 0; }
         if( 2 * count < static_cast<I64>( by_level[h].size() ) ) { continue; }

@@ -250,6 +250,19 @@ constexpr std::int64_t kFrontSmemMax   = 220 * 1024;  // one CTA of 384 threads 
 constexpr std::int64_t kFrontSmemMid   = 111 * 1024;  // two of 256 threads
 constexpr std::int64_t kFrontSmemSmall = 74 * 1024;   // three of 128 threads
 constexpr std::int32_t kFrontFew = 148, kFrontMany = 2000;
+// A front taken whole adds its children in one CTA, where the extend-add by
+// parent rows spreads a wide parent's rows over the chip.  A front of more than
+// kFrontWide rows in all whose children's update matrices have more than
+// kFrontChildEntries entries together is wide-parented; a level keeps the
+// launches for these fronts when it has fewer than kFrontSpread of them.
+// Measured on groups of 3-row leaves under fronts of 8 rows and 200 rest rows,
+// whole and apart: 3 such fronts with 65k entries of children 134 and 136 us,
+// 130k 170 and 157, 347k 281 and 198, 1391k 790 and 404; 12 fronts with 347k
+// each 309 and 256; 40 fronts with 347k each 470 and 563.  Fronts of up to 80
+// rows are as fast whole with any number of children (25 rows, 2048 children:
+// 1.3 and 2.7 ms; 64 rows, 64 children: 244 and 264 us).
+constexpr std::int64_t kFrontChildEntries = 65536;
+constexpr std::int32_t kFrontWide = 80, kFrontSpread = 32;
 
 // Shared memory of front_kernel in doubles: the front's rows (diagonal block
 // and rest columns, each rounded up to 8), the block's inverse, the update
