@@ -48,58 +48,6 @@ __device__ __forceinline__ void cp_async_8( double * smem_dst, const double * gm
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile( "cp.async.wait_all;\n" ::: "memory" ); }
 
-__device__ __forceinline__ void cp_async_4( void * smem_dst, const void * gmem_src, bool valid )
-{
-    const unsigned saddr = static_cast<unsigned>( __cvta_generic_to_shared( smem_dst ) );
-    asm volatile( "cp.async.ca.shared.global [%0], [%1], 4, %2;\n" :: "r"(saddr), "l"(gmem_src), "r"(valid ? 4 : 0) );
-}
-
-// Stages kIters elements per thread (element idx = threadIdx.x + u * kThreads)
-// of a factor block into double shared-memory cells with asynchronous copies,
-// so that all of a thread's copies are in flight together.  src( idx, fill )
-// returns the element's address, or nullptr with `fill` set to the value of a
-// cell outside the block; dst( idx ) is the cell.  FP32 storage: the float is
-// copied into the cell's first 4 bytes and widened in place by stage_finish,
-// which every thread calls for its own cells after cp_async_wait_all and
-// before the block is shared (__syncthreads).
-template<typename T, int kIters, int kThreads, typename Src, typename Dst>
-__device__ __forceinline__ void stage_block( const T * base, Src src, Dst dst )
-{
-#pragma unroll 4
-    for( int u = 0; u < kIters; ++u )
-    {
-        const int idx = threadIdx.x + u * kThreads;
-        double fill = 0.0;
-        const T * s = src( idx, fill );
-        if( s != nullptr || fill == 0.0 )
-        {
-            if constexpr ( sizeof(T) == 8 ) { cp_async_8( dst( idx ), s ? s : base, s != nullptr ); }
-            else { cp_async_4( dst( idx ), s ? s : base, s != nullptr ); }
-        }
-        else { *dst( idx ) = fill; }
-    }
-}
-
-template<typename T, int kIters, int kThreads, typename Src, typename Dst>
-__device__ __forceinline__ void stage_finish( Src src, Dst dst )
-{
-    if constexpr ( sizeof(T) == 4 )
-    {
-#pragma unroll 4
-        for( int u = 0; u < kIters; ++u )
-        {
-            const int idx = threadIdx.x + u * kThreads;
-            double fill = 0.0;
-            const T * s = src( idx, fill );
-            if( s != nullptr || fill == 0.0 )
-            {
-                double * d = dst( idx );
-                *d = static_cast<double>( *reinterpret_cast<const float *>( d ) );
-            }
-        }
-    }
-}
-
 // Programmatic dependent launch (sm_90+).  Kernels of the level schedule are
 // launched with programmatic stream serialization: a kernel lets the next one
 // in its stream launch as soon as all of its own CTAs are running
@@ -444,7 +392,7 @@ struct PotrfShared
 // Cholesky of the diagonal tile q of D by one warp, and W = U_qq^{-1} into
 // tile (q, q) of Ti.  Every lane holds the whole trailing tile in registers
 // and runs the same branch-free recurrence, so that a pivot's chain is one
-// reciprocal square root, one product and one fused multiply-add (83 cycles);
+// reciprocal square root, one product and one fused multiply-add (93 cycles);
 // lane j also carries column j of the identity through the elimination, whose
 // row r is then L^{-1}_rj = W_jr (L = U_qq^T), off the pivot chain.  With FP32 storage U is rounded as it is
 // stored and W inverts the rounded rows (the reciprocal of a stored pivot by
@@ -610,6 +558,26 @@ __device__ __noinline__ void potrf_row_substitution( const PotrfShared<kLd> sh, 
     }
 }
 
+// Cholesky of a panel's diagonal block D and the inverse T of its factor
+// (LAPACK potrf of FactorizeSupernode, Multifrontal.hpp:438-449, plus the
+// inverse that the trsm and the solves use), right-looking by 8 x 8 tiles.
+// Step b runs between two block barriers; barrier 1 divides it for the warps
+// that do not run the pivot chain:
+//   warp 0   row tile (b, b+1); arrives at barrier 1 without waiting there;
+//            update and factorization of tile (b+1, b+1), and its inverse
+//            W_{b+1} into tile (b+1, b+1) of Ti.
+//   others   until barrier 1: the other row tiles U_bc, c > b+1, in place, and
+//            T_ib = -S_ib W_b, i < b, over S_ib in tile (i, b) of Ti;
+//            after it, with row block b complete: the trailing tiles but
+//            (b+1, b+1), S_{i,b+1} = sum_{k=i..b} T_ik U_{k,b+1} into tile
+//            (i, b+1) of Ti, and the stores of what step b-1 finished.
+// Everything the others read of warp 0's tile (b+1, b+1) - U, W, the ill()
+// flag - was written before the step's last barrier; everything warp 0 reads
+// of row block b and of tile (b+1, b+1) it wrote itself or found complete at
+// the step's start.  A step lasts as long as warp 0's chain (8 pivots of ~93
+// cycles and two tile products) while the others' jobs fit beside it, which
+// they do with nine warps; step -1 only factors tile 0.
+//
 // kThreads: 384 in the panel launches and the larger small fronts, 128 in the
 // smaller ones, 256 in the persistent kernel.  The block (nb x nb, identity beyond
 // up to a multiple of 8) is in sh.D; pending: its cp.async copies may still be
@@ -1170,6 +1138,7 @@ void front_kernel( const FrontTask * __restrict__ tasks, const ExtendTask * __re
 // follow 88 fragment loads, and the results go to global memory from the
 // registers.  Bound: the launch's latency (load, 72 DMMAs a warp, store) on
 // the panel chain.
+
 // Operand-image entry of U row k, rest column `col` of a panel whose rest
 // columns start at U0 column r1 (m of them in U0, the rest U1 columns).
 __device__ __forceinline__ std::int64_t img_offset( const PanelTask & t, int k, int col, int r1, int m )
@@ -1731,7 +1700,6 @@ __global__ __launch_bounds__(kGemmThreads) void gemm_tn_kernel( const GemmTask *
 // solution itself and no CTA waits for another.
 
 constexpr int kTld = kPanel + 4;   // padded shared-memory row of 64-wide blocks (conflict-free DMMA fragments)
-// Doubles of shared memory the solve step's staged rest block takes (64 x kTld of T, rounded up).
 
 // acc[ct] (8 x 8 tile ct of this warp's 8 output rows, NCT tiles) += sum over
 // the K blocks [kb0, kb1) of A(i, kk) * B(kk, ct * 8 + j).
@@ -2001,7 +1969,7 @@ __device__ __forceinline__ void solve_step_body( const SolveRestTask & t, int up
 // changes from accumulator to operand layout by shuffles.  A CTA per such front
 // spent its time on two block barriers and on occupancy (2 to 4 an SM); of a
 // grid's leaves half have one row and six rest rows.  C2 with 16 right-hand
-// sides 1.22 -> 1.11 ms, 56^3 with 64 2.01 -> 1.89 ms, 96 meshes 481 -> 404 us.
+// sides 1.22 -> 1.11 ms, 56^3 with 64 2.01 -> 1.89 ms, 96 meshes 481 -> 403 us.
 template<typename T, int KP>
 __device__ __forceinline__ void solve_warp_body( const SolveRestTask & t, int upper, const T * __restrict__ arena,
                                                  const double * __restrict__ tinv, const std::int32_t * __restrict__ sn_inner,
