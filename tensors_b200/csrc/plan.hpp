@@ -249,6 +249,12 @@ struct FrontTask
 constexpr std::int64_t kFrontSmemMax   = 220 * 1024;  // one CTA of 384 threads per SM
 constexpr std::int64_t kFrontSmemMid   = 111 * 1024;  // two of 256 threads
 constexpr std::int64_t kFrontSmemSmall = 74 * 1024;   // three of 128 threads
+// Up to kFrontFew fronts (the chip's 148 SMs: every CTA is resident whatever its shared memory) a
+// level's small fronts are one launch (fronts of 48 and 8 rows with 130 rest rows, 120 of them: 24 us
+// against 36 in two launches).  From kFrontMany on, fronts that fit kFrontSmemSmall run with 128 threads,
+// three CTAs an SM, where a whole level's throughput counts: 2,000 fronts of 24 rows and 60 rest rows
+// 70 -> 59 us, 4,000 134 -> 115; 60 to 200 of them take 12 to 15 us with 256 threads and 14 to 15 with 128.
+// (The two cross at about 300 fronts, 20.5 and 16.3 us; below 2,000 the level is a few us either way.)
 constexpr std::int32_t kFrontFew = 148, kFrontMany = 2000;
 // A front taken whole adds its children in one CTA, where the extend-add by
 // parent rows spreads a wide parent's rows over the chip.  A front of more than
