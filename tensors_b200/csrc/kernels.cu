@@ -506,6 +506,7 @@ __device__ __forceinline__ bool potrf_diag_tile( const PotrfShared<kLd> & sh, co
         const bool ill = __any_sync( 0xffffffffu, kIllPivot * pivot < entry );
         if( lane == 0 ) { sh.ill( q ) = ill ? 1 : 0; }
     }
+    if constexpr ( kFloored ) { nonpos = 0u; }          // (a floor of zero or NaN is no failure: the refined solve reports it)
     nonpos &= ~singles;
     if( nb - o < kSub ) { nonpos &= (1u << (nb - o)) - 1u; }
     if( lane == 0 && nonpos != 0u && sh.fail() < 0 ) { sh.fail() = o + __ffs( nonpos ) - 1; }
