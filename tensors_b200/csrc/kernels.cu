@@ -10,6 +10,7 @@
 #include "kernels.cuh"
 
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 #include <type_traits>
 
@@ -361,7 +362,9 @@ template<typename T> __device__ __forceinline__ double round_to( double v ) { re
 //
 // kIllPivot (FP64): a diagonal tile with a pivot below 1 / kIllPivot of its
 // diagonal entry (a pivot's ratio does not change when rows and columns are
-// scaled) solves its row block by substitution.  The product with the tile's
+// scaled), or with one that is not a positive finite number (its row is then
+// scaled by what rsqrt gives: an infinite pivot's to zero), solves its row
+// block by substitution.  The product with the tile's
 // inverse is exact to a few roundings only while the inverse stays small: with
 // every third row within 1e-10 (squared) of the one before, |U^T U - A| is 4
 // u |A| by substitution and 12,800 by the product, and from 1e-11 on the
@@ -426,9 +429,9 @@ __device__ __forceinline__ bool potrf_diag_tile( const PotrfShared<kLd> & sh, co
 #pragma unroll
         for( int c = r; c < kSub; ++c ) { a[r][c] = sh.D( o + r, o + c ); }
     }
-    // FP64: lane r (mod 8) keeps diagonal entry r and, below, its pivot
+    // FP64: lane r (mod 8) keeps diagonal entry r and, below, its pivot and the pivot's reciprocal square root
     const double entry = sh.D( o + (lane & (kSub - 1)), o + (lane & (kSub - 1)) );
-    double pivot = entry;
+    double pivot = entry, inv = 0.0;
     __syncwarp();                                       // every lane has the tile before lane 0 writes rows over it
     auto store_row = [&]( int r, const double (&v)[kSub] )
     {
@@ -472,8 +475,8 @@ __device__ __forceinline__ bool potrf_diag_tile( const PotrfShared<kLd> & sh, co
             else { if( o + r < nb && !(d > tau) ) { low |= 1u << r; } }
         }
         if( !(d > 0.0) ) { nonpos |= 1u << r; }
-        if( (lane & (kSub - 1)) == r ) { pivot = d; }
         const double iv = rsqrt( d );
+        if( (lane & (kSub - 1)) == r ) { pivot = d; inv = iv; }
         double us[kSub];
         a[r][r] = d * iv;
         us[r] = round_to<T>( a[r][r] );
@@ -503,8 +506,11 @@ __device__ __forceinline__ bool potrf_diag_tile( const PotrfShared<kLd> & sh, co
     }
     if constexpr ( sizeof(T) == 8 )
     {
-        const bool ill = __any_sync( 0xffffffffu, kIllPivot * pivot < entry );
+        const bool ill = __any_sync( 0xffffffffu, !(kIllPivot * pivot >= entry && pivot > 0.0 && pivot <= DBL_MAX) );
         if( lane == 0 ) { sh.ill( q ) = ill ? 1 : 0; }
+        // the substitution's factors, below the diagonal of the last tile row, where T has zeros
+        const int last = kSub * ((nb + kSub - 1) / kSub) - kSub;
+        if( ill && o < last && lane < kSub ) { sh.Ti( last + lane, o + lane ) = inv; }
     }
     if constexpr ( kFloored ) { nonpos = 0u; }          // (a floor of zero or NaN is no failure: the refined solve reports it)
     nonpos &= ~singles;
@@ -537,9 +543,10 @@ __device__ __noinline__ void potrf_tile_floored( const PotrfShared<kLd> sh, cons
     if( (threadIdx.x & 31) == 0 ) { sh.raised() |= 1 << q; }
 }
 
-// U_bc = U_bb^{-T} A_bc for tile (b, c) of D (tile corners o, oc), one column per lane.
+// U_bc = U_bb^{-T} A_bc for tile (b, c) of D (tile corners o, oc), one column per lane.  last: the
+// last tile row, which holds the pivots' reciprocals.
 template<typename T, int kLd>
-__device__ __noinline__ void potrf_row_substitution( const PotrfShared<kLd> sh, int o, int oc )
+__device__ __noinline__ void potrf_row_substitution( const PotrfShared<kLd> sh, int o, int oc, int last )
 {
     const int lane = threadIdx.x & 31;
     if( lane < kSub )
@@ -550,7 +557,7 @@ __device__ __noinline__ void potrf_row_substitution( const PotrfShared<kLd> sh, 
 #pragma unroll
         for( int r = 0; r < kSub; ++r )
         {
-            x[r] *= sh.Ti( (sizeof(T) == 4 ? kPanel - kSub : o) + r, o + r );      // the pivot's reciprocal
+            x[r] *= sh.Ti( last + r, o + r );
 #pragma unroll
             for( int r2 = r + 1; r2 < kSub; ++r2 ) { x[r2] -= sh.D( o + r, o + r2 ) * x[r]; }
         }
@@ -599,7 +606,7 @@ __device__ __forceinline__ void potrf_core( const PotrfShared<kLd> & sh, const P
     {
         if( sizeof(T) == 4 ? (sh.raised() >> (o / kSub)) & 1 : sh.ill( o / kSub ) )
         {
-            potrf_row_substitution<T>( sh, o, oc );
+            potrf_row_substitution<T>( sh, o, oc, sizeof(T) == 4 ? kPanel - kSub : kSub * (nsub - 1) );
             return;
         }
         const int ow = sizeof(T) == 4 ? kPanel - kSub : o;
