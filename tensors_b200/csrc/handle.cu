@@ -350,6 +350,14 @@ int ensure_symbolic( tb_chol * h )
 // Ints of tb_chol::grown.
 std::int64_t grown_size( const tb_chol * h ) { return static_cast<std::int64_t>( tb::kGuardBlocks ) * static_cast<std::int64_t>( h->plan.spanels.size() ); }
 
+// The trace buffers for the present plan: four time stamps a task of the factorization's graph, and
+// of either sweep's.  The persistent kernels write them unchecked, so that every new plan comes by here.
+int reserve_trace( tb_chol * h )
+{
+    TB_TRY( h->trace_buf.reserve( 4 * static_cast<std::int64_t>( h->plan.dag.size() ) ) );
+    return h->solve_trace_buf.reserve( 8 * static_cast<std::int64_t>( h->plan.srest.size() ) );
+}
+
 // Binds the handle's device and stream and uploads the plan (once per
 // symbolic analysis).  Everything before this point is host-only, so the
 // symbolic phase and its getters work without a GPU.
@@ -378,6 +386,7 @@ int ensure_device( tb_chol * h )
         h->kernels_configured = true;
     }
     if( h->device_ready ) { return TB_OK; }
+    if( h->trace ) { TB_TRY( reserve_trace( h ) ); }
     {
         // the persistent launch's CTA count (the task order for it: ensure_task_graph)
         int sms = 0;
@@ -2531,8 +2540,7 @@ int tb_chol_set_trace( tb_chol * h, std::int32_t enabled )
     TB_TRY( ensure_device( h ) );
     if( enabled )
     {
-        TB_TRY( h->trace_buf.reserve( 4 * static_cast<std::int64_t>( h->plan.dag.size() ) ) );
-        TB_TRY( h->solve_trace_buf.reserve( 8 * static_cast<std::int64_t>( h->plan.srest.size() ) ) );
+        TB_TRY( reserve_trace( h ) );
     }
     if( (enabled != 0) != h->trace )
     {
@@ -2549,6 +2557,7 @@ int tb_chol_trace( tb_chol * h, std::int64_t * out, std::int64_t cap )
     if( !h->trace || h->trace_buf.ptr == nullptr ) { return fail( TB_ERR_INVALID_ARGUMENT, "trace not enabled" ); }
     const std::int64_t n = static_cast<std::int64_t>( h->plan.dag.size() );
     if( out == nullptr || cap < 6 * n ) { return fail( TB_ERR_INVALID_ARGUMENT, "trace buffer too small" ); }
+    if( h->trace_buf.size < 4 * n ) { return fail( TB_ERR_INVALID_ARGUMENT, "no trace of the present plan" ); }
     std::vector<unsigned long long> raw( static_cast<size_t>( 4 * n ) );
     TB_CUDA( cudaMemcpyAsync( raw.data(), h->trace_buf.ptr, sizeof(unsigned long long) * raw.size(), cudaMemcpyDeviceToHost, h->stream ) );
     TB_CUDA( cudaStreamSynchronize( h->stream ) );
@@ -2568,6 +2577,7 @@ int tb_chol_solve_trace( tb_chol * h, std::int64_t * out, std::int64_t cap )
     if( !h->trace || h->solve_trace_buf.ptr == nullptr ) { return fail( TB_ERR_INVALID_ARGUMENT, "trace not enabled" ); }
     const std::int64_t n = static_cast<std::int64_t>( h->plan.solve_fwd_order.size() );
     if( out == nullptr || cap < 12 * n ) { return fail( TB_ERR_INVALID_ARGUMENT, "trace buffer too small" ); }
+    if( h->solve_trace_buf.size < 8 * n ) { return fail( TB_ERR_INVALID_ARGUMENT, "no trace of the present plan" ); }
     std::vector<unsigned long long> raw( static_cast<size_t>( 8 * n ) );
     if( n > 0 )
     {
