@@ -2327,6 +2327,7 @@ int tb_chol_set_solve_schedule( tb_chol * h, std::int32_t schedule )
         else { pl.build_solve_graph( h->sym, pl.solve_default_split ); }
         if( h->device_ready )
         {
+            TB_CUDA( cudaSetDevice( h->device ) );
             cudaStream_t st_ = h->stream;
             TB_TRY( h->solve_fwd_order.upload( pl.solve_fwd_order, st_ ) );
             TB_TRY( h->solve_bwd_order.upload( pl.solve_bwd_order, st_ ) );
