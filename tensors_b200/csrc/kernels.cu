@@ -370,9 +370,11 @@ template<typename T> __device__ __forceinline__ double round_to( double v ) { re
 // u |A| by substitution and 12,800 by the product, and from 1e-11 on the
 // product's errors make a later pivot negative.  The line lies where both
 // agree: with rows within 1e-2 every such tile is below it and the product
-// still as good.  A grid Laplacian's separator has no tile below it; the check
-// alone makes a factor 0 to 1.5% slower (31^3 grid 1450 -> 1468 us),
-// substitution in every tile 1 to 8%.
+// still as good.  Grid and vector Laplacians have no tile below it, a 131^2
+// mesh 2 of 2,709; the check alone makes a factor 0 to 1.5% slower (31^3 grid
+// 1454 -> 1468 us), substitution in every tile 1 to 8%.  (The same check beside
+// the row tiles' products or after the tile's inverse took more: 45^2 grid 111
+// us, 118 and 118.)
 constexpr double kIllPivot = 16.0;
 
 template<int kLd>
